@@ -1068,11 +1068,7 @@ extern "C" int ptd_adj_create(ptd_adj** out, const ptd_params* p)
     A->rb = p->precision == PTD_PREC_FP32_RB;
     A->expm = p->model == PTD_MODEL_NONLIN_EXPM;
     derive(A->p, A->dv);
-    {   // the adjoint kernels tile like the one-cell-per-lane FP64 kernels
-        ptd_params pt = A->p;
-        pt.precision = PTD_PREC_FP64;
-        A->cfg = tuned_config(pt);
-    }
+    A->cfg.chunk3d = z_march16(A->p);   // every form's kernel has 16-row CTAs
     {   // stagnation window: ~2 n_max iterations, the PT iteration's own time scale
         const int nmax = std::max(p->nx, std::max(p->ny, p->nz));
         A->stall = std::max(10, (2 * nmax + A->nchk - 1) / A->nchk);

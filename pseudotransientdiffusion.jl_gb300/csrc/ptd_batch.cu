@@ -1391,12 +1391,27 @@ extern "C" int ptd_batch_create(ptd_batch** out, const ptd_batch_params* p, cons
         for (auto& I : b->inst) nmax = std::max(nmax, std::max(I.nx, I.ny));
         q.nx = q.ny = nmax;
         b->cfg = tuned_config(q);
-        b->cfg.chunk2d = 32;
         b->stall = std::max(10, (2 * nmax + 49) / 50);
     }
     b->nchk = b->dc ? std::max(1, std::min(p->nchk, 50)) : p->nchk;
     if (b->dc && p->itmax % b->nchk) b->nchk = p->nchk;
     b->tb = ((b->dc || b->rb) && b->nchk % 2 == 0 && !(p->flags & PTD_FLAG_DC_NO_TBLOCK)) ? 2 : 1;
+    {   // rows per y chunk: 32, shorter (>= 8, alloc_slots) where the batch
+        // would not fill the SMs, in 2-warp CTAs then.  FP32_RB steps, 8 warps
+        // x 32 rows / as taken: 48 grids of 64..512 11.6, 10.0 ms (16 rows);
+        // 32 of 128..200 3.7, 2.3 ms (8); 8 of 32..100 1.7, 1.1 ms (8).
+        auto warps = [&](int ch) {
+            long long n = 0;
+            const int cols = b->tb == 2 ? 28 : 31;
+            for (const Inst& I : b->inst)
+                n += (long long)((I.nx - 2 + cols - 1) / cols) * ((I.ny - 2 + ch - 1) / ch);
+            return n;
+        };
+        int ch = 32;
+        while (ch > 8 && warps(ch) < 33LL * sm_count()) ch /= 2;
+        b->cfg.chunk2d = ch;
+        if (b->rb) b->cfg.warps2d = ch < 32 ? 2 : 8;
+    }
     // FP32_RB: a phase is the check blocks of ~200 iterations between two rebases
     b->blocks_per_phase = std::max(1, (200 + b->nchk - 1) / b->nchk);
     cudaError_t e = cudaStreamCreateWithFlags(&b->s, cudaStreamNonBlocking);

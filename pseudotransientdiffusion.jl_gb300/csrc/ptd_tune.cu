@@ -47,37 +47,105 @@ int z_chunk(long long bxy, int nz, long long slots)
     return best;
 }
 
+namespace {
+
+// The march length (rows in 2D, planes in 3D) of a launch: `pref` while
+// `units(march)` -- the warps (2D) or CTAs (3D) of the launch -- reaches
+// `hi`, halved down to `mid` otherwise; below that halved while fewer than
+// `lo` units run.  A march step is a chain of dependent loads and arithmetic
+// of about 1 us, so a grid too small to fill the SMs is bound by the march
+// length and not by its cells; a shorter march re-evaluates one face per cell
+// column and march start.
+template <class Units>
+int march_length(int pref, int mid, long long hi, long long lo, Units units)
+{
+    int m = pref;
+    while (m > mid && units(m) < hi) m /= 2;
+    while (m > 1 && units(m) < lo) m /= 2;
+    return m;
+}
+
+long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
+
+}  // namespace
+
+// z march of the 16-row FP32 kernels (rebased form, adjoint): us per
+// iteration at march 16 and at the march taken: rebased NONLIN 32^3 22.0, 7.5
+// (1); 64^3 22.6, 11.4 (4); 128^3 47.8, 44.1 (4); 192^3 119.5, 118.2 (8).
+int z_march16(const ptd_params& p)
+{
+    const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, 15);
+    const long long sm = sm_count();
+    return march_length(16, 4, 17 * sm / 2, sm, [&](int m) { return bxy * ceil_div(p.nz - 2, m); });
+}
+
 LaunchCfg tuned_config(const ptd_params& p)
 {
     LaunchCfg c;
+    const long long sm = sm_count();
     if (p.ndim == 2) {
         // short y marches in small CTAs: many independent warps per SM hide
-        // the memory latency of the march.  Measured at 4096^2 (NONLIN) over
-        // warps {1,2,4,8} x rows {8,16,32,64}, us per iteration against the
-        // former 2 warps x 16 rows: FP64 1 x 32 587.3 (598.5), DFH 1 x 8 199.0
-        // (202.4), DF64 2 x 8 169.3 (173.4), FP32_RB 8 x 32 (two-iteration
-        // marches of 64 rows) 64.6 (65.6); FP32_DC 2 x 16.
+        // the memory latency of the march.  Measured over warps {1,2,4,8} x
+        // rows {1..64}, us per iteration of a check block at the former fixed
+        // march and at the march taken here:
+        //   FP64 NONLIN (1 warp x 32 rows before) 128^2 38.2, 4.4 (1 row);
+        //     256^2 39.5, 6.6 (1); 512^2 38.0, 14.0 (4); 1024^2 48.6, 43.3 (16);
+        //     2048^2 167.4, 163.6 (16); 4096^2 624.9 (32), 629.1 with 16
+        //   DFH NONLIN (1 x 8) 256^2 12.0, 4.8 (1); 512^2 12.5, 7.8 (2);
+        //     1021x1500 29.7, 27.3 (4); 2048^2 62.7 (8)
+        //   FP32_RB NONLIN (8 x 32, marches of twice the rows) 256^2 28.9, 4.4
+        //     (1); 512^2 30.2, 4.8 (1); 1024^2 30.1, 8.1 (4); 2048^2 48.9,
+        //     26.0 (8); 3000^2 61.1, 48.1 (16); 4096^2 78.7 (32)
+        //   FP32_RB LINSTEP 1024^2 22.3, 7.2 (4); 2048^2 39.8, 24.6 (8)
+        //   FP32_DC NONLIN (2 x 16) 256^2 8.8, 4.7 (1); 512^2 8.7, 5.5 (4);
+        //     1024^2 9.2, 8.0 (8)
+        const bool coef = p.model == PTD_MODEL_LINSTEP || p.model == PTD_MODEL_NONLIN_EXPM;
+        const bool tb = p.nchk % 2 == 0 && !(p.flags & PTD_FLAG_DC_NO_TBLOCK);   // two FP32 iterations per launch
+        auto warps = [&](int cols, int rows_per) {
+            const long long tiles = ceil_div(p.nx - 2, cols);
+            return [&p, tiles, rows_per](int m) { return tiles * ceil_div(p.ny - 2, (long long)rows_per * m); };
+        };
         switch (p.precision) {
-        case PTD_PREC_FP64: c.warps2d = 1; c.chunk2d = 32; break;
-        case PTD_PREC_DFH: c.warps2d = 1; c.chunk2d = 8; break;
-        case PTD_PREC_DF64: c.warps2d = 2; c.chunk2d = 8; break;
-        case PTD_PREC_FP32_RB: c.warps2d = 8; c.chunk2d = 32; break;
-        default: c.warps2d = 2; c.chunk2d = 16; break;
+        case PTD_PREC_FP64:
+            c.warps2d = 1;
+            c.chunk2d = march_length(32, 16, 52 * sm, 25 * sm / 2, warps(31, 1));
+            break;
+        case PTD_PREC_DFH:
+        case PTD_PREC_DF64:
+            c.warps2d = p.precision == PTD_PREC_DFH ? 1 : 2;
+            c.chunk2d = march_length(8, 4, 52 * sm, 29 * sm / 2, warps(62, 1));
+            break;
+        case PTD_PREC_FP32_RB:
+            if (coef) c.chunk2d = march_length(8, 1, 30 * sm, 30 * sm, warps(tb ? 28 : 31, tb ? 2 : 1));
+            else c.chunk2d = march_length(32, 8, 26 * sm, 15 * sm, warps(tb ? 60 : 31, tb ? 2 : 1));
+            c.warps2d = c.chunk2d == 32 ? 8 : 2;
+            break;
+        default:
+            c.warps2d = 2;
+            c.chunk2d = march_length(16, 8, 52 * sm, 15 * sm, warps(tb ? 28 : 31, 1));
+            break;
         }
+    } else if (p.ndim == 3 && (p.precision == PTD_PREC_FP32_RB || p.precision == PTD_PREC_FP32_DC)) {
+        c.rows3d = 16;
+        c.chunk3d = z_march16(p);
     } else if (p.ndim == 3) {
-        // 512-thread CTAs of 31 x 15 updated cells, 3 resident per SM at <= 40
-        // registers (456 slots on the 152 SMs of a GB300), short z marches:
-        // at 512^3 over marches {16..512}, FP64 32 planes 6926 us (64: 7016,
-        // 512: 7388), DF64 32: 2011 (64: 2043), FP32_RB 16: 1196 (64: 1236).
-        // Grids too small for whole waves at that length take the longest
-        // march that fills the slots best (wave quantization).
-        const int rows = 16, tw = 31;
-        const long long slots = 3LL * sm_count();
-        const long long bxy = (long long)((p.nx - 2 + tw - 1) / tw) * ((p.ny - 2 + rows - 2) / (rows - 1));
-        const int pref = p.precision == PTD_PREC_FP32_RB ? 16 : 32;
-        const long long nb = bxy * ((p.nz - 2 + pref - 1) / pref);
-        c.chunk3d = nb >= 4 * slots ? pref : z_chunk(bxy, p.nz, slots);
-        c.rows3d = rows;
+        // The FP64-accuracy forms.  512-thread CTAs of 31 x 15 updated cells
+        // (3 resident per SM at <= 40 registers) on large grids; 256-thread
+        // CTAs of 31 x 7 cells, whose per-plane barrier joins half the warps
+        // and whose smaller tiles waste less of a ragged grid, below 288^3
+        // (DFH: at every size).  us per iteration, 16 rows with the former
+        // march / as taken here: FP64 NONLIN 64^3 68.6, 19.4 (8 rows x 4
+        // planes); 128^3 190.4, 148.2 (8 x 4); 256^3 1050, 1001 (8 x 16);
+        // 320^3 1920 (16 x 32), 1883 (16 x 16); 512^3 7299 (16 x 32), 7406
+        // (8 x 32); DF64 LIN 64^3 20.3, 7.5 (8 x 4); 128^3 46.6, 39.4; DFH
+        // NONLIN 128^3 81.1, 62.4; 512^3 2804, 2756 (8 x 32).
+        const bool small = p.precision == PTD_PREC_DFH || (double)p.nx * p.ny * p.nz < 24e6;
+        c.rows3d = small ? 8 : 16;
+        const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, c.rows3d - 1);
+        auto ctas = [&](int m) { return bxy * ceil_div(p.nz - 2, m); };
+        if (!small) c.chunk3d = ctas(32) >= 40 * sm ? 32 : 16;
+        else if (ctas(32) >= 52 * sm) c.chunk3d = 32;
+        else c.chunk3d = march_length(16, 4, 16 * sm, 4 * sm / 3, ctas);
     }
     return c;
 }

@@ -93,6 +93,15 @@ __device__ __forceinline__ double f2d_bits(float f)
     return __hiloint2double((int)hi, (int)lo);
 }
 
+// The same for a value that is not negative (the face parameter c).
+__device__ __forceinline__ double f2d_param(float f)
+{
+    const unsigned b = __float_as_uint(f);
+    const unsigned hi = (b >> 3) + (b >= 0x7f800000u ? 0x70000000u : 0x38000000u);
+    const bool normal = b >= 0x00800000u;
+    return __hiloint2double((int)(normal ? hi : 0u), (int)(normal ? b << 29 : 0u));
+}
+
 __device__ __forceinline__ float d2f_bits(double x)
 {
     int hi = __double2hiint(x);

@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(256) pt1d_kernel(PTArgs a)
 }
 
 template <class N, int MODEL, bool CHECK>
-__global__ void __launch_bounds__(256, CHECK ? 5 : 6) pt2d_kernel(PTArgs a, int chunk)
+__global__ void __launch_bounds__(256, CHECK ? 4 : 6) pt2d_kernel(PTArgs a, int chunk)
 {
     if (step_done(a.done)) return;
     double part = 0.0;

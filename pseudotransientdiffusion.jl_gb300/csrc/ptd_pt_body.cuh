@@ -5,6 +5,7 @@
 #pragma once
 
 #include "ptd_device.cuh"
+#include "ptd_intflux.cuh"
 #include "ptd_kernels.h"
 #include "ptd_num.cuh"
 
@@ -13,6 +14,10 @@ namespace ptd {
 // w - c*t with a float damping coefficient c.
 __device__ __forceinline__ double nmadf(F64, float c, double t, double w) { return fma(-f2d_bits(c), t, w); }
 __device__ __forceinline__ float2 nmadf(DF64, float c, float2 t, float2 w) { return DF64::nmadf(t, c, w); }
+
+// The damped flux of a face; its c is never negative.
+__device__ __forceinline__ double damp(F64, float c, double t, double w) { return fma(-f2d_param(c), t, w); }
+__device__ __forceinline__ float2 damp(DF64, float c, float2 t, float2 w) { return DF64::nmadf(t, c, w); }
 
 template <class N>
 __device__ __forceinline__ typename N::T ld(const void* p, long long i)
@@ -25,41 +30,80 @@ __device__ __forceinline__ void st(void* p, long long i, typename N::T v)
     reinterpret_cast<typename N::T*>(p)[i] = v;
 }
 
+// Native FP64: t = w + u and the undamped flux u = K_f (H_R - H_L), u in
+// integer arithmetic (ptd_intflux.cuh) wherever its operands allow.  Not in
+// 1D (INTF false), where a launch is bound by its latency and not by the FP64
+// pipe (512 cells: 3.1 us per iteration in FP64, 3.2 in integers).
+template <int MODEL, bool INTF>
+__device__ __forceinline__ double flux_add(double HL, double HR, double DL, double DR, double w, double& u)
+{
+    auto bits = [](double x) { return (uint64_t)__double_as_longlong(x); };
+    const double e2 = MODEL == NONLIN_EXPM ? DL + DR : 0.0;   // D holds exp(m): K = (E_L + E_R) s^3, kappa = 1/16
+    uint64_t r = 0;
+    bool ok = false;
+    if (INTF && MODEL == LIN) ok = if_flux_lin(bits(HL), bits(HR), r);
+    else if (INTF && MODEL == LINSTEP) ok = if_flux_step(bits(HL), bits(HR), bits(DL), bits(DR), r);
+    else if (INTF) ok = if_flux_cube(bits(HL), bits(HR), r);
+    if (ok) {
+        u = __longlong_as_double((long long)r);
+        if (MODEL == NONLIN_EXPM) {
+            const double t = fma(u, e2, w);
+            u *= e2;
+            return t;
+        }
+        return w + u;
+    }
+    const double g = HR - HL;
+    double K = 1.0;
+    if (MODEL == LINSTEP) K = DL + DR;
+    if (MODEL == NONLIN || MODEL == NONLIN_EXPM) {
+        const double s = HL + HR;
+        K = s * s * s;
+        if (MODEL == NONLIN_EXPM) K *= e2;
+    }
+    u = K * g;
+    return fma(K, g, w);
+}
+
 // One face: new scaled flux, and u = K_f * g (undamped flux) when U.
-template <class N, int MODEL, bool U>
+template <class N, int MODEL, bool U, bool INTF = true>
 __device__ __forceinline__ typename N::T face_t(const PTArgs& a, const typename N::HV& HL,
                                                 const typename N::HV& HR, float hsum, typename N::T DL,
                                                 typename N::T DR, typename N::T w, typename N::T& u)
 {
     using T = typename N::T;
-    const T g = N::hdiff(HR, HL);
-    if (MODEL == LIN) {
-        if (U) u = g;
-        return nmadf(N(), a.fc_lin, N::add(g, w), w);
-    }
-    float c;
-    T K;
-    if (MODEL == LINSTEP) {
-        K = N::add(DL, DR);
-        c = a.fc_lin;
-    } else if (MODEL == NONLIN) {
-        const T s = N::hsum(HL, HR);
-        K = N::mul(N::mul(s, s), s);
-        c = nonlin_face_c(a.f, hsum);
-    } else {   // NONLIN_EXPM: D holds exp(m); K = (E_L + E_R) s^3, kappa = 1/16
-        const T s = N::hsum(HL, HR);
-        const T e2 = N::add(DL, DR);
-        K = N::mul(N::mul(N::mul(s, s), s), e2);
-        c = nonlin_face_c(a.f, hsum, 0.5f * N::lo_f(e2));
-    }
-    T t;
-    if (U) {
-        u = N::mul(K, g);
-        t = N::native ? N::mad(K, g, w) : N::add(u, w);
+    float c = a.fc_lin;
+    if (MODEL == NONLIN) c = nonlin_face_c(a.f, hsum);
+    if constexpr (N::native) {
+        if (MODEL == NONLIN_EXPM) c = nonlin_face_c(a.f, hsum, 0.5f * N::lo_f(N::add(DL, DR)));
+        return damp(N(), c, flux_add<MODEL, INTF>(HL, HR, DL, DR, w, u), w);
     } else {
-        t = N::mad(K, g, w);
+        const T g = N::hdiff(HR, HL);
+        if (MODEL == LIN) {
+            if (U) u = g;
+            return damp(N(), c, N::add(g, w), w);
+        }
+        T K;
+        if (MODEL == LINSTEP) {
+            K = N::add(DL, DR);
+        } else {
+            const T s = N::hsum(HL, HR);
+            K = N::mul(N::mul(s, s), s);
+        }
+        if (MODEL == NONLIN_EXPM) {   // D holds exp(m); K = (E_L + E_R) s^3, kappa = 1/16
+            const T e2 = N::add(DL, DR);
+            K = N::mul(K, e2);
+            c = nonlin_face_c(a.f, hsum, 0.5f * N::lo_f(e2));
+        }
+        T t;
+        if (U) {
+            u = N::mul(K, g);
+            t = N::add(u, w);
+        } else {
+            t = N::mad(K, g, w);
+        }
+        return damp(N(), c, t, w);
     }
-    return nmadf(N(), c, t, w);
 }
 
 // ---------------------------------------------------------------------------
@@ -191,14 +235,14 @@ __device__ __forceinline__ void pt1d_body(const PTArgs& a, int bx, double& part,
         if (i <= nx - 2) {
             const HV Hr = N::ldh(a.Hin, i + 1);
             if (HASD) Dr = ld<N>(a.D, i + 1);
-            wr = face_t<N, MODEL, CHECK>(a, Hc, Hr, hc + N::hf(Hr), Dc, Dr, ld<N>(a.win[0], i), ur);
+            wr = face_t<N, MODEL, CHECK, false>(a, Hc, Hr, hc + N::hf(Hr), Dc, Dr, ld<N>(a.win[0], i), ur);
             st<N>(a.wout[0], i, wr);
         }
         if (i >= 1 && i <= nx - 2) {
             const HV Hl = N::ldh(a.Hin, i - 1);
             const T Dl = HASD ? ld<N>(a.D, i - 1) : N::zero();
             T ul = N::zero();
-            const T wl = face_t<N, MODEL, CHECK>(a, Hl, Hc, N::hf(Hl) + hc, Dl, Dc, ld<N>(a.win[0], i - 1), ul);
+            const T wl = face_t<N, MODEL, CHECK, false>(a, Hl, Hc, N::hf(Hl) + hc, Dl, Dc, ld<N>(a.win[0], i - 1), ul);
             const HS Ho = N::ldo(a.Hold, i);
             const float e = cell_e<MODEL>(a, hc, MODEL == NONLIN_EXPM ? N::lo_f(Dc)
                                                  : fmaxf(fmaxf(N::lo_f(Dl), N::lo_f(Dr)), N::lo_f(Dc)));

@@ -86,11 +86,11 @@ LaunchCfg tuned_config(const ptd_params& p)
     if (p.ndim == 2) {
         // short y marches in small CTAs: many independent warps per SM hide
         // the memory latency of the march.  Measured over warps {1,2,4,8} x
-        // rows {1..64}, us per iteration of a check block at the former fixed
-        // march and at the march taken here:
-        //   FP64 NONLIN (1 warp x 32 rows before) 128^2 38.2, 4.4 (1 row);
-        //     256^2 39.5, 6.6 (1); 512^2 38.0, 14.0 (4); 1024^2 48.6, 43.3 (16);
-        //     2048^2 167.4, 163.6 (16); 4096^2 624.9 (32), 629.1 with 16
+        // rows {1..64}, us per iteration of a check block at another march (FP32
+        // forms and DFH: the former fixed one) and at the one taken here:
+        //   FP64 NONLIN 128^2 5.5 (2 rows), 4.3 (1); 512^2 11.0 (1), 10.4 (4);
+        //     1024^2 29.6 (16), 27.4 (8); 2048^2 95.0 (8), 95.6 (16); 4096^2
+        //     353.9 (8), 351.4 (16), 355.0 (32); LIN and LINSTEP alike
         //   DFH NONLIN (1 x 8) 256^2 12.0, 4.8 (1); 512^2 12.5, 7.8 (2);
         //     1021x1500 29.7, 27.3 (4); 2048^2 62.7 (8)
         //   FP32_RB NONLIN (8 x 32, marches of twice the rows) 256^2 28.9, 4.4
@@ -108,7 +108,7 @@ LaunchCfg tuned_config(const ptd_params& p)
         switch (p.precision) {
         case PTD_PREC_FP64:
             c.warps2d = 1;
-            c.chunk2d = march_length(32, 16, 52 * sm, 25 * sm / 2, warps(31, 1));
+            c.chunk2d = march_length(16, 8, 52 * sm, 25 * sm / 2, warps(31, 1));
             break;
         case PTD_PREC_DFH:
         case PTD_PREC_DF64:
@@ -129,23 +129,18 @@ LaunchCfg tuned_config(const ptd_params& p)
         c.rows3d = 16;
         c.chunk3d = z_march16(p);
     } else if (p.ndim == 3) {
-        // The FP64-accuracy forms.  512-thread CTAs of 31 x 15 updated cells
-        // (3 resident per SM at <= 40 registers) on large grids; 256-thread
-        // CTAs of 31 x 7 cells, whose per-plane barrier joins half the warps
-        // and whose smaller tiles waste less of a ragged grid, below 288^3
-        // (DFH: at every size).  us per iteration, 16 rows with the former
-        // march / as taken here: FP64 NONLIN 64^3 68.6, 19.4 (8 rows x 4
-        // planes); 128^3 190.4, 148.2 (8 x 4); 256^3 1050, 1001 (8 x 16);
-        // 320^3 1920 (16 x 32), 1883 (16 x 16); 512^3 7299 (16 x 32), 7406
-        // (8 x 32); DF64 LIN 64^3 20.3, 7.5 (8 x 4); 128^3 46.6, 39.4; DFH
-        // NONLIN 128^3 81.1, 62.4; 512^3 2804, 2756 (8 x 32).
-        const bool small = p.precision == PTD_PREC_DFH || (double)p.nx * p.ny * p.nz < 24e6;
-        c.rows3d = small ? 8 : 16;
-        const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, c.rows3d - 1);
+        // The FP64-accuracy forms: 256-thread CTAs of 31 x 7 updated cells.
+        // Their per-plane barrier joins half the warps of 512-thread CTAs (31
+        // x 15 cells) and their tiles waste less of a ragged grid; the larger
+        // halo is not what bounds them.  us per iteration, 16 rows x best
+        // march / as taken: FP64 NONLIN 64^3 17.1, 14.2 (2 planes); 128^3
+        // 95.4, 88.0 (4); 256^3 614, 571 (16); 512^3 4438, 4184 (16); LIN
+        // 512^3 4169, 4190; LINSTEP 512^3 5143, 4593 (32); DF64 LIN 128^3 42.3,
+        // 39.4; 512^3 2144, 2149 (32); DFH 512^3 2804, 2756 (32).
+        c.rows3d = 8;
+        const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, 7);
         auto ctas = [&](int m) { return bxy * ceil_div(p.nz - 2, m); };
-        if (!small) c.chunk3d = ctas(32) >= 40 * sm ? 32 : 16;
-        else if (ctas(32) >= 52 * sm) c.chunk3d = 32;
-        else c.chunk3d = march_length(16, 4, 16 * sm, 4 * sm / 3, ctas);
+        c.chunk3d = ctas(32) >= 52 * sm ? 32 : march_length(16, 4, 16 * sm, 2 * sm, ctas);
     }
     return c;
 }

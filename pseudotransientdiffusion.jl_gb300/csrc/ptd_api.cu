@@ -24,6 +24,7 @@
 
 #include "../../include/ptd.h"
 #include "ptd_internal.h"
+#include "ptd_line.h"
 #include "ptd_num.cuh"
 
 using namespace ptd;
@@ -273,7 +274,9 @@ struct ptd_ctx : ptd_ctx_base {
     int* zero_flag = nullptr;
     double* errhist = nullptr;
     int errcap = 0;
-    DevState* h_st = nullptr;     // pinned mirror of *st
+    DevState* h_st = nullptr;     // pinned mirror of *st (line: written by the kernel, then kLineErr doubles)
+    bool line = false;            // 1D: a step is one launch of the line kernel, in place on H[cur], W[0][cur]
+    LinePlan lplan;
     cudaGraphExec_t gstep[2] = {nullptr, nullptr};   // one physical step's check loop, per start parity
     cudaGraphExec_t gplain[2] = {nullptr, nullptr};
     int blocks_per_pass = 1;      // check blocks in the body of the step graph's loop
@@ -569,7 +572,10 @@ extern "C" int ptd_create(ptd_ctx** out, const ptd_params* p)
     if (!rc) rc = alloc((void**)&c->zero_flag, sizeof(int));
     c->errcap = (p->nchk <= p->itmax ? p->itmax / p->nchk : 0) + 2;
     if (!rc) rc = alloc((void**)&c->errhist, (size_t)c->errcap * sizeof(double));
-    if (!rc && cudaMallocHost((void**)&c->h_st, sizeof(DevState)) != cudaSuccess) {
+    c->line = p->ndim == 1 && p->precision == PTD_PREC_FP64 && p->resid_mode == PTD_RESID_MIXED &&
+              line_plan(p->model, p->nx, p->nchk, c->lplan);
+    if (!rc && cudaMallocHost((void**)&c->h_st, sizeof(DevState) + (c->line ? kLineErr * sizeof(double) : 0)) !=
+                   cudaSuccess) {
         cudaGetLastError();
         rc = fail(PTD_ENOMEM, "cudaMallocHost failed");
     }
@@ -595,7 +601,7 @@ extern "C" int ptd_create(ptd_ctx** out, const ptd_params* p)
             free_ctx(c);
             return rc;
         }
-    } else {
+    } else if (!c->line) {
         if ((p->flags & PTD_FLAG_AUTOTUNE) && p->ndim > 1) rc = autotune(c);
         if (!rc) rc = ensure_parts(c);
         for (int q = 0; q < 2 && !rc; ++q) {
@@ -645,7 +651,7 @@ extern "C" int ptd_set_launch_config(ptd_ctx* c, const int32_t cfg[4])
         rc = dc_set_config(c->dc, k);
     } else if (c->rb) {
         rc = rb_set_config(c->rb, k);
-    } else {
+    } else if (!c->line) {
         rc = ensure_parts(c);
         for (int q = 0; q < 2 && !rc; ++q) {
             if (c->gstep[q]) cudaGraphExecDestroy(c->gstep[q]);
@@ -767,9 +773,44 @@ extern "C" int ptd_get_state(ptd_ctx* c, double* H)
     return PTD_OK;
 }
 
+// One launch of the line kernel: a whole step with its checks, or niter
+// iterations without.
+static int run_line(ptd_ctx* c, bool checks, int niter)
+{
+    PTArgs a;
+    args_for(c, c->cur, c->zero_flag, a);
+    a.Hout = c->H[c->cur];
+    a.wout[0] = c->W[0][c->cur];
+    LineArgs l = {};
+    l.Hold = c->Hold;
+    l.st = c->h_st;
+    l.errhist = reinterpret_cast<double*>(c->h_st + 1);
+    l.errmore = c->errhist;
+    l.errhost = kLineErr;
+    l.errcap = c->errcap;
+    l.nchk = c->p.nchk;
+    l.itmax = c->p.itmax;
+    l.checks = checks;
+    l.niter = niter;
+    l.tol = c->p.tol;
+    l.norm_den = c->dv.norm_den;
+    // err > tol for certain: 1e-10 covers the rounding of either side
+    l.acc_above = c->p.norm == PTD_NORM_MAX ? c->p.tol : c->p.tol * c->p.tol * c->dv.norm_den * (1.0 + 1e-10);
+    CK(launch_line(a, l, c->p.model, c->lplan, c->stream));
+    c->launches += 1;
+    return PTD_OK;
+}
+
 // Run n PT iterations without checks starting from buffer c->cur.
 static int run_plain(ptd_ctx* c, long long n)
 {
+    while (c->line && n > 0) {
+        const int k = (int)std::min<long long>(n, 1 << 20);   // a launch of seconds at most
+        int rc = run_line(c, false, k);
+        if (rc) return rc;
+        c->iterations += k;
+        n -= k;
+    }
     while (n >= c->plain_len) {
         CK(cudaGraphLaunch(c->gplain[c->cur], c->stream));
         c->launches += c->plain_len;
@@ -804,12 +845,25 @@ static int fp64_step(ptd_ctx* c, int32_t* iters, double* err_hist, int32_t err_c
                      int* nan_flag, int* capped)
 {
     const ptd_params& p = c->p;
-    CK(launch_reset_state(c->st, c->stream));
-    c->launches += 1;
     const long long blocks_max = p.nchk <= p.itmax ? p.itmax / p.nchk : 0;
     const int start = c->cur;
     int done = DONE_RUNNING, iter = 0, nchecks = 0;
-    if (blocks_max > 0) {
+    const double* err_host = nullptr;   // the first kLineErr check residuals, on the host already
+    if (c->line) {
+        if (blocks_max > 0) {
+            int rc = run_line(c, true, 0);
+            if (rc) return rc;
+            CK(cudaStreamSynchronize(c->stream));
+            done = c->h_st->done;
+            iter = c->h_st->iter;
+            nchecks = c->h_st->nchecks;
+            err_host = reinterpret_cast<const double*>(c->h_st + 1);
+        }
+    } else {
+        CK(launch_reset_state(c->st, c->stream));
+        c->launches += 1;
+    }
+    if (blocks_max > 0 && !c->line) {
         CK(cudaGraphLaunch(c->gstep[start], c->stream));
         CK(cudaMemcpyAsync(c->h_st, c->st, sizeof(DevState), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -821,7 +875,7 @@ static int fp64_step(ptd_ctx* c, int32_t* iters, double* err_hist, int32_t err_c
         c->launches += passes * c->blocks_per_pass * c->kernels_per_block;
     }
     c->iterations += iter;
-    c->cur = (start + iter) & 1;
+    if (!c->line) c->cur = (start + iter) & 1;
     if (done == DONE_RUNNING || done == DONE_CAP) {
         const long long tail = (long long)p.itmax - iter;
         int rc = run_plain(c, tail);
@@ -834,8 +888,16 @@ static int fp64_step(ptd_ctx* c, int32_t* iters, double* err_hist, int32_t err_c
     CK(cudaMemcpyAsync(c->Hold, c->H[c->cur], bytes, cudaMemcpyDeviceToDevice, c->stream));
     if (err_hist && nchecks > 0 && *n_err < err_cap) {
         const int k = std::min(nchecks, std::min(err_cap - *n_err, c->errcap));
-        CK(cudaMemcpyAsync(err_hist + *n_err, c->errhist, (size_t)k * sizeof(double), cudaMemcpyDeviceToHost,
-                           c->stream));
+        const int kh = err_host ? std::min(k, kLineErr) : 0;
+        double* const dst = err_hist + *n_err;
+        if (kh) std::memcpy(dst, err_host, (size_t)kh * sizeof(double));
+        if (k > kh)
+            CK(cudaMemcpyAsync(dst + kh, c->errhist + kh, (size_t)(k - kh) * sizeof(double), cudaMemcpyDeviceToHost,
+                               c->stream));
+        if (c->line && p.norm != PTD_NORM_MAX) {   // the line kernel's history holds sums of squares
+            if (k > kh) CK(cudaStreamSynchronize(c->stream));
+            for (int i = 0; i < k; ++i) dst[i] = std::sqrt(dst[i]) / std::sqrt(c->dv.norm_den);
+        }
     }
     *n_err += nchecks;
     CK(cudaStreamSynchronize(c->stream));

@@ -134,15 +134,14 @@ __device__ __forceinline__ float fsqrt(float x)
 // (scripts/diff_2D_nonlin.jl:19-25).  D_f -> 0 gives Re_f -> inf, c -> 1.
 __device__ __forceinline__ float nonlin_face_c3(const FParams& a, float df)
 {
-    float re = a.fpi + fsqrt(a.fpi2 + a.fA * frcp(df));
-    float th = a.fk2 * frcp(re);
-    return frcp(1.0f + th);
+    const float re = __fadd_rn(a.fpi, fsqrt(__fmaf_rn(a.fA, frcp(df), a.fpi2)));
+    return frcp(__fmaf_rn(a.fk2, frcp(re), 1.0f));
 }
 
 __device__ __forceinline__ float nonlin_face_c(const FParams& a, float hsum, float efac = 1.0f)
 {
-    float m = 0.5f * hsum;
-    return nonlin_face_c3(a, efac * m * m * m);
+    const float m = __fmul_rn(0.5f, hsum);
+    return nonlin_face_c3(a, __fmul_rn(__fmul_rn(__fmul_rn(efac, m), m), m));
 }
 // (With s^3 = (s*s)*s already formed, 0.125f * s^3 is bit for bit the
 // D_f = m*m*m of m = s/2: scaling by powers of two commutes with rounding.)
@@ -152,9 +151,9 @@ __device__ __forceinline__ float nonlin_face_c(const FParams& a, float hsum, flo
 // (scripts/diff_2D_nonlin.jl:23,26); finite for H^3 -> 0 (e -> dt).
 __device__ __forceinline__ float nonlin_cell_e(const FParams& a, float h, float efac = 1.0f)
 {
-    float h3 = efac * h * h * h;
-    float inv = (a.fpi * h3 + fsqrt(a.fpi2 * h3 * h3 + a.fA * h3)) * a.fk1;
-    return frcp(inv + a.frdt);
+    const float h3 = __fmul_rn(__fmul_rn(__fmul_rn(efac, h), h), h);
+    const float q = __fmaf_rn(__fmul_rn(a.fpi2, h3), h3, __fmul_rn(a.fA, h3));
+    return frcp(__fmaf_rn(__fmaf_rn(a.fpi, h3, fsqrt(q)), a.fk1, a.frdt));
 }
 
 // (NONLIN_EXPM: D = exp(m) H^3 -- efac = exp(m) at the cell, the arithmetic
@@ -187,7 +186,7 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 // scripts/diff_2D_linstep.jl:18-21).
 __device__ __forceinline__ float linstep_cell_e(const FParams& a, float dmax)
 {
-    return frcp(dmax * a.fk3 + a.frdt);
+    return frcp(__fmaf_rn(dmax, a.fk3, a.frdt));
 }
 
 __device__ __forceinline__ double warp_sum(double v)

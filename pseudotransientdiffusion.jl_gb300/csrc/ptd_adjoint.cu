@@ -140,7 +140,8 @@ template <class N, bool EXPM, bool CHECK, int R, bool DELTA = false>
 __global__ void __launch_bounds__(32 * R) adj3d_kernel(const AdjArgs* __restrict__ ap, int chunk)
 {
     using T = typename N::T;
-    const AdjArgs a = *ap;
+    const AdjArgs a = *ap;   // (written by the host before the solve)
+    pdl_begin();
     if (step_done(a.done)) return;
     __shared__ T sL[2][R][32];     // lam of the plane
     __shared__ T sH[2][R][32];     // H of the plane
@@ -365,6 +366,7 @@ __global__ void __launch_bounds__(256) adj_judge_kernel(AdjState* st, const doub
                                                         cudaGraphConditionalHandle loop)
 {
     // every thread reads the flag before thread 0 can change it
+    pdl_begin();
     const bool idle = st->done != 0;
     __syncthreads();
     if (idle) {   // no PT kernel ran: the slots are stale
@@ -558,6 +560,7 @@ __global__ void __launch_bounds__(256) adj_rb_check_judge_kernel(AdjRbState* st,
                                                                  double norm_den, int stall, int phase_cap,
                                                                  cudaGraphConditionalHandle rebase)
 {
+    pdl_begin();
     // every thread reads the flags before thread 0 can change them
     const bool idle = st->skip || st->done;
     __syncthreads();
@@ -749,13 +752,11 @@ cudaError_t adj_launch_rb(ptd_adj* A, int par, bool check)
     const dim3 grid(tx, ty, (A->g.nz - 2 + ch - 1) / ch);
     const AdjArgs* ap = A->d_rbargs[par];
     if (A->expm) {
-        if (check) adj3d_kernel<F32, true, true, 16, true><<<grid, blk, 0, A->s>>>(ap, ch);
-        else adj3d_kernel<F32, true, false, 16, true><<<grid, blk, 0, A->s>>>(ap, ch);
-    } else {
-        if (check) adj3d_kernel<F32, false, true, 16, true><<<grid, blk, 0, A->s>>>(ap, ch);
-        else adj3d_kernel<F32, false, false, 16, true><<<grid, blk, 0, A->s>>>(ap, ch);
+        if (check) return launch_pdl(adj3d_kernel<F32, true, true, 16, true>, grid, blk, A->s, ap, ch);
+        return launch_pdl(adj3d_kernel<F32, true, false, 16, true>, grid, blk, A->s, ap, ch);
     }
-    return cudaGetLastError();
+    if (check) return launch_pdl(adj3d_kernel<F32, false, true, 16, true>, grid, blk, A->s, ap, ch);
+    return launch_pdl(adj3d_kernel<F32, false, false, 16, true>, grid, blk, A->s, ap, ch);
 }
 
 cudaError_t adj_launch(ptd_adj* A, int par, bool check)
@@ -766,8 +767,8 @@ cudaError_t adj_launch(ptd_adj* A, int par, bool check)
     const dim3 grid(tx, ty, (A->g.nz - 2 + ch - 1) / ch);
     const AdjArgs* ap = A->d_args[par];
 #define ADJ(NT, EX)                                                                          \
-    (check ? adj3d_kernel<NT, EX, true, 16><<<grid, blk, 0, A->s>>>(ap, ch)                   \
-           : adj3d_kernel<NT, EX, false, 16><<<grid, blk, 0, A->s>>>(ap, ch))
+    return check ? launch_pdl(adj3d_kernel<NT, EX, true, 16>, grid, blk, A->s, ap, ch)         \
+                 : launch_pdl(adj3d_kernel<NT, EX, false, 16>, grid, blk, A->s, ap, ch)
     if (A->df64) {
         if (A->expm) ADJ(DF64, true);
         else ADJ(DF64, false);
@@ -776,7 +777,6 @@ cudaError_t adj_launch(ptd_adj* A, int par, bool check)
         else ADJ(F64, false);
     }
 #undef ADJ
-    return cudaGetLastError();
 }
 
 void adj_fill(ptd_adj* A, int par, AdjArgs& a)
@@ -929,9 +929,8 @@ int adj_capture_rb(ptd_adj* A)
             par ^= 1;
         }
         if (err == cudaSuccess) {
-            adj_rb_check_judge_kernel<<<1, 256, 0, A->s>>>(A->rbst, A->parts, A->nparts, A->nchk, A->p.itmax,
-                                                           A->dv.norm_den, A->stall, A->phase_iters, rebase);
-            err = cudaGetLastError();
+            err = launch_pdl(adj_rb_check_judge_kernel, 1, 256, A->s, A->rbst, A->parts, A->nparts, A->nchk, A->p.itmax,
+                             A->dv.norm_den, A->stall, A->phase_iters, rebase);
         }
         // the judge is the capture's last node: the IF node follows it
         cudaStreamCaptureStatus cs;
@@ -1005,9 +1004,8 @@ int adj_capture(ptd_adj* A)
             par ^= 1;
         }
         if (err == cudaSuccess) {
-            adj_judge_kernel<<<1, 256, 0, A->s>>>(A->st, A->parts, A->nparts, A->nchk, A->p.itmax, A->dv.norm_den,
-                                                  A->stall, loop);
-            err = cudaGetLastError();
+            err = launch_pdl(adj_judge_kernel, 1, 256, A->s, A->st, A->parts, A->nparts, A->nchk, A->p.itmax,
+                             A->dv.norm_den, A->stall, loop);
         }
     }
     if (err == cudaSuccess) {

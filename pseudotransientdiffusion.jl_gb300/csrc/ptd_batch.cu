@@ -415,6 +415,7 @@ __global__ void __launch_bounds__(256) rb2d_batch_kernel(const RbArgs* __restric
                                                          const int* __restrict__ active, const int* nactive,
                                                          int chunk)
 {
+    pdl_begin();
     if ((int)blockIdx.x >= __ldcg(nactive)) return;
     const int4 w = work[active[blockIdx.x]];
     const RbArgs a = tab[w.x];
@@ -432,16 +433,15 @@ __global__ void __launch_bounds__(256) rb2d_batch_kernel(const RbArgs* __restric
 __global__ void __launch_bounds__(256) compact_active_kernel(const RbDev* st, const int* wfirst, const int* wcount,
                                                              int ninst, int* active, int* nactive)
 {
-    __shared__ int s_off[256];
-    __shared__ int s_base;
-    const int t = threadIdx.x;
-    if (t == 0) s_base = 0;
-    __syncthreads();
+    __shared__ int s_off[256], s_cnt[256];
+    pdl_begin();
+    const int t = threadIdx.x, lane = t & 31;
+    int base = 0;
     for (int i0 = 0; i0 < ninst; i0 += 256) {
         const int i = i0 + t;
         const int c = (i < ninst && !st[i].skip && !st[i].step_done) ? wcount[i] : 0;
         // inclusive scan of the counts over the block
-        s_off[t] = c;
+        s_cnt[t] = s_off[t] = c;
         __syncthreads();
         for (int o = 1; o < 256; o <<= 1) {
             const int v = t >= o ? s_off[t - o] : 0;
@@ -449,13 +449,15 @@ __global__ void __launch_bounds__(256) compact_active_kernel(const RbDev* st, co
             s_off[t] += v;
             __syncthreads();
         }
-        const int start = s_base + s_off[t] - c;
-        for (int q = 0; q < c; ++q) active[start + q] = wfirst[i] + q;
-        __syncthreads();
-        if (t == 255) s_base += s_off[255];
+        // a warp per instance writes its items
+        for (int k = t >> 5; k < 256 && i0 + k < ninst; k += 8) {
+            const int n = s_cnt[k], start = base + s_off[k] - n, first = n ? wfirst[i0 + k] : 0;
+            for (int q = lane; q < n; q += 32) active[start + q] = first + q;
+        }
+        base += s_off[255];
         __syncthreads();
     }
-    if (t == 0) *nactive = s_base;
+    if (t == 0) *nactive = base;
 }
 
 __global__ void rb_reset_batch_kernel(RbDev* st, int ninst)
@@ -471,6 +473,7 @@ __global__ void rb_check_judge_batch_kernel(RbDev* st, int ninst, int nchk, int 
                                             const int* wfirst, const int* wcount, int W)
 {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    pdl_begin();
     if (i >= ninst || st[i].skip || st[i].step_done) return;   // uniform over the warp; no iteration ran
     const double acc = warp_sum_range(parts, (long long)wfirst[i] * W, (long long)wcount[i] * W, norm_max);
     if ((threadIdx.x & 31) == 0) {
@@ -741,21 +744,19 @@ cudaError_t launch_rb_batch(ptd_batch* b, int par, bool check)
 {
     const dim3 blk(32, b->cfg.warps2d);
     const RbArgs* t = b->rbtab[par];
-#define RBK(M, C, T) rb2d_batch_kernel<M, C, T><<<b->nwork, blk, 0, b->s>>>(t, b->work, b->active, b->nactive, b->cfg.chunk2d)
+#define RBK(M, C, T) launch_pdl(rb2d_batch_kernel<M, C, T>, b->nwork, blk, b->s, t, b->work, b->active, b->nactive, b->cfg.chunk2d)
 #define RBB(M) (b->tb == 2 ? (check ? RBK(M, true, 2) : RBK(M, false, 2)) : (check ? RBK(M, true, 1) : RBK(M, false, 1)))
-    if (b->model == LIN) RBB(LIN);
-    else if (b->model == LINSTEP) RBB(LINSTEP);
-    else RBB(NONLIN);
+    if (b->model == LIN) return RBB(LIN);
+    if (b->model == LINSTEP) return RBB(LINSTEP);
+    return RBB(NONLIN);
 #undef RBB
 #undef RBK
-    return cudaGetLastError();
 }
 
 // The list of the running instances' work items (after every judge).
 cudaError_t compact_rb(ptd_batch* b)
 {
-    compact_active_kernel<<<1, 256, 0, b->s>>>(b->rdev, b->wfirst, b->wcount, b->ninst, b->active, b->nactive);
-    return cudaGetLastError();
+    return launch_pdl(compact_active_kernel, 1, 256, b->s, b->rdev, b->wfirst, b->wcount, b->ninst, b->active, b->nactive);
 }
 
 void build_work(ptd_batch* b, std::vector<int4>& work)
@@ -840,10 +841,8 @@ int capture_rb(ptd_batch* b)
             ++nk;
         }
         if (err == cudaSuccess) {
-            rb_check_judge_batch_kernel<<<nb, 128, 0, b->s>>>(b->rdev, n, b->nchk, b->bp.itmax, b->bp.tol,
-                                                              b->norm_den, b->bp.norm == PTD_NORM_MAX, b->parts,
-                                                              b->wfirst, b->wcount, b->cfg.warps2d);
-            err = cudaGetLastError();
+            err = launch_pdl(rb_check_judge_batch_kernel, nb, 128, b->s, b->rdev, n, b->nchk, b->bp.itmax, b->bp.tol,
+                             b->norm_den, b->bp.norm == PTD_NORM_MAX, b->parts, b->wfirst, b->wcount, b->cfg.warps2d);
             ++nk;
         }
         if (err == cudaSuccess) {

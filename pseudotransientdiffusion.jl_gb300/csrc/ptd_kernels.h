@@ -40,6 +40,23 @@ enum { NUM_F64 = 0, NUM_DF64 = 1, NUM_DFH = 2 };
 int sm_count();
 inline int fill_blocks() { return 8 * sm_count(); }
 
+// Launch of a kernel that begins with pdl_begin(): its scheduling overlaps the
+// end of the previous kernel of the stream.
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
 cudaError_t launch_pt(const PTArgs& a, int ndim, int model, bool check, int num, const LaunchCfg& cfg,
                       cudaStream_t s);
 cudaError_t launch_resid_consistent(const PTArgs& a, int ndim, int model, int num, cudaStream_t s);

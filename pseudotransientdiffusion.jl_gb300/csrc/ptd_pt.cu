@@ -32,6 +32,7 @@ namespace ptd {
 template <class N, int MODEL, bool CHECK>
 __global__ void __launch_bounds__(256) pt1d_kernel(PTArgs a)
 {
+    pdl_begin();
     if (step_done(a.done)) return;
     double part = 0.0;
     unsigned long long pmax = 0ull;
@@ -42,6 +43,7 @@ __global__ void __launch_bounds__(256) pt1d_kernel(PTArgs a)
 template <class N, int MODEL, bool CHECK>
 __global__ void __launch_bounds__(256, CHECK ? 4 : 6) pt2d_kernel(PTArgs a, int chunk)
 {
+    pdl_begin();
     if (step_done(a.done)) return;
     double part = 0.0;
     unsigned long long pmax = 0ull;
@@ -59,6 +61,7 @@ template <class N, int MODEL, bool CHECK, int R>
 __global__ void __launch_bounds__(32 * R, (CHECK || MODEL == LINSTEP || MODEL == NONLIN_EXPM) ? 32 / R : 48 / R)
     pt3d_kernel(PTArgs a, int chunk)
 {
+    pdl_begin();
     if (step_done(a.done)) return;
     double part = 0.0;
     unsigned long long pmax = 0ull;
@@ -75,6 +78,7 @@ __global__ void __launch_bounds__(32 * R, (CHECK || MODEL == LINSTEP || MODEL ==
 template <class N, int MODEL, bool CHECK>
 __global__ void __launch_bounds__(256) pt2d_pair_kernel(PTArgs a, int chunk)
 {
+    pdl_begin();
     if (step_done(a.done)) return;
     double part = 0.0;
     unsigned long long pmax = 0ull;
@@ -174,6 +178,7 @@ __global__ void __launch_bounds__(256) judge_parts_kernel(DevState* st, const do
                                                           double* errhist, int errcap, int nchk, int itmax, double tol,
                                                           double norm_den, int norm_max, cudaGraphConditionalHandle loop)
 {
+    pdl_begin();
     __shared__ double s_sum[256];
     __shared__ unsigned long long s_max[256];
     const int t = threadIdx.x;
@@ -255,35 +260,32 @@ static cudaError_t launch_model(const PTArgs& a, int ndim, const LaunchCfg& cfg,
 {
     if (ndim == 1) {
         const int bs = 256;
-        pt1d_kernel<N, MODEL, CHECK><<<(a.nx + bs - 1) / bs, bs, 0, s>>>(a);
-        return cudaGetLastError();
+        return launch_pdl(pt1d_kernel<N, MODEL, CHECK>, (a.nx + bs - 1) / bs, bs, s, a);
     }
     if constexpr (!N::native) {
         if (ndim == 2) {
             const int W = cfg.warps2d;
             const int tiles = (a.nx - 2 + 61) / 62;
             dim3 grid((tiles + W - 1) / W, (a.ny - 2 + cfg.chunk2d - 1) / cfg.chunk2d);
-            pt2d_pair_kernel<N, MODEL, CHECK><<<grid, dim3(32, W), 0, s>>>(a, cfg.chunk2d);
-            return cudaGetLastError();
+            return launch_pdl(pt2d_pair_kernel<N, MODEL, CHECK>, grid, dim3(32, W), s, a, cfg.chunk2d);
         }
     }
     if (ndim == 2) {
         const int W = cfg.warps2d;
         const int tiles = (a.nx - 2 + 30) / 31;
         dim3 grid((tiles + W - 1) / W, (a.ny - 2 + cfg.chunk2d - 1) / cfg.chunk2d);
-        pt2d_kernel<N, MODEL, CHECK><<<grid, dim3(32, W), 0, s>>>(a, cfg.chunk2d);
+        return launch_pdl(pt2d_kernel<N, MODEL, CHECK>, grid, dim3(32, W), s, a, cfg.chunk2d);
     } else {
         const int tx = (a.nx - 2 + 30) / 31;
         const int nzc = (a.nz - 2 + cfg.chunk3d - 1) / cfg.chunk3d;
         if (cfg.rows3d == 8) {
             dim3 grid(tx, (a.ny - 2 + 6) / 7, nzc);
-            pt3d_kernel<N, MODEL, CHECK, 8><<<grid, dim3(32, 8), 0, s>>>(a, cfg.chunk3d);
+            return launch_pdl(pt3d_kernel<N, MODEL, CHECK, 8>, grid, dim3(32, 8), s, a, cfg.chunk3d);
         } else {
             dim3 grid(tx, (a.ny - 2 + 14) / 15, nzc);
-            pt3d_kernel<N, MODEL, CHECK, 16><<<grid, dim3(32, 16), 0, s>>>(a, cfg.chunk3d);
+            return launch_pdl(pt3d_kernel<N, MODEL, CHECK, 16>, grid, dim3(32, 16), s, a, cfg.chunk3d);
         }
     }
-    return cudaGetLastError();
 }
 
 template <class N>
@@ -360,9 +362,8 @@ cudaError_t launch_judge_parts(DevState* st, const double* parts, long long npar
                                int nchk, int itmax, double tol, double norm_den, int norm_max,
                                cudaGraphConditionalHandle loop, cudaStream_t s)
 {
-    judge_parts_kernel<<<1, 256, 0, s>>>(st, parts, nparts, errhist, errcap, nchk, itmax, tol, norm_den, norm_max,
-                                         loop);
-    return cudaGetLastError();
+    return launch_pdl(judge_parts_kernel, 1, 256, s, st, parts, nparts, errhist, errcap, nchk, itmax, tol, norm_den,
+                      norm_max, loop);
 }
 
 // The number of check-residual slots the fused kernel of a check iteration

@@ -14,6 +14,7 @@ namespace ptd {
 template <int MODEL, bool CHECK>
 __global__ void __launch_bounds__(256) rb1d_kernel(RbArgs a)
 {
+    pdl_begin();
     if (rb_skip(a.skip)) return;
     float part = 0.0f;
     unsigned pmax = 0u;
@@ -24,6 +25,7 @@ __global__ void __launch_bounds__(256) rb1d_kernel(RbArgs a)
 template <int MODEL, bool CHECK>
 __global__ void __launch_bounds__(256) rb2d_kernel(RbArgs a, int chunk)
 {
+    pdl_begin();
     if (rb_skip(a.skip)) return;
     float part = 0.0f;
     unsigned pmax = 0u;
@@ -35,6 +37,7 @@ __global__ void __launch_bounds__(256) rb2d_kernel(RbArgs a, int chunk)
 template <int MODEL, bool CHECK>
 __global__ void __launch_bounds__(256) rb2d_tb2_pair_kernel(RbArgs a, int chunk)
 {
+    pdl_begin();
     if (rb_skip(a.skip)) return;
     float part = 0.0f;
     unsigned pmax = 0u;
@@ -51,6 +54,7 @@ __global__ void __launch_bounds__(256) rb2d_tb2_pair_kernel(RbArgs a, int chunk)
 template <int MODEL, bool CHECK>
 __global__ void __launch_bounds__(256, (MODEL == NONLIN && !CHECK) ? 8 : 0) rb2d_tb2_kernel(RbArgs a, int chunk)
 {
+    pdl_begin();
     if (rb_skip(a.skip)) return;
     float part = 0.0f;
     unsigned pmax = 0u;
@@ -62,6 +66,7 @@ __global__ void __launch_bounds__(256, (MODEL == NONLIN && !CHECK) ? 8 : 0) rb2d
 template <int MODEL, bool CHECK>
 __global__ void __launch_bounds__(512, 2) rb3d_tb2_kernel(RbArgs a, int chunk)
 {
+    pdl_begin();
     if (rb_skip(a.skip)) return;
     double part = 0.0;
     unsigned long long pmax = 0ull;
@@ -76,6 +81,7 @@ __global__ void __launch_bounds__(512, 2) rb3d_tb2_kernel(RbArgs a, int chunk)
 template <int MODEL, bool CHECK>
 __global__ void __launch_bounds__(512) rb3d_kernel(RbArgs a, int chunk)
 {
+    pdl_begin();
     if (rb_skip(a.skip)) return;
     double part = 0.0;
     unsigned long long pmax = 0ull;
@@ -200,6 +206,7 @@ __global__ void __launch_bounds__(256) rb_check_judge_kernel(RbDev* st, const do
                                                              double tol, double norm_den, int norm_max,
                                                              int phase_cap, cudaGraphConditionalHandle rebase)
 {
+    pdl_begin();
     // every thread reads the flags before thread 0 can change them
     const bool idle = st->skip || st->step_done;
     __syncthreads();
@@ -343,7 +350,7 @@ template <int MODEL, bool CHECK>
 cudaError_t rb_launch_model(const RbArgs& a, int ndim, const LaunchCfg& cfg, cudaStream_t s, int tb)
 {
     if (ndim == 1) {
-        rb1d_kernel<MODEL, CHECK><<<(a.nx + 255) / 256, 256, 0, s>>>(a);
+        return launch_pdl(rb1d_kernel<MODEL, CHECK>, (a.nx + 255) / 256, 256, s, a);
     } else if (ndim == 2 && tb == 2) {
         // twice the configured rows per y march: the march starts with two
         // extra level-1 rows (4096^2 nonlinear, 2 warps: 87.2 us per
@@ -352,29 +359,28 @@ cudaError_t rb_launch_model(const RbArgs& a, int ndim, const LaunchCfg& cfg, cud
         if (MODEL == LIN || MODEL == NONLIN) {   // two columns per lane, 60 per warp
             const int tiles = (a.nx - 1 + 59) / 60;
             dim3 grid((tiles + W - 1) / W, (a.ny - 2 + chunk - 1) / chunk);
-            rb2d_tb2_pair_kernel<MODEL, CHECK><<<grid, dim3(32, W), 0, s>>>(a, chunk);
+            return launch_pdl(rb2d_tb2_pair_kernel<MODEL, CHECK>, grid, dim3(32, W), s, a, chunk);
         } else {
             const int tiles = (a.nx - 2 + 27) / 28;
             dim3 grid((tiles + W - 1) / W, (a.ny - 2 + chunk - 1) / chunk);
-            rb2d_tb2_kernel<MODEL, CHECK><<<grid, dim3(32, W), 0, s>>>(a, chunk);
+            return launch_pdl(rb2d_tb2_kernel<MODEL, CHECK>, grid, dim3(32, W), s, a, chunk);
         }
     } else if (ndim == 2) {
         const int W = cfg.warps2d;
         const int tiles = (a.nx - 2 + 30) / 31;
         dim3 grid((tiles + W - 1) / W, (a.ny - 2 + cfg.chunk2d - 1) / cfg.chunk2d);
-        rb2d_kernel<MODEL, CHECK><<<grid, dim3(32, W), 0, s>>>(a, cfg.chunk2d);
+        return launch_pdl(rb2d_kernel<MODEL, CHECK>, grid, dim3(32, W), s, a, cfg.chunk2d);
     } else if (tb == 2) {
         // 28 x 12 level-2 cells per 16-warp CTA; the z march runs two planes
         // more than its chunk (the level-1 start)
         const int chunk = cfg.chunk3d;
         dim3 grid((a.nx - 2 + 27) / 28, (a.ny - 2 + 11) / 12, (a.nz - 2 + chunk - 1) / chunk);
-        rb3d_tb2_kernel<MODEL, CHECK><<<grid, dim3(32, 16), 0, s>>>(a, chunk);
+        return launch_pdl(rb3d_tb2_kernel<MODEL, CHECK>, grid, dim3(32, 16), s, a, chunk);
     } else {
         const int tx = (a.nx - 2 + 30) / 31;
         dim3 grid(tx, (a.ny - 2 + 14) / 15, (a.nz - 2 + cfg.chunk3d - 1) / cfg.chunk3d);
-        rb3d_kernel<MODEL, CHECK><<<grid, dim3(32, 16), 0, s>>>(a, cfg.chunk3d);
+        return launch_pdl(rb3d_kernel<MODEL, CHECK>, grid, dim3(32, 16), s, a, cfg.chunk3d);
     }
-    return cudaGetLastError();
 }
 
 // One launch of tb PT iterations (tb = 2: 2D; 3D LIN and NONLIN).
@@ -569,10 +575,9 @@ int rb_capture(RbState* rb)
             par ^= 1;
         }
         if (err == cudaSuccess) {
-            rb_check_judge_kernel<<<1, 256, 0, rb->s>>>(rb->dev, rb->parts, rb->nparts, rb->errhist, rb->errcap, nchk,
-                                                        rb->p.itmax, rb->p.tol, rb->dv.norm_den,
-                                                        rb->p.norm == PTD_NORM_MAX, rb->phase_iters, rebase);
-            err = cudaGetLastError();
+            err = launch_pdl(rb_check_judge_kernel, 1, 256, rb->s, rb->dev, rb->parts, rb->nparts, rb->errhist,
+                             rb->errcap, nchk, rb->p.itmax, rb->p.tol, rb->dv.norm_den, rb->p.norm == PTD_NORM_MAX,
+                             rb->phase_iters, rebase);
         }
         // the judge is the capture's last node: the IF node follows it
         cudaStreamCaptureStatus cs;

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "../../include/ptd.h"
+#include "ptd_flow.h"
 #include "ptd_internal.h"
 #include "ptd_line.h"
 #include "ptd_num.cuh"
@@ -274,9 +275,12 @@ struct ptd_ctx : ptd_ctx_base {
     int* zero_flag = nullptr;
     double* errhist = nullptr;
     int errcap = 0;
-    DevState* h_st = nullptr;     // pinned mirror of *st (line: written by the kernel, then kLineErr doubles)
+    DevState* h_st = nullptr;     // pinned mirror of *st (line, flow: written by the kernel, then kHostErr doubles)
     bool line = false;            // 1D: a step is one launch of the line kernel, in place on H[cur], W[0][cur]
     LinePlan lplan;
+    FlowPlan flow;                // 2D FP64: a step is one launch of the flow kernel (rows > 0)
+    void* flow_mem = nullptr;     // its exchange buffers
+    unsigned flow_tag = 1;        // tags used so far
     cudaGraphExec_t gstep[2] = {nullptr, nullptr};   // one physical step's check loop, per start parity
     cudaGraphExec_t gplain[2] = {nullptr, nullptr};
     int blocks_per_pass = 1;      // check blocks in the body of the step graph's loop
@@ -292,6 +296,8 @@ struct ptd_ctx : ptd_ctx_base {
     int num = NUM_F64;            // number type of the PT kernels
     double* stage = nullptr;      // DF64: FP64 staging field for the host boundary
 };
+
+constexpr int kHostErr = 1024;    // check residuals that the line and flow kernels leave in pinned memory
 
 static void args_for(const ptd_ctx* c, int parity, const int* done, PTArgs& a)
 {
@@ -520,6 +526,7 @@ static void free_ctx(ptd_ctx* c)
     cudaFree(c->zero_flag);
     cudaFree(c->errhist);
     cudaFree(c->stage);
+    cudaFree(c->flow_mem);
     if (c->h_st) cudaFreeHost(c->h_st);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -574,7 +581,11 @@ extern "C" int ptd_create(ptd_ctx** out, const ptd_params* p)
     if (!rc) rc = alloc((void**)&c->errhist, (size_t)c->errcap * sizeof(double));
     c->line = p->ndim == 1 && p->precision == PTD_PREC_FP64 && p->resid_mode == PTD_RESID_MIXED &&
               line_plan(p->model, p->nx, p->nchk, c->lplan);
-    if (!rc && cudaMallocHost((void**)&c->h_st, sizeof(DevState) + (c->line ? kLineErr * sizeof(double) : 0)) !=
+    if (p->ndim == 2 && p->precision == PTD_PREC_FP64 && p->resid_mode == PTD_RESID_MIXED &&
+        !(p->flags & PTD_FLAG_AUTOTUNE))
+        flow_plan(p->model, p->nx, p->ny, c->flow);
+    if (!rc && c->flow.rows) rc = alloc(&c->flow_mem, flow_bytes(c->flow));
+    if (!rc && cudaMallocHost((void**)&c->h_st, sizeof(DevState) + (c->line || c->flow.rows ? kHostErr * sizeof(double) : 0)) !=
                    cudaSuccess) {
         cudaGetLastError();
         rc = fail(PTD_ENOMEM, "cudaMallocHost failed");
@@ -583,8 +594,10 @@ extern "C" int ptd_create(ptd_ctx** out, const ptd_params* p)
         free_ctx(c);
         return rc;
     }
+    std::memset(c->h_st, 0, sizeof(DevState));
     e = cudaMemsetAsync(c->zero_flag, 0, sizeof(int), c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->st, 0, sizeof(DevState), c->stream);
+    if (e == cudaSuccess && c->flow_mem) e = cudaMemsetAsync(c->flow_mem, 0, flow_bytes(c->flow), c->stream);
     if (e != cudaSuccess) {
         free_ctx(c);
         return cuda_fail(e, "cudaMemsetAsync");
@@ -601,7 +614,7 @@ extern "C" int ptd_create(ptd_ctx** out, const ptd_params* p)
             free_ctx(c);
             return rc;
         }
-    } else if (!c->line) {
+    } else if (!c->line && !c->flow.rows) {
         if ((p->flags & PTD_FLAG_AUTOTUNE) && p->ndim > 1) rc = autotune(c);
         if (!rc) rc = ensure_parts(c);
         for (int q = 0; q < 2 && !rc; ++q) {
@@ -646,6 +659,7 @@ extern "C" int ptd_set_launch_config(ptd_ctx* c, const int32_t cfg[4])
     k.chunk3d = cfg[3];
     CK(cudaStreamSynchronize(c->stream));
     c->cfg = k;
+    c->flow = FlowPlan();   // the shape is one of the kernel of one iteration per launch
     int rc = PTD_OK;
     if (c->dc) {
         rc = dc_set_config(c->dc, k);
@@ -665,11 +679,18 @@ extern "C" int ptd_set_launch_config(ptd_ctx* c, const int32_t cfg[4])
     return rc;
 }
 
+// After a wait for the stream: whether a wait of a flow launch gave up.
+static int flow_state(const ptd_ctx* c)
+{
+    if (c->flow.rows && c->h_st->pad) return fail(PTD_ETIMEOUT, "a wait of the one-launch step gave up");
+    return PTD_OK;
+}
+
 extern "C" int ptd_sync(ptd_ctx* c)
 {
     if (!c) return fail(PTD_EINVAL, "ctx is NULL");
     CK(cudaStreamSynchronize(c->stream));
-    return PTD_OK;
+    return flow_state(c);
 }
 
 extern "C" int ptd_counters(ptd_ctx* c, int64_t* launches, int64_t* iters)
@@ -770,7 +791,7 @@ extern "C" int ptd_get_state(ptd_ctx* c, double* H)
     int rc = copy_field_out(*c, H, src, c->stream);
     if (rc) return rc;
     CK(cudaStreamSynchronize(c->stream));
-    return PTD_OK;
+    return flow_state(c);
 }
 
 // One launch of the line kernel: a whole step with its checks, or niter
@@ -786,7 +807,7 @@ static int run_line(ptd_ctx* c, bool checks, int niter)
     l.st = c->h_st;
     l.errhist = reinterpret_cast<double*>(c->h_st + 1);
     l.errmore = c->errhist;
-    l.errhost = kLineErr;
+    l.errhost = kHostErr;
     l.errcap = c->errcap;
     l.nchk = c->p.nchk;
     l.itmax = c->p.itmax;
@@ -801,6 +822,35 @@ static int run_line(ptd_ctx* c, bool checks, int niter)
     return PTD_OK;
 }
 
+// One launch of the flow kernel: a whole step with its checks, or niter
+// iterations without.
+static int run_flow(ptd_ctx* c, bool checks, int niter)
+{
+    if (c->flow_tag > 1u << 30) {   // long before tags come round
+        CK(cudaMemsetAsync(c->flow_mem, 0, flow_bytes(c->flow), c->stream));
+        c->flow_tag = 1;
+    }
+    PTArgs a;
+    args_for(c, c->cur, c->zero_flag, a);
+    FlowArgs f = {};
+    flow_buffers(c->flow, c->flow_mem, f);
+    f.st = c->h_st;
+    f.errhist = reinterpret_cast<double*>(c->h_st + 1);
+    f.errmore = c->errhist;
+    f.errhost = kHostErr;
+    f.errcap = c->errcap;
+    f.base = c->flow_tag;
+    f.nchk = c->p.nchk;
+    f.itmax = c->p.itmax;
+    f.checks = checks;
+    f.niter = niter;
+    f.tol = c->p.tol;
+    f.norm_den = c->dv.norm_den;
+    CK(launch_flow(a, f, c->p.model, c->flow, c->stream));
+    c->launches += 1;
+    return PTD_OK;
+}
+
 // Run n PT iterations without checks starting from buffer c->cur.
 static int run_plain(ptd_ctx* c, long long n)
 {
@@ -808,6 +858,15 @@ static int run_plain(ptd_ctx* c, long long n)
         const int k = (int)std::min<long long>(n, 1 << 20);   // a launch of seconds at most
         int rc = run_line(c, false, k);
         if (rc) return rc;
+        c->iterations += k;
+        n -= k;
+    }
+    while (c->flow.rows && n > 0) {
+        const int k = (int)std::min<long long>(n, 1 << 18);
+        int rc = run_flow(c, false, k);
+        if (rc) return rc;
+        c->flow_tag += k + 2;
+        c->cur ^= 1;
         c->iterations += k;
         n -= k;
     }
@@ -848,7 +907,7 @@ static int fp64_step(ptd_ctx* c, int32_t* iters, double* err_hist, int32_t err_c
     const long long blocks_max = p.nchk <= p.itmax ? p.itmax / p.nchk : 0;
     const int start = c->cur;
     int done = DONE_RUNNING, iter = 0, nchecks = 0;
-    const double* err_host = nullptr;   // the first kLineErr check residuals, on the host already
+    const double* err_host = nullptr;   // the first kHostErr check residuals, on the host already
     if (c->line) {
         if (blocks_max > 0) {
             int rc = run_line(c, true, 0);
@@ -859,11 +918,27 @@ static int fp64_step(ptd_ctx* c, int32_t* iters, double* err_hist, int32_t err_c
             nchecks = c->h_st->nchecks;
             err_host = reinterpret_cast<const double*>(c->h_st + 1);
         }
+    } else if (c->flow.rows) {
+        if (blocks_max > 0) {
+            c->h_st->done = DONE_RUNNING;
+            int rc = run_flow(c, true, 0);
+            if (rc) return rc;
+            CK(cudaStreamSynchronize(c->stream));
+            done = c->h_st->done;
+            iter = c->h_st->iter;
+            nchecks = c->h_st->nchecks;
+            err_host = reinterpret_cast<const double*>(c->h_st + 1);
+            // the warps run on until the decision reaches them, three blocks at most
+            c->flow_tag += (unsigned)iter + 3u * (unsigned)p.nchk + 2u;
+            if (done == FLOW_TIMEOUT || done == DONE_RUNNING) c->h_st->pad = 1;
+            rc = flow_state(c);
+            if (rc) return rc;
+        }
     } else {
         CK(launch_reset_state(c->st, c->stream));
         c->launches += 1;
     }
-    if (blocks_max > 0 && !c->line) {
+    if (blocks_max > 0 && !c->line && !c->flow.rows) {
         CK(cudaGraphLaunch(c->gstep[start], c->stream));
         CK(cudaMemcpyAsync(c->h_st, c->st, sizeof(DevState), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -875,7 +950,8 @@ static int fp64_step(ptd_ctx* c, int32_t* iters, double* err_hist, int32_t err_c
         c->launches += passes * c->blocks_per_pass * c->kernels_per_block;
     }
     c->iterations += iter;
-    if (!c->line) c->cur = (start + iter) & 1;
+    if (c->flow.rows) c->cur = (start + nchecks) & 1;   // one snapshot per check, in alternating buffers
+    else if (!c->line) c->cur = (start + iter) & 1;
     if (done == DONE_RUNNING || done == DONE_CAP) {
         const long long tail = (long long)p.itmax - iter;
         int rc = run_plain(c, tail);
@@ -888,7 +964,7 @@ static int fp64_step(ptd_ctx* c, int32_t* iters, double* err_hist, int32_t err_c
     CK(cudaMemcpyAsync(c->Hold, c->H[c->cur], bytes, cudaMemcpyDeviceToDevice, c->stream));
     if (err_hist && nchecks > 0 && *n_err < err_cap) {
         const int k = std::min(nchecks, std::min(err_cap - *n_err, c->errcap));
-        const int kh = err_host ? std::min(k, kLineErr) : 0;
+        const int kh = err_host ? std::min(k, kHostErr) : 0;
         double* const dst = err_hist + *n_err;
         if (kh) std::memcpy(dst, err_host, (size_t)kh * sizeof(double));
         if (k > kh)

@@ -32,6 +32,7 @@ namespace ptd {
 namespace {
 
 constexpr int kMaxWarps = 8;     // warps per CTA (13824 cells in all; at 16384 one launch per iteration is as fast)
+constexpr int kErr = 1024;       // errhost at most (shared memory of a launch)
 constexpr int kMaxCluster = 16;  // CTAs (above 8 the size is not portable: granted by kernel attribute)
 
 // One cell window of a warp: C consecutive cells per lane.
@@ -223,7 +224,7 @@ cudaLaunchConfig_t launch_of(const LinePlan& p, cudaStream_t s, cudaLaunchAttrib
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.ctas);
     cfg.blockDim = dim3(32, p.warps);
-    cfg.dynamicSmemBytes = (size_t)(4 * p.warps * p.core + 2 * kMaxWarps + kLineErr) * sizeof(double);
+    cfg.dynamicSmemBytes = (size_t)(4 * p.warps * p.core + 2 * kMaxWarps + kErr) * sizeof(double);
     cfg.stream = s;
     at->id = cudaLaunchAttributeClusterDimension;
     at->val.clusterDim.x = p.ctas;
@@ -282,6 +283,7 @@ cudaError_t launch_line(const PTArgs& a, const LineArgs& l, int model, const Lin
     la.tmax = p.tmax;
     la.core = p.core;
     la.warps = p.warps;
+    la.errhost = std::min(l.errhost, kErr);
     void* args[] = {&pa, &la};
     return cudaLaunchKernelExC(&cfg, line_kernel(model, p.c), args);
 }

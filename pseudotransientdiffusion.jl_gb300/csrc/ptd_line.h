@@ -7,8 +7,6 @@
 
 namespace ptd {
 
-constexpr int kLineErr = 1024;   // check residuals a step leaves in host-visible memory
-
 // A launch: `ctas` CTAs of `warps` warps, one cluster; windows of 32 c cells
 // per warp of which `core` are written back after at most `tmax` iterations.
 struct LinePlan {

@@ -1062,7 +1062,7 @@ int fill_tables_rb(ptd_batch* b)
                 a.wout[d] = b->w32[dd][q ^ 1] + o;
                 a.tb[d] = b->tb32[dd] + o;
             }
-            a.Rb = b->Rb32 + o;
+            a.Rb = b->Rb32 ? b->Rb32 + o : nullptr;
             a.Cb = b->Cb32 + o;
             a.Hf = b->Hf + o;
             a.Df = b->Df ? b->Df + o : nullptr;
@@ -1082,6 +1082,7 @@ int fill_tables_rb(ptd_batch* b)
             f.wb[d] = b->wb64[d] + o;
             f.w[d][0] = b->w32[d][0] + o;
             f.w[d][1] = b->w32[d][1] + o;
+            f.tb[d] = rb_qform(b->model, 2) ? b->tb32[d] + o : nullptr;
         }
         RbBaseArgs& g = bt[i];
         std::memset(&g, 0, sizeof(g));
@@ -1099,9 +1100,10 @@ int fill_tables_rb(ptd_batch* b)
         for (int d = 0; d < 2; ++d) {
             g.wb[d] = b->wb64[d] + o;
             g.tb[d] = b->tb32[d] + o;
+            for (int q = 0; q < 2; ++q) g.q[d][q] = rb_qform(b->model, 2) ? b->w32[d][q] + o : nullptr;
         }
         g.D = b->D64 ? b->D64 + o : nullptr;
-        g.Rb = b->Rb32 + o;
+        g.Rb = b->Rb32 ? b->Rb32 + o : nullptr;
         g.Cb = b->Cb32 + o;
         g.Hf = b->Hf + o;
         g.acc64 = &b->rdev[i].acc64;
@@ -1438,7 +1440,7 @@ extern "C" int ptd_batch_create(ptd_batch** out, const ptd_batch_params* p, cons
             if (!rc) rc = balloc(&b->wb64[d], db);
             if (!rc) rc = balloc(&b->tb32[d], fb);
         }
-        if (!rc) rc = balloc(&b->Rb32, fb);
+        if (!rc && !rb_qform(p->model, 2)) rc = balloc(&b->Rb32, fb);
         if (!rc) rc = balloc(&b->Cb32, fb);
         if (!rc) rc = balloc(&b->rdev, n * sizeof(RbDev));
         for (int q = 0; q < 2 && !rc; ++q) rc = balloc(&b->rbtab[q], n * sizeof(RbArgs));
@@ -1454,7 +1456,7 @@ extern "C" int ptd_batch_create(ptd_batch** out, const ptd_batch_params* p, cons
             // faces past the last one of each direction are read (never used) by the halo lanes
             float* zf[] = {b->tb32[0], b->tb32[1], b->Rb32, b->Cb32};
             for (float* z : zf)
-                if (cudaMemset(z, 0, fb) != cudaSuccess) rc = bfail(PTD_ECUDA, "batch: cudaMemset failed");
+                if (z && cudaMemset(z, 0, fb) != cudaSuccess) rc = bfail(PTD_ECUDA, "batch: cudaMemset failed");
             if (cudaMemset(b->rdev, 0, n * sizeof(RbDev)) != cudaSuccess)
                 rc = bfail(PTD_ECUDA, "batch: cudaMemset failed");
         }

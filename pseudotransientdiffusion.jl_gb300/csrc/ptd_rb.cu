@@ -162,30 +162,27 @@ __global__ void __launch_bounds__(256) rb_base_march_kernel(RbBaseArgs b, const 
             if (own) {
                 b.Hf[c] = __double2float_rn(b.H[c]);
                 const int dm = NDIM - 1;   // the march direction's index
-                if (ixc <= b.nx - 2) b.tb[0][c] = (float)(b.wb[0][c] + ur);
-                if (k <= nm - 2) b.tb[dm][c] = (float)(b.wb[dm][c] + uup);
+                if (ixc <= b.nx - 2) rb_base_face(b, 0, c, ur);
+                if (k <= nm - 2) rb_base_face(b, dm, c, uup);
                 double uyr = 0.0;
                 if (NDIM == 3 && iy <= b.ny - 2) {
                     uyr = rb_u64(b, c, c + b.sy);
-                    b.tb[1][c] = (float)(b.wb[1][c] + uyr);
+                    rb_base_face(b, 1, c, uyr);
                 }
                 if (inner) {
                     // the order of rb_base_cell: x, y, z
-                    double divw = 0.0, divu = 0.0;
-                    divw = fma(b.wb[0][c] - b.wb[0][c - 1], b.sig[0], divw);
-                    divu = fma(ur - ul, b.sig[0], divu);
-                    if (NDIM == 3) {
-                        const double uyl = rb_u64(b, c - b.sy, c);
-                        divw = fma(b.wb[1][c] - b.wb[1][c - b.sy], b.sig[1], divw);
-                        divu = fma(uyr - uyl, b.sig[1], divu);
-                    }
-                    divw = fma(b.wb[dm][c] - b.wb[dm][c - sm], b.sig[dm], divw);
+                    double divu = fma(ur - ul, b.sig[0], 0.0);
+                    if (NDIM == 3) divu = fma(uyr - rb_u64(b, c - b.sy, c), b.sig[1], divu);
                     divu = fma(uup - udn, b.sig[dm], divu);
                     const double dh = (b.H[c] - b.Hold[c]) * b.rdt;
-                    b.Rb[c] = (float)(dh + divw);
+                    if (NDIM == 2 && b.Rb) {
+                        double divw = fma(b.wb[0][c] - b.wb[0][c - 1], b.sig[0], 0.0);
+                        divw = fma(b.wb[dm][c] - b.wb[dm][c - sm], b.sig[dm], divw);
+                        b.Rb[c] = (float)(dh + divw);
+                    }
                     const double cb = divu - dh;
+                    b.Cb[c] = (float)cb;
                     if (NDIM == 3) b.Cb64[c] = cb;
-                    else b.Cb[c] = (float)cb;
                     accumulate_residual(cb, part, pmax);
                 }
             }
@@ -280,8 +277,9 @@ struct RbState {
     float* d[2] = {nullptr, nullptr};
     float* w[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
     float* tb[3] = {nullptr, nullptr, nullptr};
-    float* Rb = nullptr;
-    float* Cb = nullptr;                          // base check residual (1D, 2D: FP32)
+    bool q = false;                               // carries the flux defect (rb_qform)
+    float* Rb = nullptr;                          // not in the q form
+    float* Cb = nullptr;                          // base check residual, FP32
     double* Cb64 = nullptr;                       // base check residual (3D: FP64)
     float* Hf = nullptr;
     float* Df = nullptr;
@@ -494,6 +492,7 @@ RbFoldArgs fold_args(const RbState* rb)
         f.wb[d] = rb->wb[d];
         f.w[d][0] = rb->w[d][0];
         f.w[d][1] = rb->w[d][1];
+        f.tb[d] = rb->q ? rb->tb[d] : nullptr;
     }
     return f;
 }
@@ -516,6 +515,7 @@ RbBaseArgs base_args(const RbState* rb)
     for (int d = 0; d < rb->p.ndim; ++d) {
         b.wb[d] = rb->wb[d];
         b.tb[d] = rb->tb[d];
+        for (int q = 0; q < 2; ++q) b.q[d][q] = rb->q ? rb->w[d][q] : nullptr;
     }
     b.D = rb->D;
     b.Rb = rb->Rb;
@@ -682,8 +682,9 @@ int rb_create(const ptd_ctx_base& g, const ptd_params& p, const Derived& dv, cud
         for (int q = 0; q < 2 && !rc; ++q) rc = alloc((void**)&rb->w[d][q], fb);
         if (!rc) rc = alloc((void**)&rb->tb[d], fb);
     }
-    if (!rc) rc = alloc((void**)&rb->Rb, fb);
-    if (!rc && p.ndim < 3) rc = alloc((void**)&rb->Cb, (size_t)g.nfield * sizeof(float));
+    rb->q = rb_qform(p.model, p.ndim);
+    if (!rc && !rb->q) rc = alloc((void**)&rb->Rb, fb);
+    if (!rc) rc = alloc((void**)&rb->Cb, fb);
     if (!rc && p.ndim == 3) rc = alloc((void**)&rb->Cb64, (size_t)g.nfield * sizeof(double));
     if (!rc) rc = alloc((void**)&rb->Hf, fb);
     if (!rc && (p.model == PTD_MODEL_LINSTEP || p.model == PTD_MODEL_NONLIN_EXPM)) rc = alloc((void**)&rb->Df, fb);
@@ -704,7 +705,7 @@ int rb_create(const ptd_ctx_base& g, const ptd_params& p, const Derived& dv, cud
             // faces past the last one of each direction are read (never used) by the halo lanes
             if (e == cudaSuccess) e = cudaMemsetAsync(rb->tb[d], 0, fb, s);
         }
-        if (e == cudaSuccess) e = cudaMemsetAsync(rb->Rb, 0, fb, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(rb->q ? rb->Cb : rb->Rb, 0, fb, s);
         if (e != cudaSuccess) rc = cuda_fail(e, "rb: cudaMemsetAsync");
     }
     if (rc) {

@@ -424,7 +424,7 @@ class GridBench:
         # the native-FP64 kernel's own ceiling: FP64 instructions per cell x
         # cells / launch time against this GPU's FP64 FMA rate, measured now
         fp64_pipe = None
-        per_cell = {2: 10, 3: 14}.get(self.s.ndim) if self.s.model == self.ptdiff.scripts.NONLIN else None
+        per_cell = {2: 9, 3: 13}.get(self.s.ndim) if self.s.model == self.ptdiff.scripts.NONLIN else None
         if per_cell:
             rate = ctypes.c_double(0.0)
             self.ptdiff._abi.check(self.ptdiff._abi.lib().ptd_measure_fp64_rate(ctypes.byref(rate)),

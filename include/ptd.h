@@ -307,7 +307,7 @@ PTD_API int ptd_solve_2d_noalloc(const ptd_params* p, double* H, const double* D
 /* Diagnostic, no reference counterpart: the FP64 FMA throughput of the
  * current GPU in operations per second (8 independent FMA chains per thread,
  * 8 CTAs of 256 threads per SM, CUDA-event timed; ~20 ms).  It is the roofline
- * of the native-FP64 PT kernels, which need 10 (2D) / 14 (3D) FP64
+ * of the native-FP64 PT kernels, which need 9 (2D) / 13 (3D) FP64
  * instructions per cell and so are bound by this rate rather than by HBM. */
 PTD_API int ptd_measure_fp64_rate(double* ops_per_s);
 

@@ -11,8 +11,11 @@
 // integers, added, subtracted and multiplied keeping the top 64 bits of each
 // product, and the flux is rounded once to 53 bits: 30 to 60 integer
 // instructions and up to eight 32-bit multiplies, leaving two FP64
-// instructions per face.  Measured (us per iteration, FP64 / integers): NONLIN
-// 4096^2 625 / 352, 512^3 7299 / 4191.
+// instructions per face.  The same difference serves H - Hold of the update: 9
+// (2D) and 13 (3D) FP64 instructions per cell instead of 18 and 26 (NONLIN).
+// us per iteration, FP64 / face flux in integers / H - Hold too: NONLIN 4096^2
+// 625 / 352 / 326, 512^3 7299 / 4191 / 4084; LIN 4096^2 431 / 353 / 325, 512^3
+// 4169 / 3908 (H - Hold too); LINSTEP 512^3 5922 / 4593 / 4500.
 //
 // Error: at most 0.6 ulp of the flux (an aligned sum or difference loses
 // < 2^-61, the cube < 2^-56 relative, then one rounding), against up to 4 ulp

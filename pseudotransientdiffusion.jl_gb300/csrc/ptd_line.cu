@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) pt_line_kernel(PTArgs a, LineA
                 float eq = e[q];
                 if (MODEL == NONLIN || MODEL == NONLIN_EXPM)
                     eq = cell_e<MODEL>(a, N::hf(H[q]), MODEL == NONLIN_EXPM ? N::lo_f(D[q]) : 0.0f);
-                const double Hn = h_update_sq<N>(a, H[q], Ho[q], N::sub(W[q], wl), eq);
+                const double Hn = h_update_sq<N, false>(a, H[q], Ho[q], N::sub(W[q], wl), eq);
                 if (CHECK && upd[q] && core[q]) {
                     const double ul = q > 0 ? u[q > 0 ? q - 1 : 0] : Uprev;
                     const double r = N::sub(N::mul(N::sub(u[q], ul), cst<N>(a, 0)), N::mul(N::hdn(Hn, Ho[q]), cst<N>(a, 3)));

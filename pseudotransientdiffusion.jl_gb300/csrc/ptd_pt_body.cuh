@@ -197,22 +197,34 @@ __device__ __forceinline__ float cell_e(const PTArgs& a, float h, float dmax)
     return nonlin_cell_e(a.f, h);
 }
 
+// H - Hold: integer arithmetic for native FP64 (not in 1D).
+template <class N, bool INTF>
+__device__ __forceinline__ typename N::T h_change(const typename N::HV& H, typename N::HS Ho)
+{
+    if constexpr (N::native && INTF) {
+        uint64_t r;
+        if (if_flux_lin((uint64_t)__double_as_longlong(Ho), (uint64_t)__double_as_longlong(H), r))
+            return __longlong_as_double((long long)r);
+    }
+    return N::hdo(H, Ho);
+}
+
 // H_new = H - e*((H - Hold)/dt + div)
-template <class N>
+template <class N, bool INTF = true>
 __device__ __forceinline__ typename N::HS h_update(const PTArgs& a, const typename N::HV& Hc, typename N::HS Ho,
                                                    typename N::T div, float e)
 {
-    const typename N::T Rp = N::mad(N::hdo(Hc, Ho), cst<N>(a, 3), div);
+    const typename N::T Rp = N::mad(h_change<N, INTF>(Hc, Ho), cst<N>(a, 3), div);
     return N::hstep(Hc, Rp, e);
 }
 
 // The same for square cells from the undivided flux differences:
 // H_new = H - (e sigma)*((H - Hold) rdt/sigma + sum_d (w_R - w_L)).
-template <class N>
+template <class N, bool INTF = true>
 __device__ __forceinline__ typename N::HS h_update_sq(const PTArgs& a, const typename N::HV& Hc, typename N::HS Ho,
                                                       typename N::T dsum, float e)
 {
-    const typename N::T Rp = N::mad(N::hdo(Hc, Ho), cst<N>(a, 4), dsum);
+    const typename N::T Rp = N::mad(h_change<N, INTF>(Hc, Ho), cst<N>(a, 4), dsum);
     return N::hstep(Hc, Rp, e * a.fsig);
 }
 
@@ -246,7 +258,7 @@ __device__ __forceinline__ void pt1d_body(const PTArgs& a, int bx, double& part,
             const HS Ho = N::ldo(a.Hold, i);
             const float e = cell_e<MODEL>(a, hc, MODEL == NONLIN_EXPM ? N::lo_f(Dc)
                                                  : fmaxf(fmaxf(N::lo_f(Dl), N::lo_f(Dr)), N::lo_f(Dc)));
-            const HS Hn = h_update_sq<N>(a, Hc, Ho, N::sub(wr, wl), e);   // one dimension: sigma is the only one
+            const HS Hn = h_update_sq<N, false>(a, Hc, Ho, N::sub(wr, wl), e);   // one dimension: sigma is the only one
             N::sth(a.Hout, i, Hn);
             if (CHECK) {
                 const T r = N::sub(N::mul(N::sub(ur, ul), cst<N>(a, 0)), N::mul(N::hdn(Hn, Ho), cst<N>(a, 3)));

@@ -521,11 +521,13 @@ __global__ void __launch_bounds__(256) rb_fold_batch_kernel(const RbFoldArgs* __
     if (st[w.x].step_done) return;
     const int parity = (st[w.x].phase_iter / tb) & 1;   // one buffer swap per launch of tb iterations
     const RbFoldArgs f = ftab[w.x];
-    for (int k = threadIdx.x; k < w.z; k += blockDim.x) rb_fold_elem(f, parity, (long long)w.y + k);
+    // (a chunk starts at an even element; only a field's last chunk may have an odd count)
+    for (int k = 2 * threadIdx.x; k < w.z; k += 2 * blockDim.x) rb_fold_pair(f, parity, (long long)w.y + k);
 }
 
 // Base quantities of every running instance (of all instances at a step
 // start: use_st = 0), one chunk of an instance's padded field per CTA.
+template <bool Q>
 __global__ void __launch_bounds__(256) rb_base_batch_kernel(const RbBaseArgs* __restrict__ btab, const RbDev* st,
                                                             const int4* __restrict__ fwork, int use_st)
 {
@@ -537,7 +539,7 @@ __global__ void __launch_bounds__(256) rb_base_batch_kernel(const RbBaseArgs* __
     for (int k = threadIdx.x; k < w.z; k += blockDim.x) {
         const long long e = (long long)w.y + k;
         const int ix = (int)(e % b.sy), iy = (int)(e / b.sy);
-        if (ix < b.nx) rb_base_cell(b, ix, iy, 0, part, pmax);   // padding columns hold no cell
+        if (ix < b.nx) rb_base_cell<Q>(b, ix, iy, 0, part, pmax);   // padding columns hold no cell
     }
     block_reduce_residual(b.acc64, b.norm_max, part, pmax, b.parts, blockIdx.x);   // the chunk's slot
 }
@@ -753,6 +755,13 @@ cudaError_t launch_rb_batch(ptd_batch* b, int par, bool check)
 #undef RBK
 }
 
+// The base quantities of the running instances (use_st 0: of all).
+void launch_base_batch(ptd_batch* b, int use_st)
+{
+    if (rb_qform(b->model, 2)) rb_base_batch_kernel<true><<<b->nfwork, 256, 0, b->s>>>(b->btab, b->rdev, b->fwork, use_st);
+    else rb_base_batch_kernel<false><<<b->nfwork, 256, 0, b->s>>>(b->btab, b->rdev, b->fwork, use_st);
+}
+
 // The list of the running instances' work items (after every judge).
 cudaError_t compact_rb(ptd_batch* b)
 {
@@ -855,7 +864,7 @@ int capture_rb(ptd_batch* b)
         err = cudaGetLastError();
     }
     if (err == cudaSuccess) {
-        rb_base_batch_kernel<<<b->nfwork, 256, 0, b->s>>>(b->btab, b->rdev, b->fwork, 1);
+        launch_base_batch(b, 1);
         err = cudaGetLastError();
     }
     if (err == cudaSuccess) {
@@ -1654,7 +1663,7 @@ static int batch_rb_step(ptd_batch* b, int32_t* iters, double* err_last, int* na
     const int n = b->ninst, nb = (n + 127) / 128;
     rb_reset_batch_kernel<<<nb, 128, 0, b->s>>>(b->rdev, n);
     BCK(cudaGetLastError());
-    rb_base_batch_kernel<<<b->nfwork, 256, 0, b->s>>>(b->btab, b->rdev, b->fwork, 0);
+    launch_base_batch(b, 0);
     BCK(cudaGetLastError());
     rb_base_judge_batch_kernel<<<1, 256, 0, b->s>>>(b->rdev, n, b->bp.tol, b->norm_den, b->bp.norm == PTD_NORM_MAX,
                                                     cudaGraphConditionalHandle{}, 0, b->passes, b->parts64,

@@ -91,9 +91,9 @@ __global__ void __launch_bounds__(512) rb3d_kernel(RbArgs a, int chunk)
 
 __global__ void rb_fold_kernel(RbFoldArgs f, int parity)
 {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < f.n;
-         t += (long long)gridDim.x * blockDim.x)
-        rb_fold_elem(f, parity, t);
+    for (long long t = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x); t < f.n;
+         t += 2 * (long long)gridDim.x * blockDim.x)
+        rb_fold_pair(f, parity, t);
 }
 
 __global__ void __launch_bounds__(256) rb_base_kernel(RbBaseArgs b, const RbDev* st)
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256) rb_base_kernel(RbBaseArgs b, const RbDev*
          t += (long long)gridDim.x * blockDim.x) {
         const int ix = (int)(t % b.nx);
         const long long rest = t / b.nx;
-        rb_base_cell(b, ix, (int)(rest % b.ny), (int)(rest / b.ny), part, pmax);
+        rb_base_cell<false>(b, ix, (int)(rest % b.ny), (int)(rest / b.ny), part, pmax);
     }
     block_reduce_residual(b.acc64, b.norm_max, part, pmax, b.parts, blockIdx.x);
 }
@@ -119,9 +119,8 @@ __global__ void __launch_bounds__(256) rb_base_kernel(RbBaseArgs b, const RbDev*
 // first step evaluate theirs, and in 3D both y faces are evaluated per cell.
 // Every face is the same rb_u64 evaluation, so the quantities are
 // rb_base_cell's bit for bit; the residual goes into the block's slot.
-constexpr int kBaseChunk = 32;   // rows (2D) / planes (3D) per warp
-template <int NDIM>
-__global__ void __launch_bounds__(256) rb_base_march_kernel(RbBaseArgs b, const RbDev* st)
+template <int NDIM, bool Q>
+__global__ void __launch_bounds__(256) rb_base_march_kernel(RbBaseArgs b, const RbDev* st, int chunk)
 {
     if (st && st->step_done) return;   // uniform over the grid
     const int lane = threadIdx.x;
@@ -132,16 +131,16 @@ __global__ void __launch_bounds__(256) rb_base_march_kernel(RbBaseArgs b, const 
     long long sm;   // the march: y in 2D, z in 3D
     if (NDIM == 2) {
         iy = 0;
-        k0 = (blockIdx.y * blockDim.y + threadIdx.y) * kBaseChunk;
+        k0 = (blockIdx.y * blockDim.y + threadIdx.y) * chunk;
         nm = b.ny;
         sm = b.sy;
     } else {
         iy = blockIdx.y * blockDim.y + threadIdx.y;
-        k0 = blockIdx.z * kBaseChunk;
+        k0 = blockIdx.z * chunk;
         nm = b.nz;
         sm = b.sz;
     }
-    k1 = min(k0 + kBaseChunk, nm);
+    k1 = min(k0 + chunk, nm);
     double part = 0.0;
     unsigned long long pmax = 0ull;
     if (k0 < k1 && iy < b.ny) {   // uniform over the warp
@@ -153,35 +152,35 @@ __global__ void __launch_bounds__(256) rb_base_march_kernel(RbBaseArgs b, const 
             const bool min_ = k >= 1 && k <= nm - 2;
             const bool inner = xin && yin && min_;
             // x faces: right by every lane, left from the lane below
-            const double ur = ixc <= b.nx - 2 ? rb_u64(b, c, c + 1) : 0.0;
+            const double ur = ixc <= b.nx - 2 ? rb_u64<Q>(b, c, c + 1) : 0.0;
             double ul = __shfl_up_sync(FULL, ur, 1);
-            if (lane == 0 && inner) ul = rb_u64(b, c - 1, c);
+            if (lane == 0 && inner) ul = rb_u64<Q>(b, c - 1, c);
             // march faces: above now, below from the previous step
-            const double uup = k <= nm - 2 ? rb_u64(b, c, c + sm) : 0.0;
-            if (k == k0 && inner) udn = rb_u64(b, c - sm, c);
+            const double uup = k <= nm - 2 ? rb_u64<Q>(b, c, c + sm) : 0.0;
+            if (k == k0 && inner) udn = rb_u64<Q>(b, c - sm, c);
             if (own) {
-                b.Hf[c] = __double2float_rn(b.H[c]);
+                b.Hf[c] = rb_f32<Q>(b.H[c]);
                 const int dm = NDIM - 1;   // the march direction's index
-                if (ixc <= b.nx - 2) rb_base_face(b, 0, c, ur);
-                if (k <= nm - 2) rb_base_face(b, dm, c, uup);
+                if (ixc <= b.nx - 2) rb_base_face<Q>(b, 0, c, ur);
+                if (k <= nm - 2) rb_base_face<Q>(b, dm, c, uup);
                 double uyr = 0.0;
                 if (NDIM == 3 && iy <= b.ny - 2) {
-                    uyr = rb_u64(b, c, c + b.sy);
-                    rb_base_face(b, 1, c, uyr);
+                    uyr = rb_u64<Q>(b, c, c + b.sy);
+                    rb_base_face<Q>(b, 1, c, uyr);
                 }
                 if (inner) {
                     // the order of rb_base_cell: x, y, z
                     double divu = fma(ur - ul, b.sig[0], 0.0);
-                    if (NDIM == 3) divu = fma(uyr - rb_u64(b, c - b.sy, c), b.sig[1], divu);
+                    if (NDIM == 3) divu = fma(uyr - rb_u64<Q>(b, c - b.sy, c), b.sig[1], divu);
                     divu = fma(uup - udn, b.sig[dm], divu);
                     const double dh = (b.H[c] - b.Hold[c]) * b.rdt;
-                    if (NDIM == 2 && b.Rb) {
+                    if (!Q) {
                         double divw = fma(b.wb[0][c] - b.wb[0][c - 1], b.sig[0], 0.0);
                         divw = fma(b.wb[dm][c] - b.wb[dm][c - sm], b.sig[dm], divw);
-                        b.Rb[c] = (float)(dh + divw);
+                        b.Rb[c] = rb_f32<Q>(dh + divw);
                     }
                     const double cb = divu - dh;
-                    b.Cb[c] = (float)cb;
+                    b.Cb[c] = rb_f32<Q>(cb);
                     if (NDIM == 3) b.Cb64[c] = cb;
                     accumulate_residual(cb, part, pmax);
                 }
@@ -296,6 +295,7 @@ struct RbState {
     long long nparts = 0;
     double* parts64 = nullptr;                    // FP64 residual slots of the base kernel
     long long nparts64 = 0;
+    int base_chunk = 32;                          // march of the base kernel
     int phase_iters = 200;                        // PT iterations of a phase at most
     int tblk = 1;                                 // iterations per launch (2: temporal blocking, 2D)
     cudaGraphExec_t gphase = nullptr;
@@ -440,17 +440,18 @@ long long rb_check_slots(const RbState* rb)
 dim3 base_grid(const RbState* rb)
 {
     const ptd_params& p = rb->p;
-    const unsigned gx = (p.nx + 31) / 32;
-    if (p.ndim == 2) return dim3(gx, ((p.ny + kBaseChunk - 1) / kBaseChunk + 7) / 8, 1);
-    return dim3(gx, (p.ny + 7) / 8, (p.nz + kBaseChunk - 1) / kBaseChunk);
+    const unsigned gx = (p.nx + 31) / 32, ch = rb->base_chunk;
+    if (p.ndim == 2) return dim3(gx, ((p.ny + ch - 1) / ch + 7) / 8, 1);
+    return dim3(gx, (p.ny + 7) / 8, (p.nz + ch - 1) / ch);
 }
 
 // One rebase's base kernel: 1D grid-stride, 2D / 3D the march kernel.
 cudaError_t launch_base(const RbState* rb, const RbBaseArgs& b, const RbDev* st)
 {
     if (rb->p.ndim == 1) rb_base_kernel<<<fill_blocks(), 256, 0, rb->s>>>(b, st);
-    else if (rb->p.ndim == 2) rb_base_march_kernel<2><<<base_grid(rb), dim3(32, 8), 0, rb->s>>>(b, st);
-    else rb_base_march_kernel<3><<<base_grid(rb), dim3(32, 8), 0, rb->s>>>(b, st);
+    else if (rb->p.ndim == 3) rb_base_march_kernel<3, true><<<base_grid(rb), dim3(32, 8), 0, rb->s>>>(b, st, rb->base_chunk);
+    else if (rb->q) rb_base_march_kernel<2, true><<<base_grid(rb), dim3(32, 8), 0, rb->s>>>(b, st, rb->base_chunk);
+    else rb_base_march_kernel<2, false><<<base_grid(rb), dim3(32, 8), 0, rb->s>>>(b, st, rb->base_chunk);
     return cudaGetLastError();
 }
 
@@ -658,6 +659,7 @@ int rb_create(const ptd_ctx_base& g, const ptd_params& p, const Derived& dv, cud
     // / 5800 / 5600 / 5500 / 5300, the 3D 512^3 steps 1450 / 1370 / 1330
     // against 790 / 700 / 680; without the cap the 2D steps did not converge.
     rb->phase_iters = std::max(p.nchk, 200);
+    rb->base_chunk = rb_base_march(p);
     // two iterations per launch with an even check cadence: 2D (every model),
     // and 3D (LIN, NONLIN) when asked for (PTD_FLAG_RB_TBLOCK_3D: at 512^3
     // 1233 against 1243 us per iteration, issue-bound at half the bytes)

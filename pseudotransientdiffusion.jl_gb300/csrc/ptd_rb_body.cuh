@@ -51,6 +51,7 @@
 #pragma once
 
 #include "ptd_device.cuh"
+#include "ptd_intflux.cuh"
 #include "ptd_kernels.h"
 
 namespace ptd {
@@ -913,24 +914,44 @@ struct RbFoldArgs {
     int ndim;
 };
 
-__device__ __forceinline__ void rb_fold_elem(const RbFoldArgs& f, int parity, long long t)
+// Elements t and t + 1 (t even; the last one of an odd field alone).
+__device__ __forceinline__ void rb_fold_pair(const RbFoldArgs& f, int parity, long long t)
 {
-    // both buffers cleared: the next iteration may start on either parity
     const float* dp = parity ? f.d[1] : f.d[0];
-    f.H[t] += (double)dp[t];
-    f.d[0][t] = 0.0f;
-    f.d[1][t] = 0.0f;
+    if (t + 1 >= f.n) {
+        f.H[t] += (double)dp[t];
+        f.d[0][t] = f.d[1][t] = 0.0f;
+        for (int d = 0; d < f.ndim; ++d) {
+            f.wb[d][t] += (double)f.w[d][parity][t] - (f.tb[d] ? (double)f.tb[d][t] : 0.0);
+            if (!f.tb[d]) f.w[d][0][t] = f.w[d][1][t] = 0.0f;
+        }
+        return;
+    }
+    auto at2 = [t](auto* p) { return reinterpret_cast<float2*>(const_cast<float*>(p) + t); };
+    auto at2d = [t](double* p) { return reinterpret_cast<double2*>(p + t); };
+    const float2 zero = make_float2(0.0f, 0.0f), dd = *at2(dp);
+    double2 H = *at2d(f.H);
+    H.x += (double)dd.x;
+    H.y += (double)dd.y;
+    *at2d(f.H) = H;
+    *at2(f.d[0]) = zero;
+    *at2(f.d[1]) = zero;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         if (d < f.ndim) {
-            const float* wp = parity ? f.w[d][1] : f.w[d][0];
+            const float2 w = *at2(parity ? f.w[d][1] : f.w[d][0]);
+            double2 b = *at2d(f.wb[d]);
             if (f.tb[d]) {
-                f.wb[d][t] += (double)wp[t] - (double)f.tb[d][t];
-                continue;
+                const float2 tb = *at2(f.tb[d]);
+                b.x += (double)w.x - (double)tb.x;
+                b.y += (double)w.y - (double)tb.y;
+            } else {
+                b.x += (double)w.x;
+                b.y += (double)w.y;
+                *at2(f.w[d][0]) = zero;
+                *at2(f.w[d][1]) = zero;
             }
-            f.wb[d][t] += (double)wp[t];
-            f.w[d][0][t] = 0.0f;
-            f.w[d][1][t] = 0.0f;
+            *at2d(f.wb[d]) = b;
         }
     }
 }
@@ -959,8 +980,26 @@ struct RbBaseArgs {
     int norm_max;
 };
 
+// The undamped flux of a face.  In the q form with integer arithmetic
+// (ptd_intflux.cuh): a rebase is bound by the FP64 pipe (84 % busy).  (Not in
+// the omega form of D = H^3 in 1D and 2D, where a last-bit change of t_b can
+// move a step's iteration count.)
+template <bool Q>
 __device__ __forceinline__ double rb_u64(const RbBaseArgs& b, long long cL, long long cR)
 {
+    if (Q) {
+        auto bits = [](double x) { return (uint64_t)__double_as_longlong(x); };
+        const uint64_t hl = bits(b.H[cL]), hr = bits(b.H[cR]);
+        uint64_t r;
+        bool ok;
+        if (b.model == LIN) ok = if_flux_lin(hl, hr, r);
+        else if (b.model == LINSTEP) ok = if_flux_step(hl, hr, bits(b.D[cL]), bits(b.D[cR]), r);
+        else ok = if_flux_cube(hl, hr, r);
+        if (ok) {
+            const double u = __longlong_as_double((long long)r);
+            return b.model == NONLIN_EXPM ? (b.D[cL] + b.D[cR]) * u : u;
+        }
+    }
     const double g = b.H[cR] - b.H[cL];
     if (b.model == LIN) return g;
     if (b.model == LINSTEP) return (b.D[cL] + b.D[cR]) * g;
@@ -969,12 +1008,21 @@ __device__ __forceinline__ double rb_u64(const RbBaseArgs& b, long long cL, long
     return s * s * s * g;
 }
 
+// A double rounded to the nearest float, in the q form with integer operations
+// (the hardware conversion issues on the FP64 pipe).
+template <bool Q>
+__device__ __forceinline__ float rb_f32(double x)
+{
+    return Q ? d2f_rn_bits(x) : __double2float_rn(x);
+}
+
 // t_b of the face to +d of cell c, whose undamped flux is u
+template <bool Q>
 __device__ __forceinline__ void rb_base_face(const RbBaseArgs& b, int d, long long c, double u)
 {
-    const float t = (float)(b.wb[d][c] + u);
+    const float t = rb_f32<Q>(b.wb[d][c] + u);
     b.tb[d][c] = t;
-    if (b.q[d][0]) {
+    if (Q) {
         b.q[d][0][c] = t;
         b.q[d][1][c] = t;
     }
@@ -982,6 +1030,7 @@ __device__ __forceinline__ void rb_base_face(const RbBaseArgs& b, int d, long lo
 
 // The base quantities of the cell (ix, iy, iz); its check residual goes into
 // (part, pmax).
+template <bool Q>
 __device__ __forceinline__ void rb_base_cell(const RbBaseArgs& b, int ix, int iy, int iz, double& part,
                                              unsigned long long& pmax)
 {
@@ -989,7 +1038,7 @@ __device__ __forceinline__ void rb_base_cell(const RbBaseArgs& b, int ix, int iy
     const int co[3] = {ix, iy, iz};
     const int nn[3] = {b.nx, b.ny, b.nz};
     const long long c = iz * b.sz + iy * b.sy + ix;
-    b.Hf[c] = __double2float_rn(b.H[c]);
+    b.Hf[c] = rb_f32<Q>(b.H[c]);
     bool inner = true;
 #pragma unroll
     for (int d = 0; d < 3; ++d) inner = inner && (d >= b.ndim || (co[d] >= 1 && co[d] <= nn[d] - 2));
@@ -999,20 +1048,20 @@ __device__ __forceinline__ void rb_base_cell(const RbBaseArgs& b, int ix, int iy
         if (d >= b.ndim) continue;
         double ur = 0.0;
         if (co[d] <= nn[d] - 2) {
-            ur = rb_u64(b, c, c + stp[d]);
-            rb_base_face(b, d, c, ur);
+            ur = rb_u64<Q>(b, c, c + stp[d]);
+            rb_base_face<Q>(b, d, c, ur);
         }
         if (inner) {
-            const double ul = rb_u64(b, c - stp[d], c);
-            if (b.Rb) divw = fma(b.wb[d][c] - b.wb[d][c - stp[d]], b.sig[d], divw);
+            const double ul = rb_u64<Q>(b, c - stp[d], c);
+            if (!Q) divw = fma(b.wb[d][c] - b.wb[d][c - stp[d]], b.sig[d], divw);
             divu = fma(ur - ul, b.sig[d], divu);
         }
     }
     if (inner) {
         const double dh = (b.H[c] - b.Hold[c]) * b.rdt;
-        if (b.Rb) b.Rb[c] = (float)(dh + divw);
+        if (!Q) b.Rb[c] = rb_f32<Q>(dh + divw);
         const double cb = divu - dh;
-        b.Cb[c] = (float)cb;
+        b.Cb[c] = rb_f32<Q>(cb);
         accumulate_residual(cb, part, pmax);
     }
 }

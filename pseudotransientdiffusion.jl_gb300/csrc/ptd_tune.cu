@@ -79,6 +79,16 @@ int z_march16(const ptd_params& p)
     return march_length(16, 4, 17 * sm / 2, sm, [&](int m) { return bxy * ceil_div(p.nz - 2, m); });
 }
 
+// March of the rebased form's base kernel (rows in 2D, planes in 3D, per warp
+// of 32 cells): us of a rebase at march 32 and at the march taken: 2D NONLIN
+// 256^2 124, 28 (1); 600x500 134, 53 (4); 2048^2 506, 457 (8); 3D NONLIN
+// 50x40x45 131, 33 (2); 100x90x80 175, 106 (8); 320x255x191 1290, 1239 (16).
+int rb_base_march(const ptd_params& p)
+{
+    const long long sm = sm_count(), line = ceil_div(p.nx, 32) * (p.ndim == 3 ? p.ny : 1), n = p.ndim == 3 ? p.nz : p.ny;
+    return march_length(16, 8, 120 * sm, 15 * sm, [&](int m) { return line * ceil_div(n, m); });
+}
+
 LaunchCfg tuned_config(const ptd_params& p)
 {
     LaunchCfg c;

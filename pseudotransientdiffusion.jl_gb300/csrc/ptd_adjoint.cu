@@ -68,7 +68,7 @@ struct F32 {
     __device__ static __forceinline__ T mul(T a, T b) { return a * b; }
     __device__ static __forceinline__ T mad(T a, T b, T c) { return fmaf(a, b, c); }
     __device__ static __forceinline__ float lo_f(T a) { return a; }
-    __device__ static __forceinline__ double to_d(T a) { return (double)a; }
+    __device__ static __forceinline__ double to_d(T a) { return f2d_exact(a); }
     __device__ static __forceinline__ T zero() { return 0.0f; }
     __device__ static __forceinline__ T shfl_down(T v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
     __device__ static __forceinline__ T shfl_up(T v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(32 * R) adj3d_kernel(const AdjArgs* __restrict
                     q = N::mad(N::sub(N::sub(ky, kyb), N::add(ny_, nyb)), acst<N>(a, 1), q);
                     q = N::mad(N::sub(N::sub(kz, kzb), N::add(nz_, nzb)), acst<N>(a, 2), q);
                     if (DELTA) {   // C_b + (the same terms of the changes)
-                        accumulate_residual(a.Cb[idx] + N::to_d(q) - N::to_d(lnew) * a.rdt, part, pmax);
+                        accumulate_residual(fma(-N::to_d(lnew), a.rdt, a.Cb[idx] + N::to_d(q)), part, pmax);
                     } else {
                         const T res = N::add(N::sub(gg, N::mul(lnew, acst<N>(a, 3))), q);
                         accumulate_residual(N::to_d(res), part, pmax);

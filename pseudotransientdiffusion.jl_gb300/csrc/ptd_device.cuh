@@ -105,6 +105,16 @@ __device__ __forceinline__ double f2d_bits(float f)
     return __hiloint2double((int)hi, (int)lo);
 }
 
+// The same, exact for denormals too (scaled by 2^64 first).
+__device__ __forceinline__ double f2d_exact(float f)
+{
+    const bool tiny = fabsf(f) < 0x1p-126f;
+    const unsigned b = __float_as_uint(tiny ? f * 0x1p64f : f);
+    const unsigned m = b & 0x7fffffffu;
+    const unsigned bias = m >= 0x7f800000u ? 0x70000000u : tiny ? 0x34000000u : 0x38000000u;
+    return __hiloint2double((int)((b & 0x80000000u) | (m != 0u ? (m >> 3) + bias : 0u)), (int)(b << 29));
+}
+
 // The same for a value that is not negative (the face parameter c).
 __device__ __forceinline__ double f2d_param(float f)
 {

@@ -115,7 +115,7 @@ struct DF64 {
         return fast_two_sum(s.x, __fadd_rn(s.y, __fsub_rn(w.y, e)));
     }
     __device__ static __forceinline__ float lo_f(T a) { return a.x; }
-    __device__ static __forceinline__ double to_d(T a) { return (double)a.x + (double)a.y; }
+    __device__ static __forceinline__ double to_d(T a) { return f2d_exact(a.x) + f2d_exact(a.y); }
     __device__ static __forceinline__ T zero() { return make_float2(0.0f, 0.0f); }
     __device__ static __forceinline__ T shfl_down(T v, int d)
     {

@@ -635,6 +635,15 @@ __device__ __forceinline__ void rb2d_tb2_pair_body(const RbArgs& a, int tile, in
 }
 
 // ---------------------------------------------------------------------------
+// The check residual of a 3D cell in FP64, its FP32 parts widened by integer
+// operations (the hardware conversion issues on the FP64 pipe, which bounds a
+// check launch: a check of 320x255x191 cost 155 us more than a plain iteration
+// with it, 112 so).
+__device__ __forceinline__ double rb_residual64(double cb, float divu, float d, float rdt)
+{
+    return fma(-f2d_exact(d), f2d_bits(rdt), cb + f2d_exact(divu));
+}
+
 // 3D: R warps as the y rows of an x-y tile, z march (ptd_pt_body.cuh).
 template <int MODEL, bool CHECK, int R>
 __device__ __forceinline__ void rb3d_body(const RbArgs& a, int bx, int by, int bz, int chunk, double& part,
@@ -732,7 +741,7 @@ __device__ __forceinline__ void rb3d_body(const RbArgs& a, int bx, int by, int b
                     // 3D: the FP64 pipe, otherwise idle in this kernel, forms and sums the
                     // residual from an FP64 base term (an FP32 residual, or an FP32 base term
                     // widened here, made the 512^3 step 7-16 ms longer)
-                    accumulate_residual(a.Cb64[idx] + (double)divu - (double)dnew * (double)a.rdt, part, pmax);
+                    accumulate_residual(rb_residual64(a.Cb64[idx], divu, dnew, a.rdt), part, pmax);
                 }
             }
             dc = dn;
@@ -875,7 +884,7 @@ __device__ __forceinline__ void rb3d_tb2_body(const RbArgs& a, int bx, int by, i
                 if (CHECK) {
                     const float uy2b = su2[r - 1][lane];
                     const float divu = fmaf(uz2 - uz2b, s2, fmaf(uy2 - uy2b, s1, (ux2 - ux2l) * s0));
-                    accumulate_residual(a.Cb64[o0] + (double)divu - (double)q * (double)rdt, part, pmax);
+                    accumulate_residual(rb_residual64(a.Cb64[o0], divu, q, rdt), part, pmax);
                 }
             }
             if (own_x) a.wout[0][o0] = wx2;

@@ -275,10 +275,10 @@ struct ptd_ctx : ptd_ctx_base {
     int* zero_flag = nullptr;
     double* errhist = nullptr;
     int errcap = 0;
-    DevState* h_st = nullptr;     // pinned mirror of *st (line, flow: written by the kernel, then kHostErr doubles)
-    bool line = false;            // 1D: a step is one launch of the line kernel, in place on H[cur], W[0][cur]
+    DevState* h_st = nullptr;     // pinned mirror of *st (line, flow: written by the kernel, with a HostSteps after it)
+    bool line = false;            // 1D: steps are one launch of the line kernel, in place on H[cur], W[0][cur]
     LinePlan lplan;
-    FlowPlan flow;                // 2D FP64: a step is one launch of the flow kernel (rows > 0)
+    FlowPlan flow;                // 2D FP64: steps are one launch of the flow kernel (rows > 0)
     void* flow_mem = nullptr;     // its exchange buffers
     unsigned flow_tag = 1;        // tags used so far
     cudaGraphExec_t gstep[2] = {nullptr, nullptr};   // one physical step's check loop, per start parity
@@ -297,7 +297,7 @@ struct ptd_ctx : ptd_ctx_base {
     double* stage = nullptr;      // DF64: FP64 staging field for the host boundary
 };
 
-constexpr int kHostErr = 1024;    // check residuals that the line and flow kernels leave in pinned memory
+static HostSteps* host_steps(const ptd_ctx* c) { return reinterpret_cast<HostSteps*>(c->h_st + 1); }
 
 static void args_for(const ptd_ctx* c, int parity, const int* done, PTArgs& a)
 {
@@ -578,14 +578,15 @@ extern "C" int ptd_create(ptd_ctx** out, const ptd_params* p)
     if (!rc) rc = alloc((void**)&c->st, sizeof(DevState));
     if (!rc) rc = alloc((void**)&c->zero_flag, sizeof(int));
     c->errcap = (p->nchk <= p->itmax ? p->itmax / p->nchk : 0) + 2;
-    if (!rc) rc = alloc((void**)&c->errhist, (size_t)c->errcap * sizeof(double));
     c->line = p->ndim == 1 && p->precision == PTD_PREC_FP64 && p->resid_mode == PTD_RESID_MIXED &&
               line_plan(p->model, p->nx, p->nchk, c->lplan);
     if (p->ndim == 2 && p->precision == PTD_PREC_FP64 && p->resid_mode == PTD_RESID_MIXED &&
         !(p->flags & PTD_FLAG_AUTOTUNE))
         flow_plan(p->model, p->nx, p->ny, c->flow);
     if (!rc && c->flow.rows) rc = alloc(&c->flow_mem, flow_bytes(c->flow));
-    if (!rc && cudaMallocHost((void**)&c->h_st, sizeof(DevState) + (c->line || c->flow.rows ? kHostErr * sizeof(double) : 0)) !=
+    if ((c->line || c->flow.rows) && c->errcap < 1 << 30) c->errcap += kHostErr;   // room for several steps
+    if (!rc) rc = alloc((void**)&c->errhist, (size_t)c->errcap * sizeof(double));
+    if (!rc && cudaMallocHost((void**)&c->h_st, sizeof(DevState) + (c->line || c->flow.rows ? sizeof(HostSteps) : 0)) !=
                    cudaSuccess) {
         cudaGetLastError();
         rc = fail(PTD_ENOMEM, "cudaMallocHost failed");
@@ -794,9 +795,9 @@ extern "C" int ptd_get_state(ptd_ctx* c, double* H)
     return flow_state(c);
 }
 
-// One launch of the line kernel: a whole step with its checks, or niter
+// One launch of the line kernel: up to nsteps steps with their checks, or niter
 // iterations without.
-static int run_line(ptd_ctx* c, bool checks, int niter)
+static int run_line(ptd_ctx* c, int nsteps, int niter)
 {
     PTArgs a;
     args_for(c, c->cur, c->zero_flag, a);
@@ -805,14 +806,15 @@ static int run_line(ptd_ctx* c, bool checks, int niter)
     LineArgs l = {};
     l.Hold = c->Hold;
     l.st = c->h_st;
-    l.errhist = reinterpret_cast<double*>(c->h_st + 1);
+    l.out = host_steps(c);
     l.errmore = c->errhist;
-    l.errhost = kHostErr;
     l.errcap = c->errcap;
     l.nchk = c->p.nchk;
     l.itmax = c->p.itmax;
-    l.checks = checks;
+    l.checks = nsteps > 0;
     l.niter = niter;
+    l.nsteps = nsteps;
+    l.itlimit = 1 << 20;
     l.tol = c->p.tol;
     l.norm_den = c->dv.norm_den;
     // err > tol for certain: 1e-10 covers the rounding of either side
@@ -822,9 +824,9 @@ static int run_line(ptd_ctx* c, bool checks, int niter)
     return PTD_OK;
 }
 
-// One launch of the flow kernel: a whole step with its checks, or niter
+// One launch of the flow kernel: up to nsteps steps with their checks, or niter
 // iterations without.
-static int run_flow(ptd_ctx* c, bool checks, int niter)
+static int run_flow(ptd_ctx* c, int nsteps, int niter)
 {
     if (c->flow_tag > 1u << 30) {   // long before tags come round
         CK(cudaMemsetAsync(c->flow_mem, 0, flow_bytes(c->flow), c->stream));
@@ -835,15 +837,16 @@ static int run_flow(ptd_ctx* c, bool checks, int niter)
     FlowArgs f = {};
     flow_buffers(c->flow, c->flow_mem, f);
     f.st = c->h_st;
-    f.errhist = reinterpret_cast<double*>(c->h_st + 1);
+    f.out = host_steps(c);
     f.errmore = c->errhist;
-    f.errhost = kHostErr;
     f.errcap = c->errcap;
     f.base = c->flow_tag;
     f.nchk = c->p.nchk;
     f.itmax = c->p.itmax;
-    f.checks = checks;
+    f.checks = nsteps > 0;
     f.niter = niter;
+    f.nsteps = c->p.nchk <= 4096 ? nsteps : std::min(nsteps, 1);   // (tags of a launch: see flow_tags)
+    f.itlimit = 1 << 17;
     f.tol = c->p.tol;
     f.norm_den = c->dv.norm_den;
     CK(launch_flow(a, f, c->p.model, c->flow, c->stream));
@@ -856,14 +859,14 @@ static int run_plain(ptd_ctx* c, long long n)
 {
     while (c->line && n > 0) {
         const int k = (int)std::min<long long>(n, 1 << 20);   // a launch of seconds at most
-        int rc = run_line(c, false, k);
+        int rc = run_line(c, 0, k);
         if (rc) return rc;
         c->iterations += k;
         n -= k;
     }
     while (c->flow.rows && n > 0) {
         const int k = (int)std::min<long long>(n, 1 << 18);
-        int rc = run_flow(c, false, k);
+        int rc = run_flow(c, 0, k);
         if (rc) return rc;
         c->flow_tag += k + 2;
         c->cur ^= 1;
@@ -898,47 +901,46 @@ extern "C" int ptd_iterate(ptd_ctx* c, int32_t niter)
     return run_plain(c, niter);
 }
 
-// One physical step of the FP64 solver.  Returns the PT iteration count in
-// *iters and appends the step's errors to err_hist.
-static int fp64_step(ptd_ctx* c, int32_t* iters, double* err_hist, int32_t err_cap, int32_t* n_err,
-                     int* nan_flag, int* capped)
+// Physical steps of the FP64 solver, at least one and at most *nsteps (the
+// line and flow kernels take several in a launch).  Returns the number of
+// steps in *nsteps, their PT iteration counts in iters, and appends their
+// errors to err_hist; a step with a NaN residual is the last one.
+static int fp64_steps(ptd_ctx* c, int* nsteps, int32_t* iters, double* err_hist, int32_t err_cap, int32_t* n_err,
+                      int* nan_flag, int* capped)
 {
     const ptd_params& p = c->p;
     const long long blocks_max = p.nchk <= p.itmax ? p.itmax / p.nchk : 0;
     const int start = c->cur;
     int done = DONE_RUNNING, iter = 0, nchecks = 0;
     const double* err_host = nullptr;   // the first kHostErr check residuals, on the host already
-    if (c->line) {
+    const int most = std::min(*nsteps, kHostSteps);
+    *nsteps = 1;
+    if (c->line || c->flow.rows) {
         if (blocks_max > 0) {
-            int rc = run_line(c, true, 0);
-            if (rc) return rc;
-            CK(cudaStreamSynchronize(c->stream));
-            done = c->h_st->done;
-            iter = c->h_st->iter;
-            nchecks = c->h_st->nchecks;
-            err_host = reinterpret_cast<const double*>(c->h_st + 1);
-        }
-    } else if (c->flow.rows) {
-        if (blocks_max > 0) {
+            const HostSteps& out = *host_steps(c);
             c->h_st->done = DONE_RUNNING;
-            int rc = run_flow(c, true, 0);
+            int rc = c->line ? run_line(c, most, 0) : run_flow(c, most, 0);
             if (rc) return rc;
             CK(cudaStreamSynchronize(c->stream));
             done = c->h_st->done;
             iter = c->h_st->iter;
             nchecks = c->h_st->nchecks;
-            err_host = reinterpret_cast<const double*>(c->h_st + 1);
-            // the warps run on until the decision reaches them, three blocks at most
-            c->flow_tag += (unsigned)iter + 3u * (unsigned)p.nchk + 2u;
-            if (done == FLOW_TIMEOUT || done == DONE_RUNNING) c->h_st->pad = 1;
+            err_host = out.err;
+            if (c->flow.rows && (done == FLOW_TIMEOUT || done == DONE_RUNNING)) c->h_st->pad = 1;
             rc = flow_state(c);
             if (rc) return rc;
+            *nsteps = out.nsteps;
+            for (int s = 0; s < out.nsteps; ++s) {
+                iters[s] = out.iters[s];
+                if (s < out.nsteps - 1) c->iterations += out.iters[s];
+                c->flow_tag += flow_tags(out.iters[s], p.nchk);
+            }
         }
     } else {
         CK(launch_reset_state(c->st, c->stream));
         c->launches += 1;
     }
-    if (blocks_max > 0 && !c->line && !c->flow.rows) {
+    if (blocks_max > 0 && !err_host) {
         CK(cudaGraphLaunch(c->gstep[start], c->stream));
         CK(cudaMemcpyAsync(c->h_st, c->st, sizeof(DevState), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -959,14 +961,18 @@ static int fp64_step(ptd_ctx* c, int32_t* iters, double* err_hist, int32_t err_c
         iter = p.itmax;
         *capped = 1;
     }
-    *iters = iter;
+    iters[*nsteps - 1] = iter;
+    // (the line and flow kernels leave Hold = H)
+    const bool copy = !err_host || *capped;
     const size_t bytes = (size_t)c->nfield * sizeof(double);
-    CK(cudaMemcpyAsync(c->Hold, c->H[c->cur], bytes, cudaMemcpyDeviceToDevice, c->stream));
+    if (copy) CK(cudaMemcpyAsync(c->Hold, c->H[c->cur], bytes, cudaMemcpyDeviceToDevice, c->stream));
+    bool wait = copy;
     if (err_hist && nchecks > 0 && *n_err < err_cap) {
         const int k = std::min(nchecks, std::min(err_cap - *n_err, c->errcap));
         const int kh = err_host ? std::min(k, kHostErr) : 0;
         double* const dst = err_hist + *n_err;
         if (kh) std::memcpy(dst, err_host, (size_t)kh * sizeof(double));
+        wait = wait || k > kh;
         if (k > kh)
             CK(cudaMemcpyAsync(dst + kh, c->errhist + kh, (size_t)(k - kh) * sizeof(double), cudaMemcpyDeviceToHost,
                                c->stream));
@@ -976,7 +982,7 @@ static int fp64_step(ptd_ctx* c, int32_t* iters, double* err_hist, int32_t err_c
         }
     }
     *n_err += nchecks;
-    CK(cudaStreamSynchronize(c->stream));
+    if (wait) CK(cudaStreamSynchronize(c->stream));
     *nan_flag = done == DONE_NAN;
     return PTD_OK;
 }
@@ -990,18 +996,24 @@ extern "C" int ptd_step(ptd_ctx* c, int32_t nsteps, int32_t* iters_per_step, dou
     if (err_cap < 0) return fail(PTD_EINVAL, "err_cap must be >= 0");
     int32_t ne = 0;
     int any_capped = 0;
-    for (int s = 0; s < nsteps; ++s) {
-        int32_t it = 0;
-        int nan_flag = 0, capped = 0;
-        int rc = c->dc   ? dc_step(c->dc, *c, &it, err_hist, err_cap, &ne, &nan_flag, &capped)
-                 : c->rb ? rb_step(c->rb, &it, err_hist, err_cap, &ne, &nan_flag, &capped)
-                         : fp64_step(c, &it, err_hist, err_cap, &ne, &nan_flag, &capped);
+    for (int s = 0; s < nsteps;) {
+        int32_t it[kHostSteps];
+        int k = nsteps - s, nan_flag = 0, capped = 0;
+        int rc;
+        if (c->dc || c->rb) {
+            k = 1;
+            rc = c->dc ? dc_step(c->dc, *c, it, err_hist, err_cap, &ne, &nan_flag, &capped)
+                       : rb_step(c->rb, it, err_hist, err_cap, &ne, &nan_flag, &capped);
+        } else {
+            rc = fp64_steps(c, &k, it, err_hist, err_cap, &ne, &nan_flag, &capped);
+        }
         if (rc) return rc;
-        if (iters_per_step) iters_per_step[s] = it;
+        if (iters_per_step) std::copy(it, it + k, iters_per_step + s);
+        s += k;
         any_capped |= capped;
         if (nan_flag) {
             if (n_err) *n_err = ne;
-            return fail(PTD_ENAN, "residual is NaN after physical step %d", s + 1);
+            return fail(PTD_ENAN, "residual is NaN after physical step %d", s);
         }
     }
     if (n_err) *n_err = ne;

@@ -1,4 +1,4 @@
-// ptd_flow.cu -- host side of the one-launch 2D step (ptd_flow.cuh): the tile
+// ptd_flow.cu -- host side of the 2D flow kernel (ptd_flow.cuh): the tile
 // of a warp, the exchange buffers and the cooperative launch.
 #include <mutex>
 
@@ -24,12 +24,14 @@ const void* flow_kernel(int model, int rows)
 
 // The lowest tile whose warps fit (one SM is left to the judge): the more and
 // smaller the tiles, the better the warps of an SM hide one another's latency
-// (500x333 NONLIN: 2 rows 6.0 us per iteration, 3 6.1, 4 6.4, 6 7.9).  Tiles
-// of 8 rows (up to 600 K cells) were slower than one launch per iteration.
+// (500x333 NONLIN: 2 rows 6.0 us per iteration, 3 6.1, 4 6.4, 6 7.9).  Taller
+// tiles than 5 rows (468 K cells) are slower than one launch per iteration for
+// NONLIN and LINSTEP (768x600 in 6 rows 17.8, 16.4; one launch each 15.2,
+// 15.9), than 6 rows for LIN.
 bool flow_plan(int model, int nx, int ny, FlowPlan& p)
 {
     const int most = sm_count() - 1;
-    for (int rows : {1, 2, 3, 4, 6}) {
+    for (int rows : {1, 2, 3, 4, 5, 6}) {
         p = FlowPlan();
         if (!flow_kernel(model, rows)) return false;
         const long long ntx = (nx - 2 + 30) / 31, nty = (ny - 2 + rows - 1) / rows, n = ntx * nty;
@@ -55,7 +57,8 @@ bool flow_plan(int model, int nx, int ny, FlowPlan& p)
 size_t flow_bytes(const FlowPlan& p)
 {
     const size_t n = (size_t)p.ntx * p.nty;
-    return (2 * n * 2 * 32 + 2 * n * 2 * p.rows + 2 * n) * sizeof(uint4) + (size_t)p.ctas * 128;
+    return (2 * n * 2 * 32 + 2 * n * 2 * p.rows + 2 * n) * sizeof(uint4) + (2 * n * 32 + 2 * n * p.rows) * sizeof(double) +
+           (size_t)p.ctas * 128;
 }
 
 void flow_buffers(const FlowPlan& p, void* mem, FlowArgs& f)
@@ -64,7 +67,9 @@ void flow_buffers(const FlowPlan& p, void* mem, FlowArgs& f)
     f.halo_y = static_cast<uint4*>(mem);
     f.halo_x = f.halo_y + 2 * n * 2 * 32;
     f.parts = f.halo_x + 2 * n * 2 * p.rows;
-    f.ctl = reinterpret_cast<unsigned long long*>(f.parts + 2 * n);
+    f.edge_y = reinterpret_cast<double*>(f.parts + 2 * n);
+    f.edge_x = f.edge_y + 2 * n * 32;
+    f.ctl = reinterpret_cast<unsigned long long*>(f.edge_x + 2 * n * p.rows);
     f.ntx = p.ntx;
     f.nwarps = (int)n;
 }

@@ -1,4 +1,4 @@
-// ptd_flow.cuh -- a whole physical step of a 2D grid (native FP64) in one
+// ptd_flow.cuh -- whole physical steps of a 2D grid (native FP64) in one
 // launch.
 //
 // One launch per iteration costs a grid that fits the chip about 4 us of
@@ -22,6 +22,12 @@
 // the step has stopped.  A snapshot is overwritten (two checks later) only
 // once the decision on it is known.
 //
+// Between two steps of a launch a warp reads back the snapshot that the
+// decision was on (its own stores), takes its H as Hold and exchanges edges:
+// about 2 us, where the end of a launch, the host's wait, a copy of Hold and
+// the next launch cost 38 (a solve of 5 steps of 128^2: 1.04 ms with a launch
+// per step, 0.81 in one).
+//
 // All CTAs must run at once: the launch is cooperative, and every wait has a
 // limit after which its warp gives up and the step ends with FLOW_TIMEOUT.
 //
@@ -30,9 +36,10 @@
 // Bound by the FP64 pipe and, on small grids, by the latency of an iteration
 // (about 1700 cycles of dependent arithmetic for the first row of a tile, 1200
 // for each other, and 1400-2000 of exchange through L2).  us per iteration
-// with checks every 10, one launch per iteration / here: NONLIN 64^2 3.8, 2.5;
-// 128^2 4.1, 2.6; 256^2 5.4, 3.4; 500x333 8.0, 6.0; 512^2 10.2, 7.8; 768x600
-// 16.2, 14.8; LINSTEP 500x333 8.1, 6.0; LIN 128^2 3.7, 2.2; 768x600 19.1, 12.7.
+// with checks every 10, one launch per iteration / here: NONLIN 128^2 4.1, 2.5;
+// 256^2 5.2, 3.2; 512^2 10.0, 7.3; 640^2 13.2, 10.3; 768x600 15.2, 11.9;
+// LINSTEP 500x333 8.1, 5.5; 768x600 15.9, 12.2; LIN 768x600 15.0, 11.8; 730x740
+// 16.3, 14.2.
 // (Evaluating the faces of several rows as one branch-free group was no
 // faster, and tiles of 10 rows in 8-warp CTAs slower: 128^2 2.6, 8.3.)
 #pragma once
@@ -69,10 +76,12 @@ __device__ __forceinline__ void flow_judge(const PTArgs& a, const FlowArgs& f)
     const int t = threadIdx.y * 32 + threadIdx.x, nt = min((int)blockDim.y * 32, 256);   // threads that sum
     if (t == 0) s_lost = 0;
     __syncthreads();
-    int iter = 0;
-    // every pass is a check block of nchk iterations, so it ends within itmax/nchk passes
+    int iter = 0, nchecks = 0, step = 0;   // of the step; of the launch
+    unsigned base = f.base, total = 0;
+    const int blocks = f.itmax / f.nchk;
+    // every pass is a check block of nchk iterations, so a step ends within itmax/nchk passes
     for (int n = 0;; ++n) {
-        const unsigned tag = f.base + (unsigned)n + 1u;
+        const unsigned tag = base + (unsigned)n + 1u;
         const uint4* parts = f.parts + (size_t)(n & 1) * f.nwarps;
         double sum = 0.0;
         unsigned long long mx = 0ull;
@@ -108,21 +117,34 @@ __device__ __forceinline__ void flow_judge(const PTArgs& a, const FlowArgs& f)
             if (!(err > f.tol)) done = (err != err) ? DONE_NAN : DONE_CONVERGED;
             else if (iter + f.nchk > f.itmax) done = DONE_CAP;
             if (s_lost) done = FLOW_TIMEOUT;
+            if (done == DONE_CONVERGED && step + 1 < f.nsteps && total + (unsigned)iter < (unsigned)f.itlimit &&
+                nchecks + 1 <= f.errcap - blocks)
+                done = FLOW_NEXT;
             s_done = done;
-            if (n < f.errhost) f.errhist[n] = err;
-            else if (n < f.errcap) f.errmore[n] = err;
-            if (done != DONE_RUNNING) {
+            if (nchecks < kHostErr) f.out->err[nchecks] = err;
+            else if (nchecks < f.errcap) f.errmore[nchecks] = err;
+            if (done != DONE_RUNNING) f.out->iters[step] = iter;
+            if (done != DONE_RUNNING && done != FLOW_NEXT) {
                 f.st->done = done;
-                f.st->nchecks = n + 1;
+                f.st->nchecks = nchecks + 1;
                 f.st->iter = iter;
                 f.st->err = err;
+                f.out->nsteps = step + 1;
             }
         }
         __syncthreads();
         const int done = s_done;
         const unsigned long long word = ((unsigned long long)tag << 32) | (unsigned)done;
         for (int c = t; c < (int)gridDim.x - 1; c += (int)blockDim.y * 32) *(volatile unsigned long long*)(f.ctl + 16 * c) = word;
-        if (done != DONE_RUNNING) return;
+        if (done != DONE_RUNNING && done != FLOW_NEXT) return;
+        nchecks += 1;
+        if (done == FLOW_NEXT) {
+            base += flow_tags(iter, f.nchk);
+            total += (unsigned)iter;
+            step += 1;
+            iter = 0;
+            n = -1;
+        }
         __syncthreads();   // s_sum of this check is read before the next one writes it
     }
 }
@@ -202,16 +224,23 @@ __global__ void __launch_bounds__(32 * kWarps, 1) pt2d_flow_kernel(PTArgs a, Flo
     const bool putx = (lane == 1 && left) || (lane == 31 && right);
     const bool gety_b = below && upd, gety_t = above && upd;
 
-    // stores the tile's cells and faces in the buffers of parity par
+    // the tile's cells and faces in the buffers of parity par: stored (with
+    // the faces that the neighbours own, in buffers of this warp), and read
+    // back by the threads that stored them
+    auto buf_h = [&](int par) { return static_cast<double*>(par ? a.Hout : const_cast<void*>(a.Hin)); };
+    auto buf_x = [&](int par) { return static_cast<double*>(par ? a.wout[0] : const_cast<void*>(a.win[0])); };
+    auto buf_y = [&](int par) { return static_cast<double*>(par ? a.wout[1] : const_cast<void*>(a.win[1])); };
+    auto edge_y = [&](int par) { return f.edge_y + ((size_t)par * f.nwarps + w) * 32 + lane; };
+    auto edge_x = [&](int par) { return f.edge_x + ((size_t)par * f.nwarps + w) * R; };
     auto snapshot = [&](int par) {
-        double* const Hd = static_cast<double*>(par ? a.Hout : const_cast<void*>(a.Hin));
-        double* const X = static_cast<double*>(par ? a.wout[0] : const_cast<void*>(a.win[0]));
-        double* const Y = static_cast<double*>(par ? a.wout[1] : const_cast<void*>(a.win[1]));
+        double *const Hd = buf_h(par), *const X = buf_x(par), *const Y = buf_y(par);
+        if (f.checks) *edge_y(par) = wyb;
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             if (j0 + q <= ny - 2) {
                 const long long c = at(j0 + q) + ic;
                 if (own_x) X[c] = wx[q];
+                else if (f.checks && lane == 0) edge_x(par)[q] = wx[q];
                 if (upd) {
                     Y[c] = wy[q];
                     Hd[c] = H[q];
@@ -219,6 +248,23 @@ __global__ void __launch_bounds__(32 * kWarps, 1) pt2d_flow_kernel(PTArgs a, Flo
             }
         }
         if (ty == 0 && upd) Y[ic] = wyb;
+    };
+    auto restore = [&](int par) {
+        const double *const Hd = buf_h(par), *const X = buf_x(par), *const Y = buf_y(par);
+        wyb = __ldcg(edge_y(par));
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            if (j0 + q <= ny - 2) {
+                const long long c = at(j0 + q) + ic;
+                if (own_x) wx[q] = __ldcg(X + c);
+                else if (lane == 0) wx[q] = __ldcg(edge_x(par) + q);
+                if (upd) {
+                    wy[q] = __ldcg(Y + c);
+                    H[q] = __ldcg(Hd + c);
+                    sHo[q][lane] = H[q];   // the next step's Hold
+                }
+            }
+        }
     };
 
     double part = 0.0;
@@ -271,93 +317,113 @@ __global__ void __launch_bounds__(32 * kWarps, 1) pt2d_flow_kernel(PTArgs a, Flo
         }
     };
 
+    unsigned base = f.base;   // tags of the step start above it
     // the decision published last: how many checks are decided, and the outcome
-    // (a word of an earlier launch counts as none); lane 0's reading for all
+    // (a word of an earlier step counts as none); lane 0's reading for all
     auto decided = [&](unsigned long long word, int& n, int& done) {
-        const unsigned d = (unsigned)(word >> 32) - f.base;
+        const unsigned d = (unsigned)(word >> 32) - base;
         n = __shfl_sync(FULL, d < 0x80000000u ? (int)d : 0, 0);
         done = __shfl_sync(FULL, (int)(unsigned)word, 0);
         if (n == 0) done = DONE_RUNNING;
     };
-    const int total = f.checks ? f.itmax : f.niter;
-    int left_in_block = f.checks ? f.nchk : total + 1;   // iterations to the next check
-    int nchecks = 0;
-    bool stop = false;
-    // every pass is one iteration; with checks the judge's decision ends it
-    // within itmax iterations (plus those run before the decision arrives)
-    for (int k = 0; !stop && (f.checks || k < total); ++k) {
-        const unsigned long long word = f.checks && lane == 0 ? *ctl : 0ull;   // read now, looked at after the iteration
-        if (left_in_block == 1) iteration(std::true_type{});
-        else iteration(std::false_type{});
-        const int par = (k + 1) & 1;
-        const unsigned tag = f.base + (unsigned)k + 1u;
-        // publish the edges, first of all
-        if (below && upd) flow_store(hy(par, w, 0), H[0], tag);
-        if (above && upd) flow_store(hy(par, w, 1), H[R - 1], tag);
-        if (putx) {
-            uint4* const o = hx(par, w, lane == 1 ? 0 : 1);
-#pragma unroll
-            for (int q = 0; q < R; ++q) flow_store(o + q, H[q], tag);
-        }
-        int nd = 0, done = DONE_RUNNING;
-        if (f.checks) decided(word, nd, done);
-        if (--left_in_block == 0) {
-            left_in_block = f.nchk;
-            // the snapshot of two checks ago is given up: its decision must be known
-            for (int wait = kFlowWait; nd < nchecks - 1 && done == DONE_RUNNING; --wait) {
-                decided(lane == 0 ? *ctl : 0ull, nd, done);
-                if (wait == 0) done = FLOW_TIMEOUT;
+    int flip = 0;   // parity of the buffers that hold the step's first state
+    // every pass is a step (a launch without checks: its iterations)
+    for (bool first = true;; first = false) {
+        int left_in_block = f.checks ? f.nchk : f.niter + 1;   // iterations to the next check
+        int nchecks = 0, nd = 0, done = DONE_RUNNING;          // checks posted, decided
+        bool stop = false;
+        // every pass is one iteration (a step after the first begins with an
+        // exchange alone); with checks the judge's decision ends it within itmax
+        // iterations (plus those run before the decision arrives)
+        for (int k = first ? 0 : -1; !stop && (f.checks || k < f.niter); ++k) {
+            const unsigned long long word = f.checks && lane == 0 ? *ctl : 0ull;   // read now, looked at after the iteration
+            if (k >= 0) {
+                if (left_in_block == 1) iteration(std::true_type{});
+                else iteration(std::false_type{});
             }
-            if (done == DONE_RUNNING) {
-                snapshot((nchecks + 1) & 1);
-                const double v = a.norm_max ? __longlong_as_double((long long)warp_max_u64(pmax)) : warp_sum(part);
-                if (lane == 0) flow_store(f.parts + (size_t)(nchecks & 1) * f.nwarps + w, v, f.base + (unsigned)nchecks + 1u);
-                nchecks += 1;
-                part = 0.0;
-                pmax = 0ull;
-            }
-        }
-        stop = done != DONE_RUNNING;
-        if (!f.checks && k == total - 1) break;
-        // the neighbours' edges of the same iteration
-        bool ok = stop;
-        for (int wait = kFlowWait; !ok; --wait) {
-            uint4 vb = make_uint4(0, tag, 0, tag), vt = vb, vx[R];
-            if (gety_b) vb = flow_load(hy(par, w - f.ntx, 1));
-            if (gety_t) vt = flow_load(hy(par, w + f.ntx, 0));
-            bool here = true;
-            if (getx) {
-                const uint4* const src = hx(par, lane == 0 ? w - 1 : w + 1, lane == 0 ? 1 : 0);
+            const int par = (k + 1) & 1;
+            const unsigned tag = base + (unsigned)k + 1u;
+            // publish the edges, first of all
+            if (below && upd) flow_store(hy(par, w, 0), H[0], tag);
+            if (above && upd) flow_store(hy(par, w, 1), H[R - 1], tag);
+            if (putx) {
+                uint4* const o = hx(par, w, lane == 1 ? 0 : 1);
 #pragma unroll
-                for (int q = 0; q < R; ++q) vx[q] = flow_load(src + q);
-#pragma unroll
-                for (int q = 0; q < R; ++q) here = here && flow_ready(vx[q], tag);
+                for (int q = 0; q < R; ++q) flow_store(o + q, H[q], tag);
             }
-            here = here && flow_ready(vb, tag) && flow_ready(vt, tag);
-            ok = __all_sync(FULL, here);
-            if (ok) {
-                if (gety_b) Hb = flow_value(vb);
-                if (gety_t) Ht = flow_value(vt);
+            if (f.checks) decided(word, nd, done);
+            if (k >= 0 && --left_in_block == 0) {
+                left_in_block = f.nchk;
+                // the snapshot of two checks ago is given up: its decision must be known
+                for (int wait = kFlowWait; nd < nchecks - 1 && done == DONE_RUNNING; --wait) {
+                    decided(lane == 0 ? *ctl : 0ull, nd, done);
+                    if (wait == 0) done = FLOW_TIMEOUT;
+                }
+                if (done == DONE_RUNNING) {
+                    snapshot((flip + nchecks + 1) & 1);
+                    const double v = a.norm_max ? __longlong_as_double((long long)warp_max_u64(pmax)) : warp_sum(part);
+                    if (lane == 0) flow_store(f.parts + (size_t)(nchecks & 1) * f.nwarps + w, v, base + (unsigned)nchecks + 1u);
+                    nchecks += 1;
+                    part = 0.0;
+                    pmax = 0ull;
+                }
+            }
+            stop = done != DONE_RUNNING;
+            if (!f.checks && k == f.niter - 1) break;
+            // the neighbours' edges of the same iteration
+            bool ok = stop;
+            for (int wait = kFlowWait; !ok; --wait) {
+                uint4 vb = make_uint4(0, tag, 0, tag), vt = vb, vx[R];
+                if (gety_b) vb = flow_load(hy(par, w - f.ntx, 1));
+                if (gety_t) vt = flow_load(hy(par, w + f.ntx, 0));
+                bool here = true;
                 if (getx) {
+                    const uint4* const src = hx(par, lane == 0 ? w - 1 : w + 1, lane == 0 ? 1 : 0);
 #pragma unroll
-                    for (int q = 0; q < R; ++q) {
-                        if (lane == 0) H[q] = flow_value(vx[q]);
-                        else sHr[q] = flow_value(vx[q]);   // (read by this lane alone)
+                    for (int q = 0; q < R; ++q) vx[q] = flow_load(src + q);
+#pragma unroll
+                    for (int q = 0; q < R; ++q) here = here && flow_ready(vx[q], tag);
+                }
+                here = here && flow_ready(vb, tag) && flow_ready(vt, tag);
+                ok = __all_sync(FULL, here);
+                if (ok) {
+                    if (gety_b) Hb = flow_value(vb);
+                    if (gety_t) Ht = flow_value(vt);
+                    if (getx) {
+#pragma unroll
+                        for (int q = 0; q < R; ++q) {
+                            if (lane == 0) H[q] = flow_value(vx[q]);
+                            else sHr[q] = flow_value(vx[q]);   // (read by this lane alone)
+                        }
+                    }
+                } else {
+                    // a neighbour may have left: the step has stopped
+                    if (f.checks) decided(lane == 0 ? *ctl : 0ull, nd, done);
+                    if (wait == 0) done = FLOW_TIMEOUT;
+                    if (done != DONE_RUNNING) {
+                        stop = true;
+                        break;
                     }
                 }
-            } else {
-                // a neighbour may have left: the step has stopped
-                if (f.checks) decided(lane == 0 ? *ctl : 0ull, nd, done);
-                if (wait == 0) done = FLOW_TIMEOUT;
-                if (done != DONE_RUNNING) {
-                    stop = true;
-                    break;
-                }
             }
+            if (done == FLOW_TIMEOUT && lane == 0) f.st->pad = 1;
         }
-        if (done == FLOW_TIMEOUT && lane == 0) f.st->pad = 1;
+        if (!f.checks) {
+            snapshot(1);
+            return;
+        }
+        flip = (flip + nd) & 1;
+        if (done == DONE_CONVERGED || done == DONE_NAN || done == FLOW_NEXT) restore(flip);
+        if (done != FLOW_NEXT) break;
+        base += flow_tags(nd * f.nchk, f.nchk);
+        part = 0.0;
+        pmax = 0ull;
     }
-    if (!f.checks) snapshot(1);
+    // Hold of the next step (a step stopped by itmax goes on from its own)
+    double* const Od = static_cast<double*>(const_cast<void*>(a.Hold));
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+        if (upd && j0 + q <= ny - 2) Od[at(j0 + q) + ic] = sHo[q][lane];
 }
 
 template <int MODEL>
@@ -368,8 +434,10 @@ const void* flow_kernel_of(int rows)
     case 2: return (const void*)pt2d_flow_kernel<MODEL, 2>;
     case 3: return (const void*)pt2d_flow_kernel<MODEL, 3>;
     case 4: return (const void*)pt2d_flow_kernel<MODEL, 4>;
-    case 6: return (const void*)pt2d_flow_kernel<MODEL, 6>;
+    case 5: return (const void*)pt2d_flow_kernel<MODEL, 5>;
     }
+    if constexpr (MODEL == LIN)
+        if (rows == 6) return (const void*)pt2d_flow_kernel<MODEL, 6>;
     return nullptr;
 }
 

@@ -1,4 +1,4 @@
-// ptd_flow.h -- host interface of the one-launch 2D step (ptd_flow.cuh).
+// ptd_flow.h -- host interface of the 2D kernel that holds whole steps (ptd_flow.cuh).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -20,19 +20,28 @@ struct FlowArgs {
     uint4* halo_y;             // [parity][warp][bottom, top][lane]
     uint4* halo_x;             // [parity][warp][left, right][row]
     uint4* parts;              // [parity][warp]: check residuals
+    double* edge_y;            // [parity][warp][lane]: flux on a tile's lower edge at a check
+    double* edge_x;            // [parity][warp][row]: flux on its left edge
     unsigned long long* ctl;   // [CTA][16]: the latest decision, one line per CTA
-    DevState* st;              // host-visible: the outcome
-    double* errhist;           // host-visible: err of the first errhost checks,
+    DevState* st;              // host-visible: the outcome,
+    HostSteps* out;            // the steps, and err of the first checks,
     double* errmore;           // device memory: of the others, each at its index
-    int errhost, errcap;
+    int errcap;
     unsigned base;             // tags of this launch start above it
     int ntx, nwarps;           // warp tiles in x and in all
     int nchk, itmax, checks, niter;   // checks 0: niter iterations without checks
+    int nsteps, itlimit;       // steps at most, and none begun after that many iterations
     double tol, norm_den;
 };
 
-// Done states of a launch besides DONE_*: a wait that gave up.
-enum { FLOW_TIMEOUT = 4 };
+// Done states besides DONE_*: a wait that gave up; a step that converged, and
+// the next one begins in the same launch.
+enum { FLOW_TIMEOUT = 4, FLOW_NEXT = 5 };
+
+// Tags that a step of iter iterations uses: its warps run on until the
+// decision reaches them, three check blocks at most, and the next step's first
+// exchange has one.
+__host__ __device__ inline unsigned flow_tags(int iter, int nchk) { return (unsigned)iter + 3u * (unsigned)nchk + 2u; }
 
 // False: the grid does not fit the registers of the SMs (or the model has no flow kernel).
 bool flow_plan(int model, int nx, int ny, FlowPlan& p);

@@ -24,6 +24,15 @@ struct DevState {
 
 enum { DONE_RUNNING = 0, DONE_CONVERGED = 1, DONE_NAN = 2, DONE_CAP = 3 };
 
+// The outcome of a launch of several physical steps (line and flow kernels),
+// host-visible: the steps it ended, their iterations, and the residuals of its
+// first kHostErr checks.
+constexpr int kHostErr = 1024, kHostSteps = 256;
+struct HostSteps {
+    int nsteps, iters[kHostSteps];
+    double err[kHostErr];
+};
+
 struct LaunchCfg {
     int chunk2d = 64;   // rows per 2D y-march
     int warps2d = 4;    // 31-cell strips per 2D block

@@ -1,16 +1,18 @@
-// ptd_line.cu -- a whole physical step of a 1D grid in one launch.
+// ptd_line.cu -- whole physical steps of a 1D grid in one launch.
 //
 // A 1D grid is too small for one launch per PT iteration to do anything but
 // wait: 512 cells take 3.1 us per iteration, nearly all of it launch gap and
 // memory latency.  Here one thread-block cluster (up to 16 CTAs) keeps H and
-// the fluxes in its shared memory for the whole step.  A warp loads a window
+// the fluxes in its shared memory from the first step to the last.  A warp loads a window
 // of 32 C cells, runs up to `tmax` PT iterations on it in registers -- the
 // outermost cells go stale one per iteration and side -- and writes back the
 // cells in the middle, which are still exact; then one cluster barrier, and
 // the next block.  The last block of a check also leaves the warp's residual
 // in shared memory, and after the barrier every warp sums all of them in the
 // same order and takes the same decision, so the step needs no judge and no
-// second launch.  The arithmetic is pt1d_body's, operation for operation.
+// second launch, and goes straight on to the next one with Hold = H (10 steps
+// of 512 cells: 1.17 ms with a launch per step, 1.04 in one).  The arithmetic
+// is pt1d_body's, operation for operation.
 //
 // Bound by the latency of a chain of six dependent FP64 instructions per
 // iteration (64-76 cycles each, which is also what a scheduler needs to issue
@@ -32,7 +34,6 @@ namespace ptd {
 namespace {
 
 constexpr int kMaxWarps = 8;     // warps per CTA (13824 cells in all; at 16384 one launch per iteration is as fast)
-constexpr int kErr = 1024;       // errhost at most (shared memory of a launch)
 constexpr int kMaxCluster = 16;  // CTAs (above 8 the size is not portable: granted by kernel attribute)
 
 // One cell window of a warp: C consecutive cells per lane.
@@ -49,7 +50,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) pt_line_kernel(PTArgs a, LineA
     double* sH = smem;
     double* sW = smem + 2 * slice;
     double* sR = smem + 4 * slice;
-    double* sE = sR + 2 * kMaxWarps;   // CTA 0: acc of the first errhost checks
+    double* sE = sR + 2 * kMaxWarps;   // CTA 0: acc of the first kHostErr checks
     double* const Hg = static_cast<double*>(a.Hout);
     double* const Wg = static_cast<double*>(a.wout[0]);
     double* const Og = l.Hold;
@@ -87,11 +88,15 @@ __global__ void __launch_bounds__(32 * kMaxWarps) pt_line_kernel(PTArgs a, LineA
         return cluster.map_shared_rank(base, (unsigned)r) + (j - r * slice);
     };
     int iter = 0, nchecks = 0, done = DONE_RUNNING, buf = 0;
+    int steps = 0;                                     // steps ended,
+    unsigned total = 0;                                // their iterations
+    const int blocks = l.itmax / max(l.nchk, 1);       // checks of a step at most
+    bool begin = false;                                // a step begins: Hold = H
     double acc = 0.0;
     const int nchk = l.checks ? l.nchk : l.niter;      // iterations of one check block
     cluster.sync();
     // every pass runs 1..tmax iterations of a check block, so the loop ends
-    // within itmax (niter) passes
+    // within nsteps * itmax (niter) passes
     for (int left = l.checks ? (nchk <= l.itmax ? nchk : 0) : l.niter; left > 0;) {
         const int n = min(left, l.tmax);
         const bool check = l.checks && n == left;
@@ -101,7 +106,9 @@ __global__ void __launch_bounds__(32 * kMaxWarps) pt_line_kernel(PTArgs a, LineA
             const bool in = j >= 0 && j < nx;
             H[q] = in ? *at(sH + buf * slice, j) : 0.0;
             W[q] = in ? *at(sW + buf * slice, j) : 0.0;
+            if (begin) Ho[q] = H[q];
         }
+        begin = false;
         double part = 0.0;
         unsigned long long pmax = 0ull;
         auto iteration = [&](auto chk) {
@@ -167,7 +174,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) pt_line_kernel(PTArgs a, LineA
             // memory until the end: the next barrier would wait for a store to
             // the host
             if (rank == 0 && warp == 0 && lane == 0) {
-                if (nchecks < l.errhost) sE[nchecks] = acc;
+                if (nchecks < kHostErr) sE[nchecks] = acc;
                 else if (nchecks < l.errcap) l.errmore[nchecks] = acc;
             }
             nchecks += 1;
@@ -178,6 +185,16 @@ __global__ void __launch_bounds__(32 * kMaxWarps) pt_line_kernel(PTArgs a, LineA
                 if (!(err > l.tol)) done = (err != err) ? DONE_NAN : DONE_CONVERGED;
             }
             if (done == DONE_RUNNING && iter + nchk > l.itmax) done = DONE_CAP;
+            if (done != DONE_RUNNING) {
+                if (rank == 0 && warp == 0 && lane == 0) l.out->iters[steps] = iter;
+                steps += 1;
+                total += iter;
+                if (done == DONE_CONVERGED && steps < l.nsteps && total < (unsigned)l.itlimit && nchecks <= l.errcap - blocks) {
+                    done = DONE_RUNNING;
+                    begin = true;
+                    iter = 0;
+                }
+            }
             left = done == DONE_RUNNING ? nchk : 0;
         }
     }
@@ -187,17 +204,20 @@ __global__ void __launch_bounds__(32 * kMaxWarps) pt_line_kernel(PTArgs a, LineA
             const int j = x0 + lane * C + q;
             Hg[j] = sH[buf * slice + j - first];
             Wg[j] = sW[buf * slice + j - first];
+            // the next step's Hold; a step stopped by itmax goes on from its own
+            if (l.checks) Og[j] = done == DONE_CAP ? Ho[q] : Hg[j];
         }
     }
     if (l.checks && rank == 0 && warp == 0) {
         __syncwarp();
-        for (int k = lane; k < min(nchecks, l.errhost); k += 32) l.errhist[k] = sE[k];
+        for (int k = lane; k < min(nchecks, kHostErr); k += 32) l.out->err[k] = sE[k];
     }
     if (l.checks && rank == 0 && warp == 0 && lane == 0) {
         l.st->done = done;
         l.st->nchecks = nchecks;
         l.st->iter = iter;
         l.st->acc = acc;
+        l.out->nsteps = steps;
     }
     cluster.sync();   // no CTA leaves while another may read its shared memory
 }
@@ -224,7 +244,7 @@ cudaLaunchConfig_t launch_of(const LinePlan& p, cudaStream_t s, cudaLaunchAttrib
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.ctas);
     cfg.blockDim = dim3(32, p.warps);
-    cfg.dynamicSmemBytes = (size_t)(4 * p.warps * p.core + 2 * kMaxWarps + kErr) * sizeof(double);
+    cfg.dynamicSmemBytes = (size_t)(4 * p.warps * p.core + 2 * kMaxWarps + kHostErr) * sizeof(double);
     cfg.stream = s;
     at->id = cudaLaunchAttributeClusterDimension;
     at->val.clusterDim.x = p.ctas;
@@ -283,7 +303,6 @@ cudaError_t launch_line(const PTArgs& a, const LineArgs& l, int model, const Lin
     la.tmax = p.tmax;
     la.core = p.core;
     la.warps = p.warps;
-    la.errhost = std::min(l.errhost, kErr);
     void* args[] = {&pa, &la};
     return cudaLaunchKernelExC(&cfg, line_kernel(model, p.c), args);
 }

@@ -1,4 +1,4 @@
-// ptd_line.h -- host interface of the one-launch 1D step (ptd_line.cu).
+// ptd_line.h -- host interface of the 1D kernel that holds whole steps (ptd_line.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -15,10 +15,11 @@ struct LinePlan {
 
 struct LineArgs {
     double* Hold;
-    DevState* st;        // host-visible: the outcome of the step (checks)
-    double* errhist;     // host-visible: acc (sum R^2, or max |R|) of the first errhost checks,
+    DevState* st;        // host-visible: the outcome of the launch (checks),
+    HostSteps* out;      // its steps, and acc (sum R^2, or max |R|) of its first checks,
     double* errmore;     // device memory: of the others, each at its index
-    int errhost, errcap, nchk, itmax, checks, niter;   // checks 0: niter iterations without checks
+    int errcap, nchk, itmax, checks, niter;   // checks 0: niter iterations without checks
+    int nsteps, itlimit; // steps at most, and none begun after that many iterations
     double tol, norm_den;
     double acc_above;    // an acc above it has err > tol
     int tmax, core, warps;

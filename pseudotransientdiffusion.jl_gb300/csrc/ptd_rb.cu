@@ -89,6 +89,19 @@ __global__ void __launch_bounds__(512) rb3d_kernel(RbArgs a, int chunk)
     if (CHECK) block_reduce_residual(a.acc, a.norm_max, part, pmax, a.parts, block_slot());
 }
 
+// Pairs of cells (LIN, NONLIN): 8-warp CTAs of 62 x 7 updated cells.
+template <int MODEL, bool CHECK>
+__global__ void __launch_bounds__(256) rb3d_pair_kernel(RbArgs a, int chunk)
+{
+    pdl_begin();
+    if (rb_skip(a.skip)) return;
+    double part = 0.0;
+    unsigned long long pmax = 0ull;
+    if constexpr (MODEL == LIN || MODEL == NONLIN)
+        rb3d_pair_body<MODEL, CHECK, 8>(a, blockIdx.x, blockIdx.y, blockIdx.z, chunk, part, pmax);
+    if (CHECK) block_reduce_residual(a.acc, a.norm_max, part, pmax, a.parts, block_slot());
+}
+
 __global__ void rb_fold_kernel(RbFoldArgs f, int parity)
 {
     for (long long t = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x); t < f.n;
@@ -374,6 +387,9 @@ cudaError_t rb_launch_model(const RbArgs& a, int ndim, const LaunchCfg& cfg, cud
         const int chunk = cfg.chunk3d;
         dim3 grid((a.nx - 2 + 27) / 28, (a.ny - 2 + 11) / 12, (a.nz - 2 + chunk - 1) / chunk);
         return launch_pdl(rb3d_tb2_kernel<MODEL, CHECK>, grid, dim3(32, 16), s, a, chunk);
+    } else if (rb3d_pair(MODEL, a.nx, a.ny, a.nz)) {
+        dim3 grid((a.nx - 2 + 61) / 62, (a.ny - 2 + 6) / 7, (a.nz - 2 + cfg.chunk3d - 1) / cfg.chunk3d);
+        return launch_pdl(rb3d_pair_kernel<MODEL, CHECK>, grid, dim3(32, 8), s, a, cfg.chunk3d);
     } else {
         const int tx = (a.nx - 2 + 30) / 31;
         dim3 grid(tx, (a.ny - 2 + 14) / 15, (a.nz - 2 + cfg.chunk3d - 1) / cfg.chunk3d);
@@ -432,6 +448,7 @@ long long rb_check_slots(const RbState* rb)
     }
     const long long nzc = (p.nz - 2 + c.chunk3d - 1) / c.chunk3d;
     if (rb->tblk == 2) return (long long)((p.nx - 2 + 27) / 28) * ((p.ny - 2 + 11) / 12) * nzc;
+    if (rb3d_pair(p.model, p.nx, p.ny, p.nz)) return (long long)((p.nx - 2 + 61) / 62) * ((p.ny - 2 + 6) / 7) * nzc;
     return (long long)((p.nx - 2 + 30) / 31) * ((p.ny - 2 + 14) / 15) * nzc;
 }
 

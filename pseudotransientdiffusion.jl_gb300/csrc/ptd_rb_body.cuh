@@ -758,6 +758,132 @@ __device__ __forceinline__ void rb3d_body(const RbArgs& a, int bx, int by, int b
 }
 
 // ---------------------------------------------------------------------------
+// 3D with two x-adjacent cells per lane (LIN and NONLIN): rb3d_body on tiles of
+// 64 columns x R rows, lane L holding the columns 62 bx + 2 L and + 2 L + 1
+// (one aligned 8-byte pair; 1..62 are updated), every pair of faces and cells
+// as one FP32x2 evaluation, and the loads of a plane issued a plane ahead.
+// Each cell's arithmetic is rb3d_body's, operation for operation.  Fewer
+// instructions per cell (NONLIN 320x255x191: 89 against 109 million of a warp), but half the
+// warps; bound by the latency of a plane on small grids and by HBM on large
+// ones.  us per iteration with checks every 10, rb3d_body / here: LIN 64^3 8.0,
+// 6.4; 128^3 26.4, 22.6; 320x255x191 146, 133; 512^3 1164, 1012; NONLIN 64^3
+// 8.6, 6.9; 96^3 17.9, 15.9; 128^3 30.4, 29.4; 192^3 82, 86; 320x255x191 153,
+// 158.  (Staging the loads through a shared-memory ring with cp.async was
+// slower: 128^3 40; so were 16 rows and, for LIN, 32-bit offsets.)
+template <int MODEL, bool CHECK, int R>
+__device__ __forceinline__ void rb3d_pair_body(const RbArgs& a, int bx, int by, int bz, int chunk, double& part,
+                                               unsigned long long& pmax)
+{
+    constexpr bool Q = true;   // carries q, not omega
+    static_assert(MODEL == LIN || MODEL == NONLIN, "the pair kernel serves LIN and NONLIN");
+    __shared__ float2 sd[2][R][32];
+    __shared__ float2 sh[2][R][32];
+    __shared__ float2 sw[2][R][32];
+    __shared__ float2 su[CHECK ? 2 : 1][CHECK ? R : 1][32];
+    const int lane = threadIdx.x, r = threadIdx.y;
+    const int nx = a.nx, ny = a.ny, nz = a.nz;
+    const int c0 = 62 * bx + 2 * lane;
+    const int j = (R - 1) * by + r;
+    const int k0 = 1 + bz * chunk;
+    const int k1 = min(k0 + chunk, nz - 1);
+    if (k0 >= k1) return;   // uniform over the block
+    const long long sy = a.sy, sz = a.sz;
+    // a pair past the row pitch is read at the row's last pair, a row past the
+    // grid at its last row: their values feed only faces and cells that are
+    // discarded
+    const int cl = min(c0, (int)sy - 2), jc = min(j, ny - 1);
+    const bool row = j >= 1 && j <= ny - 2 && r >= 1;                     // of updated cells (uniform over the warp)
+    const bool u0 = lane >= 1 && c0 <= nx - 2, u1 = lane <= 30 && c0 + 1 <= nx - 2;   // updated columns
+    const bool x0 = (lane >= 1 || bx == 0) && c0 <= nx - 2, x1 = u1;      // x faces stored
+    const bool yf = j <= ny - 2, ystore = yf && (r >= 1 || by == 0);      // y faces evaluated, stored
+    const bool top = r == R - 1, up_ok = jc + 1 < ny;
+    auto ld2 = [&](const float* p, long long o) { return *reinterpret_cast<const float2*>(p + o); };
+    auto st2 = [&](float* p, long long o, float2 v, bool ma, bool mb) {
+        if (ma && mb) {
+            *reinterpret_cast<float2*>(p + o) = v;
+        } else {
+            if (ma) p[o] = v.x;
+            if (mb) p[o + 1] = v.y;
+        }
+    };
+    // right neighbours of the two cells; left faces from right faces
+    auto right = [&](float2 v) { return f2(v.y, __shfl_down_sync(FULL, v.x, 1)); };
+    auto left = [&](float2 w) { return f2(__shfl_up_sync(FULL, w.y, 1), w.x); };
+    const float2 z2 = f2(0.0f), s0 = f2(a.sig[0]), s1 = f2(a.sig[1]), s2 = f2(a.sig[2]), rdt = f2(a.rdt);
+    long long idx = (long long)k0 * sz + (long long)jc * sy + cl;
+    float2 dc = ld2(a.din, idx), hc = ld2(a.Hf, idx), wzb = z2, uzb = z2;
+    if (row) {
+        wzb = rb_face2<MODEL, CHECK, Q>(a, ld2(a.din, idx - sz), dc, ld2(a.Hf, idx - sz), hc, z2, z2,
+                                        ld2(a.win[2], idx - sz), z2, uzb);
+        if (k0 == 1) st2(a.wout[2], idx - sz, wzb, u0, u1);
+    }
+    int p = 0;
+    sd[0][r][lane] = dc;
+    sh[0][r][lane] = hc;
+    // the loads of a plane are issued a plane ahead
+    float2 dn = z2, hn = z2, wx = z2, wy = z2, wz = z2, cb = z2, du = dc, hu = hc;
+    auto load = [&](long long o) {
+        dn = ld2(a.din, o + sz);
+        hn = ld2(a.Hf, o + sz);
+        if (yf) wy = ld2(a.win[1], o);
+        if (row) {
+            wx = ld2(a.win[0], o);
+            wz = ld2(a.win[2], o);
+            cb = ld2(a.Cb, o);
+        }
+        if (top && up_ok) {
+            du = ld2(a.din, o + sy);
+            hu = ld2(a.Hf, o + sy);
+        }
+    };
+    load(idx);
+    __syncthreads();
+    for (int k = k0; k < k1; ++k, idx += sz) {
+        if (!top) {
+            du = sd[p][r + 1][lane];
+            hu = sh[p][r + 1][lane];
+        }
+        float2 ux = z2, uy = z2, uz = z2, wxn = z2, wyn = z2, wzn = z2;
+        if (yf) {
+            wyn = rb_face2<MODEL, CHECK, Q>(a, dc, du, hc, hu, z2, z2, wy, z2, uy);
+            if (ystore) st2(a.wout[1], idx, wyn, u0, u1);
+        }
+        sw[p][r][lane] = wyn;
+        if (CHECK) su[p][r][lane] = uy;
+        sd[p ^ 1][r][lane] = dn;
+        sh[p ^ 1][r][lane] = hn;
+        if (row) {
+            wxn = rb_face2<MODEL, CHECK, Q>(a, dc, right(dc), hc, right(hc), z2, z2, wx, z2, ux);
+            wzn = rb_face2<MODEL, CHECK, Q>(a, dc, dn, hc, hn, z2, z2, wz, z2, uz);
+            st2(a.wout[0], idx, wxn, x0, x1);
+            st2(a.wout[2], idx, wzn, u0, u1);
+        }
+        const float2 d0 = dc, h0 = hc, cb0 = cb;
+        dc = dn;
+        hc = hn;
+        if (k + 1 < k1) load(idx + sz);
+        __syncthreads();
+        if (row) {
+            const float2 wyb = sw[p][r - 1][lane], wxl = left(wxn);
+            const float2 e = f2(-rb_cell_e<MODEL>(a, h0.x + d0.x, 0.0f), -rb_cell_e<MODEL>(a, h0.y + d0.y, 0.0f));
+            const float2 div = fma2(sub2(wzn, wzb), s2, fma2(sub2(wyn, wyb), s1, mul2(sub2(wxn, wxl), s0)));
+            const float2 dnew = fma2(e, fma2(d0, rdt, sub2(div, cb0)), d0);
+            st2(a.dout, idx, dnew, u0, u1);
+            if (CHECK) {
+                const float2 uyb = su[p][r - 1][lane], uxl = left(ux);
+                const float2 divu = fma2(sub2(uz, uzb), s2, fma2(sub2(uy, uyb), s1, mul2(sub2(ux, uxl), s0)));
+                const double2 c64 = *reinterpret_cast<const double2*>(a.Cb64 + idx);
+                if (u0) accumulate_residual(rb_residual64(c64.x, divu.x, dnew.x, a.rdt), part, pmax);
+                if (u1) accumulate_residual(rb_residual64(c64.y, divu.y, dnew.y, a.rdt), part, pmax);
+            }
+        }
+        wzb = wzn;
+        uzb = uz;
+        p ^= 1;
+    }
+}
+
+// ---------------------------------------------------------------------------
 // 3D, two iterations per launch (temporal blocking in z, LIN and NONLIN).
 // The tile is R warps (y rows) x 32 lanes (x columns): lane L <-> column
 // 28 bx + L - 1, row r <-> row (R-4) by + r - 1.  The first iteration (level 1)

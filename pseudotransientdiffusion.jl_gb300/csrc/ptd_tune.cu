@@ -79,6 +79,24 @@ int z_march16(const ptd_params& p)
     return march_length(16, 4, 17 * sm / 2, sm, [&](int m) { return bxy * ceil_div(p.nz - 2, m); });
 }
 
+// Whether the 3D rebased form runs two cells per lane (rb3d_pair_body): always
+// for LIN; for NONLIN, whose one-cell kernel hides its longer chains behind
+// twice the warps, while the fields (40 bytes a cell) fit the L2 cache.
+bool rb3d_pair(int model, long long nx, long long ny, long long nz)
+{
+    return model == LIN || (model == NONLIN && nx * ny * nz <= 2400000);
+}
+
+// Its march: us per iteration at marches 2, 4, 8, 16: NONLIN 64^3 6.9, 8.3,
+// 12.0, 19.5; 96^3 15.4, 15.9, 16.5, 22.0; LIN 192^3 85, 74.5, 72.0, 72.3;
+// 512^3 1239, 1107, 1046, 1012.
+int z_march_pair(const ptd_params& p)
+{
+    const long long bxy = ceil_div(p.nx - 2, 62) * ceil_div(p.ny - 2, 7);
+    const long long sm = sm_count();
+    return march_length(16, 4, 4 * sm, 7 * sm / 4, [&](int m) { return bxy * ceil_div(p.nz - 2, m); });
+}
+
 // March of the rebased form's base kernel (rows in 2D, planes in 3D, per warp
 // of 32 cells): us of a rebase at march 32 and at the march taken: 2D NONLIN
 // 256^2 124, 28 (1); 600x500 134, 53 (4); 2048^2 506, 457 (8); 3D NONLIN
@@ -137,7 +155,8 @@ LaunchCfg tuned_config(const ptd_params& p)
         }
     } else if (p.ndim == 3 && (p.precision == PTD_PREC_FP32_RB || p.precision == PTD_PREC_FP32_DC)) {
         c.rows3d = 16;
-        c.chunk3d = z_march16(p);
+        const bool pair = p.precision == PTD_PREC_FP32_RB && rb3d_pair(p.model, p.nx, p.ny, p.nz);
+        c.chunk3d = pair ? z_march_pair(p) : z_march16(p);
     } else if (p.ndim == 3) {
         // The FP64-accuracy forms: 256-thread CTAs of 31 x 7 updated cells.
         // Their per-plane barrier joins half the warps of 512-thread CTAs (31

@@ -746,29 +746,29 @@ namespace {
 
 cudaError_t adj_launch_rb(ptd_adj* A, int par, bool check)
 {
-    const dim3 blk(32, 16);
-    const int tx = (A->g.nx - 2 + 30) / 31, ty = (A->g.ny - 2 + 14) / 15;
+    const dim3 blk(32, 8);
+    const int tx = (A->g.nx - 2 + 30) / 31, ty = (A->g.ny - 2 + 6) / 7;
     const int ch = A->cfg.chunk3d;
     const dim3 grid(tx, ty, (A->g.nz - 2 + ch - 1) / ch);
     const AdjArgs* ap = A->d_rbargs[par];
     if (A->expm) {
-        if (check) return launch_pdl(adj3d_kernel<F32, true, true, 16, true>, grid, blk, A->s, ap, ch);
-        return launch_pdl(adj3d_kernel<F32, true, false, 16, true>, grid, blk, A->s, ap, ch);
+        if (check) return launch_pdl(adj3d_kernel<F32, true, true, 8, true>, grid, blk, A->s, ap, ch);
+        return launch_pdl(adj3d_kernel<F32, true, false, 8, true>, grid, blk, A->s, ap, ch);
     }
-    if (check) return launch_pdl(adj3d_kernel<F32, false, true, 16, true>, grid, blk, A->s, ap, ch);
-    return launch_pdl(adj3d_kernel<F32, false, false, 16, true>, grid, blk, A->s, ap, ch);
+    if (check) return launch_pdl(adj3d_kernel<F32, false, true, 8, true>, grid, blk, A->s, ap, ch);
+    return launch_pdl(adj3d_kernel<F32, false, false, 8, true>, grid, blk, A->s, ap, ch);
 }
 
 cudaError_t adj_launch(ptd_adj* A, int par, bool check)
 {
-    const dim3 blk(32, 16);
-    const int tx = (A->g.nx - 2 + 30) / 31, ty = (A->g.ny - 2 + 14) / 15;
+    const dim3 blk(32, 8);
+    const int tx = (A->g.nx - 2 + 30) / 31, ty = (A->g.ny - 2 + 6) / 7;
     const int ch = A->cfg.chunk3d;
     const dim3 grid(tx, ty, (A->g.nz - 2 + ch - 1) / ch);
     const AdjArgs* ap = A->d_args[par];
 #define ADJ(NT, EX)                                                                          \
-    return check ? launch_pdl(adj3d_kernel<NT, EX, true, 16>, grid, blk, A->s, ap, ch)         \
-                 : launch_pdl(adj3d_kernel<NT, EX, false, 16>, grid, blk, A->s, ap, ch)
+    return check ? launch_pdl(adj3d_kernel<NT, EX, true, 8>, grid, blk, A->s, ap, ch)         \
+                 : launch_pdl(adj3d_kernel<NT, EX, false, 8>, grid, blk, A->s, ap, ch)
     if (A->df64) {
         if (A->expm) ADJ(DF64, true);
         else ADJ(DF64, false);
@@ -1066,7 +1066,7 @@ extern "C" int ptd_adj_create(ptd_adj** out, const ptd_params* p)
     A->rb = p->precision == PTD_PREC_FP32_RB;
     A->expm = p->model == PTD_MODEL_NONLIN_EXPM;
     derive(A->p, A->dv);
-    A->cfg.chunk3d = z_march16(A->p);   // every form's kernel has 16-row CTAs
+    A->cfg.chunk3d = z_march8(A->p, A->rb ? 2 : 4);   // every form's kernel has 8-row CTAs
     {   // stagnation window: ~2 n_max iterations, the PT iteration's own time scale
         const int nmax = std::max(p->nx, std::max(p->ny, p->nz));
         A->stall = std::max(10, (2 * nmax + A->nchk - 1) / A->nchk);
@@ -1111,7 +1111,7 @@ extern "C" int ptd_adj_create(ptd_adj** out, const ptd_params* p)
         rc = set_error(PTD_ENOMEM, "adjoint: cudaMallocHost failed");
     // residual slots: one per CTA of a check launch, one per CTA of the
     // grid-stride reductions (sums of squares, misfit, rebase)
-    A->nparts = (long long)((A->g.nx - 2 + 30) / 31) * ((A->g.ny - 2 + 14) / 15) *
+    A->nparts = (long long)((A->g.nx - 2 + 30) / 31) * ((A->g.ny - 2 + 6) / 7) *
                 ((A->g.nz - 2 + A->cfg.chunk3d - 1) / A->cfg.chunk3d);
     A->nparts64 = fill_blocks();
     if (!rc) rc = al((void**)&A->parts, (size_t)A->nparts * sizeof(double));

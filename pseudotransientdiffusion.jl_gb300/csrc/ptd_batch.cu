@@ -408,9 +408,11 @@ __global__ void tofloat_batch_kernel(const double* src, float* dst, long long n)
 // entry after one load, so once most instances have stopped a launch costs
 // their remaining work rather than a table walk per work item of the whole
 // batch.  (A persistent grid walking the list held 74-98 registers against
-// the march's 40-64.)
+// the march's 40-64.)  The check variants are held to 40 registers (46-76
+// without a bound): a step of 48 LINSTEP instances of 64^2 to 512^2 7.62 ms
+// without, 7.54 at 48, 7.45 at 40, 7.80 at 32.
 template <int MODEL, bool CHECK, int TB>
-__global__ void __launch_bounds__(256) rb2d_batch_kernel(const RbArgs* __restrict__ tab,
+__global__ void __launch_bounds__(256, CHECK ? 6 : 0) rb2d_batch_kernel(const RbArgs* __restrict__ tab,
                                                          const int4* __restrict__ work,
                                                          const int* __restrict__ active, const int* nactive,
                                                          int chunk)

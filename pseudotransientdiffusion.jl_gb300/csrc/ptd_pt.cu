@@ -56,9 +56,13 @@ __global__ void __launch_bounds__(256, CHECK ? 4 : 6) pt2d_kernel(PTArgs a, int 
 // Resident CTAs per SM the register allocation must allow: 48 warps (3 CTAs
 // of 16 warps) for the plain iterations of the LIN and NONLIN models, which
 // fit in 40 registers (DFH NONLIN with a 24-byte spill), 32 warps for the
-// check iterations and the models with a per-cell field (more live values).
+// check iterations and the models with a per-cell field (more live values),
+// 40 for the check iterations of the double-float forms (8 rows; a check of
+// DF64 LIN 126^3 22 us over a plain iteration at 32 warps, 18 at 40; FP64 is
+// slower at 24 or 40).
 template <class N, int MODEL, bool CHECK, int R>
-__global__ void __launch_bounds__(32 * R, (CHECK || MODEL == LINSTEP || MODEL == NONLIN_EXPM) ? 32 / R : 48 / R)
+__global__ void __launch_bounds__(32 * R, CHECK ? (N::native || R > 8 ? 32 : 40) / R
+                                                : (MODEL == LINSTEP || MODEL == NONLIN_EXPM) ? 32 / R : 48 / R)
     pt3d_kernel(PTArgs a, int chunk)
 {
     pdl_begin();
@@ -74,9 +78,10 @@ __global__ void __launch_bounds__(32 * R, (CHECK || MODEL == LINSTEP || MODEL ==
 // (ptd_pair_body.cuh), 62-cell tiles.  (The same pairing in 3D was slower than
 // the one-cell kernel at 512^3 -- DF64 2244 against 2045 us: its 60-96
 // registers leave 16-32 resident warps per SM for a march with a barrier per
-// plane.)
+// plane.)  Check variants at 80 registers: DFH 1021x1500 21 -> 19 us over a
+// plain iteration (24-28 at 64 and 48).
 template <class N, int MODEL, bool CHECK>
-__global__ void __launch_bounds__(256) pt2d_pair_kernel(PTArgs a, int chunk)
+__global__ void __launch_bounds__(256, CHECK ? 3 : 0) pt2d_pair_kernel(PTArgs a, int chunk)
 {
     pdl_begin();
     if (step_done(a.done)) return;

@@ -33,9 +33,12 @@ __global__ void __launch_bounds__(256) rb2d_kernel(RbArgs a, int chunk)
     rb2d_body<MODEL, CHECK>(a, blockIdx.x * blockDim.y + threadIdx.y, blockIdx.y, chunk, part, pmax, warp_slot());
 }
 
-// Two iterations per launch, two columns per lane (LIN, NONLIN).
+// Two iterations per launch, two columns per lane (LIN, NONLIN).  The NONLIN
+// check variant is held to the plain one's 64 registers: at its natural 73 a
+// check of 2048^2 cost 43 us more than a plain iteration, 26 so (at 48 39; LIN
+// at 48 or less likewise slower).
 template <int MODEL, bool CHECK>
-__global__ void __launch_bounds__(256) rb2d_tb2_pair_kernel(RbArgs a, int chunk)
+__global__ void __launch_bounds__(256, (MODEL == NONLIN && CHECK) ? 4 : 0) rb2d_tb2_pair_kernel(RbArgs a, int chunk)
 {
     pdl_begin();
     if (rb_skip(a.skip)) return;
@@ -75,17 +78,17 @@ __global__ void __launch_bounds__(512, 2) rb3d_tb2_kernel(RbArgs a, int chunk)
     if (CHECK) block_reduce_residual(a.acc, a.norm_max, part, pmax, a.parts, block_slot());
 }
 
-// 16-warp CTAs of 31 x 15 updated cells.  (32-row tiles, 1024-thread CTAs
+// CTAs of 31 x 15 updated cells, 31 x 7 for small grids (rb3d_rows).  (32-row tiles, 1024-thread CTAs
 // of 31 x 31 cells, gave the same iterates bit for bit but took 1.31 against
 // 1.24 ms per iteration at 512^3: the per-plane barrier of twice the warps.)
-template <int MODEL, bool CHECK>
-__global__ void __launch_bounds__(512) rb3d_kernel(RbArgs a, int chunk)
+template <int MODEL, bool CHECK, int R>
+__global__ void __launch_bounds__(32 * R) rb3d_kernel(RbArgs a, int chunk)
 {
     pdl_begin();
     if (rb_skip(a.skip)) return;
     double part = 0.0;
     unsigned long long pmax = 0ull;
-    rb3d_body<MODEL, CHECK, 16>(a, blockIdx.x, blockIdx.y, blockIdx.z, chunk, part, pmax);
+    rb3d_body<MODEL, CHECK, R>(a, blockIdx.x, blockIdx.y, blockIdx.z, chunk, part, pmax);
     if (CHECK) block_reduce_residual(a.acc, a.norm_max, part, pmax, a.parts, block_slot());
 }
 
@@ -392,8 +395,10 @@ cudaError_t rb_launch_model(const RbArgs& a, int ndim, const LaunchCfg& cfg, cud
         return launch_pdl(rb3d_pair_kernel<MODEL, CHECK>, grid, dim3(32, 8), s, a, cfg.chunk3d);
     } else {
         const int tx = (a.nx - 2 + 30) / 31;
-        dim3 grid(tx, (a.ny - 2 + 14) / 15, (a.nz - 2 + cfg.chunk3d - 1) / cfg.chunk3d);
-        return launch_pdl(rb3d_kernel<MODEL, CHECK>, grid, dim3(32, 16), s, a, cfg.chunk3d);
+        const int R = rb3d_rows(a.nx, a.ny, a.nz);
+        dim3 grid(tx, (a.ny - 2 + R - 2) / (R - 1), (a.nz - 2 + cfg.chunk3d - 1) / cfg.chunk3d);
+        return R == 8 ? launch_pdl(rb3d_kernel<MODEL, CHECK, 8>, grid, dim3(32, 8), s, a, cfg.chunk3d)
+                      : launch_pdl(rb3d_kernel<MODEL, CHECK, 16>, grid, dim3(32, 16), s, a, cfg.chunk3d);
     }
 }
 
@@ -449,7 +454,8 @@ long long rb_check_slots(const RbState* rb)
     const long long nzc = (p.nz - 2 + c.chunk3d - 1) / c.chunk3d;
     if (rb->tblk == 2) return (long long)((p.nx - 2 + 27) / 28) * ((p.ny - 2 + 11) / 12) * nzc;
     if (rb3d_pair(p.model, p.nx, p.ny, p.nz)) return (long long)((p.nx - 2 + 61) / 62) * ((p.ny - 2 + 6) / 7) * nzc;
-    return (long long)((p.nx - 2 + 30) / 31) * ((p.ny - 2 + 14) / 15) * nzc;
+    const int R = rb3d_rows(p.nx, p.ny, p.nz);
+    return (long long)((p.nx - 2 + 30) / 31) * ((p.ny - 2 + R - 2) / (R - 1)) * nzc;
 }
 
 // The grid of rb_base_march_kernel (8 warps per CTA); its CTA count is the

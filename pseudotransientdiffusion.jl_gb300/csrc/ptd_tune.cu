@@ -97,6 +97,21 @@ int z_march_pair(const ptd_params& p)
     return march_length(16, 4, 4 * sm, 7 * sm / 4, [&](int m) { return bxy * ceil_div(p.nz - 2, m); });
 }
 
+// Rows of a CTA of the 3D rebased form's one-cell kernel: 8 while the fields
+// fit the L2 cache (half the warps per barrier), 16 above (less halo).
+int rb3d_rows(long long nx, long long ny, long long nz) { return nx * ny * nz <= 2400000 ? 8 : 16; }
+
+// z march of the 8-row FP32 kernels and of the adjoint, at least per_sm CTAs
+// per SM down to a march of one plane.  A gradient of 72^3 at marches 1, 2, 3,
+// 4, 6: rebased 11.2, 10.4, 10.2, 10.1, 10.5 ms; FP64 37.3, 34.9, 35.6, 36.8,
+// 39.6 (16-row CTAs at their best: 10.4, 38.3).
+int z_march8(const ptd_params& p, int per_sm)
+{
+    const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, 7);
+    const long long sm = sm_count();
+    return march_length(16, 4, 8 * sm, per_sm * sm, [&](int m) { return bxy * ceil_div(p.nz - 2, m); });
+}
+
 // March of the rebased form's base kernel (rows in 2D, planes in 3D, per warp
 // of 32 cells): us of a rebase at march 32 and at the march taken: 2D NONLIN
 // 256^2 124, 28 (1); 600x500 134, 53 (4); 2048^2 506, 457 (8); 3D NONLIN
@@ -156,7 +171,8 @@ LaunchCfg tuned_config(const ptd_params& p)
     } else if (p.ndim == 3 && (p.precision == PTD_PREC_FP32_RB || p.precision == PTD_PREC_FP32_DC)) {
         c.rows3d = 16;
         const bool pair = p.precision == PTD_PREC_FP32_RB && rb3d_pair(p.model, p.nx, p.ny, p.nz);
-        c.chunk3d = pair ? z_march_pair(p) : z_march16(p);
+        const bool rb8 = p.precision == PTD_PREC_FP32_RB && rb3d_rows(p.nx, p.ny, p.nz) == 8;
+        c.chunk3d = pair ? z_march_pair(p) : rb8 ? z_march8(p, 2) : z_march16(p);
     } else if (p.ndim == 3) {
         // The FP64-accuracy forms: 256-thread CTAs of 31 x 7 updated cells.
         // Their per-plane barrier joins half the warps of 512-thread CTAs (31

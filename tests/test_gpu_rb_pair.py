@@ -44,3 +44,26 @@ def test_pair_kernel_marches(name, shape, march):
             sol.iterate(21)
             out.append(sol.get_state())
     assert np.array_equal(out[0], out[1])
+
+
+# the first grids above the line where the one-cell kernel takes 16-row CTAs
+def test_large_one_cell_kernel_is_the_two_iterations_kernel():
+    s = S.SCRIPTS["diff_3D_nonlin_multixpu"]
+    shape = (137, 134, 132)
+    a = solve(s, shape, precision="fp32_rb", itmax=40)
+    b = solve(s, shape, precision="fp32_rb", itmax=40, rb_tblock_3d=True)
+    assert a[0] == b[0] and np.array_equal(a[2], b[2])
+
+
+@pytest.mark.parametrize("shape", [(137, 134, 132), (133, 136, 132)])
+def test_one_cell_kernel_above_and_below_the_line(shape):
+    """Either solver stops a step at an RMS residual of tol, so the solutions
+    differ by dt 2 tol at most (the step's operator is at least 1/dt)."""
+    s = S.SCRIPTS["diff_3D_linstep_multixpu"]
+    out = []
+    for prec in ("fp64", "fp32_rb"):
+        H = S.initial_condition(s, *shape)
+        with ptdiff.Solver(ptdiff.make_params(s, shape, precision=prec, nt=1)) as sol:
+            sol.solve(H, S.step_field(s, *shape))
+        out.append(H)
+    assert np.sqrt(np.mean((out[0] - out[1]) ** 2)) <= s.dt * 2 * s.tol

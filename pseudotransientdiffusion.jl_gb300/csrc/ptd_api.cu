@@ -278,7 +278,7 @@ struct ptd_ctx : ptd_ctx_base {
     DevState* h_st = nullptr;     // pinned mirror of *st (line, flow: written by the kernel, with a HostSteps after it)
     bool line = false;            // 1D: steps are one launch of the line kernel, in place on H[cur], W[0][cur]
     LinePlan lplan;
-    FlowPlan flow;                // 2D FP64: steps are one launch of the flow kernel (rows > 0)
+    FlowPlan flow;                // 2D, 3D FP64: steps are one launch of the flow kernel (rows > 0)
     void* flow_mem = nullptr;     // its exchange buffers
     unsigned flow_tag = 1;        // tags used so far
     cudaGraphExec_t gstep[2] = {nullptr, nullptr};   // one physical step's check loop, per start parity
@@ -580,9 +580,9 @@ extern "C" int ptd_create(ptd_ctx** out, const ptd_params* p)
     c->errcap = (p->nchk <= p->itmax ? p->itmax / p->nchk : 0) + 2;
     c->line = p->ndim == 1 && p->precision == PTD_PREC_FP64 && p->resid_mode == PTD_RESID_MIXED &&
               line_plan(p->model, p->nx, p->nchk, c->lplan);
-    if (p->ndim == 2 && p->precision == PTD_PREC_FP64 && p->resid_mode == PTD_RESID_MIXED &&
+    if (p->ndim > 1 && p->precision == PTD_PREC_FP64 && p->resid_mode == PTD_RESID_MIXED &&
         !(p->flags & PTD_FLAG_AUTOTUNE))
-        flow_plan(p->model, p->nx, p->ny, c->flow);
+        flow_plan(p->model, p->ndim, p->nx, p->ny, p->nz, c->flow);
     if (!rc && c->flow.rows) rc = alloc(&c->flow_mem, flow_bytes(c->flow));
     if ((c->line || c->flow.rows) && c->errcap < 1 << 30) c->errcap += kHostErr;   // room for several steps
     if (!rc) rc = alloc((void**)&c->errhist, (size_t)c->errcap * sizeof(double));

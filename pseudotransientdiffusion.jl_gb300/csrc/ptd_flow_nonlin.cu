@@ -1,8 +1,11 @@
-// ptd_flow_nonlin.cu -- the one-launch 2D step of the NONLIN model (ptd_flow.cuh).
-#include "ptd_flow.cuh"
+// ptd_flow_nonlin.cu -- the flow kernels of the NONLIN model (ptd_flow.cuh, ptd_flow3.cuh).
+#include "ptd_flow3.cuh"
 
 namespace ptd {
 
-const void* flow_kernel_nonlin(int rows) { return flow_kernel_of<NONLIN>(rows); }
+const void* flow_kernel_nonlin(int rows, int planes, int warps)
+{
+    return planes ? flow3_kernel_of<NONLIN>(rows, planes, warps) : flow_kernel_of<NONLIN>(rows);
+}
 
 }  // namespace ptd

@@ -185,7 +185,12 @@ LaunchCfg tuned_config(const ptd_params& p)
         c.rows3d = 8;
         const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, 7);
         auto ctas = [&](int m) { return bxy * ceil_div(p.nz - 2, m); };
-        c.chunk3d = ctas(32) >= 52 * sm ? 32 : march_length(16, 4, 16 * sm, 2 * sm, ctas);
+        // below 4 planes the line is where a shorter march no longer paid: FP64
+        // 66^3 at 4, 2 planes 22.0, 21.0 (480, 960 CTAs), 80^3 27.6, 26.3
+        // (720, 1440), 96^3 44.0, 43.2 (1344, 2632); DFH 62x72x66 13.3, 11.7
+        // (320, 640), 80^3 19.3, 19.4
+        const long long lo = (p.precision == PTD_PREC_FP64 ? 5 : 3) * sm;
+        c.chunk3d = ctas(32) >= 52 * sm ? 32 : march_length(16, 4, 16 * sm, lo, ctas);
     }
     return c;
 }

@@ -177,15 +177,17 @@ PTD_API int ptd_iterate(ptd_ctx* ctx, int32_t niter);  /* niter PT iterations, n
 PTD_API int ptd_get_state(ptd_ctx* ctx, double* H);    /* H out */
 
 /* Launch shape of one iteration per launch: {warps per 2D CTA, rows per 2D y
- * march, warps per 3D CTA, planes per 3D z march}.  (FP64 grids whose step is
- * one launch use none of it until a shape is set: 1D up to 13824 cells, 2D
- * LIN, LINSTEP and NONLIN up to about 550000 cells, mixed residual.) */
+ * march, warps per 3D CTA, planes per 3D z march}.  (FP64 grids that take
+ * whole steps in one launch use none of it until a shape is set: 1D up to
+ * 13824 cells; LIN, LINSTEP and NONLIN in 2D up to about 470000 cells (LIN
+ * 560000) and in 3D from 32768 to about 260000 cells (LIN 300000); mixed
+ * residual.) */
 PTD_API int ptd_launch_config(ptd_ctx* ctx, int32_t cfg[4]);
 /* Set it (e.g. a shape found by PTD_FLAG_AUTOTUNE on another context of the
  * same size): warps per 2D CTA in {1,2,4,8}, rows per 2D march in [1,4096],
- * warps per 3D CTA in {8,16} (the FP32 forms use 16), planes per 3D march in
- * [1,4096].  The state is kept; a 2D context runs one iteration per launch
- * from then on. */
+ * warps per 3D CTA in {8,16} (16 for the FP32 forms, which choose their rows
+ * themselves), planes per 3D march in [1,4096].  The state is kept; a 2D or 3D
+ * context runs one iteration per launch from then on. */
 PTD_API int ptd_set_launch_config(ptd_ctx* ctx, const int32_t cfg[4]);
 
 /* The context's CUDA stream (cudaStream_t) and a device synchronize of it. */
@@ -193,7 +195,8 @@ PTD_API void* ptd_stream(ptd_ctx* ctx);
 PTD_API int ptd_sync(ptd_ctx* ctx);
 
 /* Counters since ptd_create: kernels launched by the library (each kernel of
- * a replayed CUDA graph counts) and PT iterations executed. */
+ * a replayed CUDA graph counts; several steps in one launch count as one) and
+ * PT iterations executed. */
 PTD_API int ptd_counters(ptd_ctx* ctx, int64_t* kernel_launches, int64_t* pt_iterations);
 
 PTD_API void ptd_destroy(ptd_ctx* ctx);

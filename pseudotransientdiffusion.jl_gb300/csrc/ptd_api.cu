@@ -10,9 +10,12 @@
 // with the iterations, the checks and the stopping decision all on the GPU:
 // one check block (nchk fused PT kernels, the last one also forming the
 // residual, then a one-thread judge kernel that computes err and sets a done
-// flag) is the body of a WHILE node of a CUDA graph, which the judge ends, so one graph launch runs a whole physical step and the host reads the
-// small device state once per step.  The iteration count is exactly the
-// reference's (the first multiple of nchk at which err <= tol).
+// flag) is the body of a WHILE node of a CUDA graph, which the judge ends, so
+// one graph launch runs a whole physical step and the host reads the small
+// device state once per step.  FP64 grids that fit the SMs take several steps
+// in one kernel launch instead (ptd_line.cu, ptd_flow.cuh, ptd_flow3.cuh).  The
+// iteration count is exactly the reference's (the first multiple of nchk at
+// which err <= tol).
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>

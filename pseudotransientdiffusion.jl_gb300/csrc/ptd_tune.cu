@@ -69,9 +69,10 @@ long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 
 }  // namespace
 
-// z march of the 16-row FP32 kernels (rebased form, adjoint): us per
-// iteration at march 16 and at the march taken: rebased NONLIN 32^3 22.0, 7.5
-// (1); 64^3 22.6, 11.4 (4); 128^3 47.8, 44.1 (4); 192^3 119.5, 118.2 (8).
+// z march of the 16-row FP32 kernels (defect correction, rebased form on large
+// grids): us per iteration at march 16 and at the march taken: rebased NONLIN
+// 64^3 19.4, 8.6 (4); 128^3 33.5, 30.4 (4); 192^3 83.7, 82.2 (8); 320x255x191
+// 153 (16).
 int z_march16(const ptd_params& p)
 {
     const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, 15);
@@ -131,9 +132,9 @@ LaunchCfg tuned_config(const ptd_params& p)
         // the memory latency of the march.  Measured over warps {1,2,4,8} x
         // rows {1..64}, us per iteration of a check block at another march (FP32
         // forms and DFH: the former fixed one) and at the one taken here:
-        //   FP64 NONLIN 128^2 5.5 (2 rows), 4.3 (1); 512^2 11.0 (1), 10.4 (4);
-        //     1024^2 29.6 (16), 27.4 (8); 2048^2 95.0 (8), 95.6 (16); 4096^2
-        //     353.9 (8), 351.4 (16), 355.0 (32); LIN and LINSTEP alike
+        //   FP64 NONLIN (grids that do not fit the flow kernel) 768x600 15.2
+        //     (4); 1024^2 30.6 (16), 26.5 (8); 2048^2 92.9 (8), 93.6 (16);
+        //     4096^2 345.8 (8), 340.1 (16), 342.7 (32); LIN and LINSTEP alike
         //   DFH NONLIN (1 x 8) 256^2 12.0, 4.8 (1); 512^2 12.5, 7.8 (2);
         //     1021x1500 29.7, 27.3 (4); 2048^2 62.7 (8)
         //   FP32_RB NONLIN (8 x 32, marches of twice the rows) 256^2 28.9, 4.4
@@ -178,10 +179,10 @@ LaunchCfg tuned_config(const ptd_params& p)
         // Their per-plane barrier joins half the warps of 512-thread CTAs (31
         // x 15 cells) and their tiles waste less of a ragged grid; the larger
         // halo is not what bounds them.  us per iteration, 16 rows x best
-        // march / as taken: FP64 NONLIN 64^3 17.1, 14.2 (2 planes); 128^3
-        // 95.4, 88.0 (4); 256^3 614, 571 (16); 512^3 4438, 4184 (16); LIN
-        // 512^3 4169, 4190; LINSTEP 512^3 5143, 4593 (32); DF64 LIN 128^3 42.3,
-        // 39.4; 512^3 2144, 2149 (32); DFH 512^3 2804, 2756 (32).
+        // march / as taken: FP64 NONLIN 128^3 96.6, 88.4 (4 planes); 256^3
+        // 596, 562 (16); 512^3 4317, 4079 (32); LIN 512^3 3904, 3901; LINSTEP
+        // 512^3 4881, 4496 (32); DF64 LIN 128^3 42.0, 38.9; NONLIN 512^3 2128,
+        // 2142 (32); DFH 512^3 2762, 2726 (32).
         c.rows3d = 8;
         const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, 7);
         auto ctas = [&](int m) { return bxy * ceil_div(p.nz - 2, m); };

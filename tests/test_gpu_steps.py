@@ -69,3 +69,24 @@ def test_nan_ends_the_steps(name, shape):
     with ptdiff.Solver(ptdiff.make_params(s, shape, nt=6)) as sol:
         iters, _, st = sol.solve(H0, raise_on_nan=False)
     assert st == ptdiff._abi.PTD_ENAN and iters[0] > 0 and not iters[1:].any()
+
+
+@pytest.mark.parametrize("name,shape", [("diff_1D_nonlin", (70,)), ("diff_2D_nonlin", (64, 41)), ("diff_2D_nonlin", (61, 40)),
+                                        ("diff_3D_nonlin_multixpu", (32, 9, 10)), ("diff_3D_nonlin_multixpu", (35, 9, 10))])
+@pytest.mark.parametrize("kw", [{}, {"precision": "df64"}, {"precision": "dfh"}, {"precision": "fp32_rb"}, {"autotune": True}])
+def test_a_new_state_leaves_nothing_of_the_last(name, shape, kw):
+    """With rows that fill the pitch and rows that do not, after steps from
+    another state and after the autotuner's: bit for bit a fresh context."""
+    s = S.SCRIPTS[name]
+    H0 = S.initial_condition(s, *shape)
+    out = []
+    for used in (False, True):
+        with ptdiff.Solver(ptdiff.make_params(s, shape, **dict(kw, autotune=kw.get("autotune", False) and used))) as sol:
+            if used:
+                sol.set_state(np.asfortranarray(2.0 * H0 + 1.0))
+                sol.step(1)
+                sol.iterate(3)
+            sol.set_state(H0)
+            sol.iterate(15)
+            out.append(sol.get_state())
+    assert np.array_equal(out[0], out[1])

@@ -69,7 +69,7 @@ DTYPES = {"fp64": "f64", "df64": "df64 (f32x2)", "dfh": "f64 state, df64 (f32x2)
 TRAFFIC = {("3d_nonlin_512", "fp64"): "pt_kernel_3d_nonlin_512.md",
            ("2d_nonlin_4096", "fp64"): "pt_kernel_2d_nonlin_4096.md",
            ("2d_nonlin_4096", "fp32_rb"): "rb2d_tb2_pair_nonlin_4096.md",
-           ("3d_nonlin_512", "fp32_rb"): "rb3d_nonlin_320x255x191.md"}
+           ("3d_nonlin_512", "fp32_rb"): "rb3d_nonlin_256.md"}
 
 
 def log(*a):
@@ -363,13 +363,11 @@ class GridBench:
         if precision == "fp32_rb":
             # one FP32 iteration reads delta, H_b (FP32), the fluxes omega_d, the
             # base flux defects t_b,d and R_b, writes delta and omega_d: (2+3nd+2)*4 B
-            # per cell; where it carries the flux defect q_d (3D; 2D LIN, LINSTEP) it
-            # reads C_b and no t_b,d: (2+2nd+2)*4 B; a launch runs two iterations
-            # (temporal blocking) with an even check cadence in 2D
-            q = nd == 3 or (nd == 2 and self.s.model in (0, 1))
+            # per cell; a launch runs two iterations (temporal blocking) with an even
+            # check cadence in 2D
             tb_ok = nd == 2   # 3D: one iteration per launch unless PTD_FLAG_RB_TBLOCK_3D
             ipl = 2 if tb_ok and self.s.nout % 2 == 0 else 1
-            nbytes = (2 + (2 if q else 3) * nd + 2) * 4 * self.cells
+            nbytes = (2 + 3 * nd + 2) * 4 * self.cells
             kname = {1: "rb1d_kernel", 2: "rb2d_kernel", 3: "rb3d_kernel"}[nd]
             if ipl == 2:
                 kname = "rb2d_tb2_pair_kernel" if nd == 2 and self.s.model in (0, 2) else f"rb{nd}d_tb2_kernel"

@@ -529,7 +529,6 @@ __global__ void __launch_bounds__(256) rb_fold_batch_kernel(const RbFoldArgs* __
 
 // Base quantities of every running instance (of all instances at a step
 // start: use_st = 0), one chunk of an instance's padded field per CTA.
-template <bool Q>
 __global__ void __launch_bounds__(256) rb_base_batch_kernel(const RbBaseArgs* __restrict__ btab, const RbDev* st,
                                                             const int4* __restrict__ fwork, int use_st)
 {
@@ -541,7 +540,7 @@ __global__ void __launch_bounds__(256) rb_base_batch_kernel(const RbBaseArgs* __
     for (int k = threadIdx.x; k < w.z; k += blockDim.x) {
         const long long e = (long long)w.y + k;
         const int ix = (int)(e % b.sy), iy = (int)(e / b.sy);
-        if (ix < b.nx) rb_base_cell<Q>(b, ix, iy, 0, part, pmax);   // padding columns hold no cell
+        if (ix < b.nx) rb_base_cell(b, ix, iy, 0, part, pmax);   // padding columns hold no cell
     }
     block_reduce_residual(b.acc64, b.norm_max, part, pmax, b.parts, blockIdx.x);   // the chunk's slot
 }
@@ -757,13 +756,6 @@ cudaError_t launch_rb_batch(ptd_batch* b, int par, bool check)
 #undef RBK
 }
 
-// The base quantities of the running instances (use_st 0: of all).
-void launch_base_batch(ptd_batch* b, int use_st)
-{
-    if (rb_qform(b->model, 2)) rb_base_batch_kernel<true><<<b->nfwork, 256, 0, b->s>>>(b->btab, b->rdev, b->fwork, use_st);
-    else rb_base_batch_kernel<false><<<b->nfwork, 256, 0, b->s>>>(b->btab, b->rdev, b->fwork, use_st);
-}
-
 // The list of the running instances' work items (after every judge).
 cudaError_t compact_rb(ptd_batch* b)
 {
@@ -866,7 +858,7 @@ int capture_rb(ptd_batch* b)
         err = cudaGetLastError();
     }
     if (err == cudaSuccess) {
-        launch_base_batch(b, 1);
+        rb_base_batch_kernel<<<b->nfwork, 256, 0, b->s>>>(b->btab, b->rdev, b->fwork, 1);
         err = cudaGetLastError();
     }
     if (err == cudaSuccess) {
@@ -1073,7 +1065,7 @@ int fill_tables_rb(ptd_batch* b)
                 a.wout[d] = b->w32[dd][q ^ 1] + o;
                 a.tb[d] = b->tb32[dd] + o;
             }
-            a.Rb = b->Rb32 ? b->Rb32 + o : nullptr;
+            a.Rb = b->Rb32 + o;
             a.Cb = b->Cb32 + o;
             a.Hf = b->Hf + o;
             a.Df = b->Df ? b->Df + o : nullptr;
@@ -1093,7 +1085,6 @@ int fill_tables_rb(ptd_batch* b)
             f.wb[d] = b->wb64[d] + o;
             f.w[d][0] = b->w32[d][0] + o;
             f.w[d][1] = b->w32[d][1] + o;
-            f.tb[d] = rb_qform(b->model, 2) ? b->tb32[d] + o : nullptr;
         }
         RbBaseArgs& g = bt[i];
         std::memset(&g, 0, sizeof(g));
@@ -1111,10 +1102,9 @@ int fill_tables_rb(ptd_batch* b)
         for (int d = 0; d < 2; ++d) {
             g.wb[d] = b->wb64[d] + o;
             g.tb[d] = b->tb32[d] + o;
-            for (int q = 0; q < 2; ++q) g.q[d][q] = rb_qform(b->model, 2) ? b->w32[d][q] + o : nullptr;
         }
         g.D = b->D64 ? b->D64 + o : nullptr;
-        g.Rb = b->Rb32 ? b->Rb32 + o : nullptr;
+        g.Rb = b->Rb32 + o;
         g.Cb = b->Cb32 + o;
         g.Hf = b->Hf + o;
         g.acc64 = &b->rdev[i].acc64;
@@ -1451,7 +1441,7 @@ extern "C" int ptd_batch_create(ptd_batch** out, const ptd_batch_params* p, cons
             if (!rc) rc = balloc(&b->wb64[d], db);
             if (!rc) rc = balloc(&b->tb32[d], fb);
         }
-        if (!rc && !rb_qform(p->model, 2)) rc = balloc(&b->Rb32, fb);
+        if (!rc) rc = balloc(&b->Rb32, fb);
         if (!rc) rc = balloc(&b->Cb32, fb);
         if (!rc) rc = balloc(&b->rdev, n * sizeof(RbDev));
         for (int q = 0; q < 2 && !rc; ++q) rc = balloc(&b->rbtab[q], n * sizeof(RbArgs));
@@ -1467,7 +1457,7 @@ extern "C" int ptd_batch_create(ptd_batch** out, const ptd_batch_params* p, cons
             // faces past the last one of each direction are read (never used) by the halo lanes
             float* zf[] = {b->tb32[0], b->tb32[1], b->Rb32, b->Cb32};
             for (float* z : zf)
-                if (z && cudaMemset(z, 0, fb) != cudaSuccess) rc = bfail(PTD_ECUDA, "batch: cudaMemset failed");
+                if (cudaMemset(z, 0, fb) != cudaSuccess) rc = bfail(PTD_ECUDA, "batch: cudaMemset failed");
             if (cudaMemset(b->rdev, 0, n * sizeof(RbDev)) != cudaSuccess)
                 rc = bfail(PTD_ECUDA, "batch: cudaMemset failed");
         }
@@ -1665,7 +1655,7 @@ static int batch_rb_step(ptd_batch* b, int32_t* iters, double* err_last, int* na
     const int n = b->ninst, nb = (n + 127) / 128;
     rb_reset_batch_kernel<<<nb, 128, 0, b->s>>>(b->rdev, n);
     BCK(cudaGetLastError());
-    launch_base_batch(b, 0);
+    rb_base_batch_kernel<<<b->nfwork, 256, 0, b->s>>>(b->btab, b->rdev, b->fwork, 0);
     BCK(cudaGetLastError());
     rb_base_judge_batch_kernel<<<1, 256, 0, b->s>>>(b->rdev, n, b->bp.tol, b->norm_den, b->bp.norm == PTD_NORM_MAX,
                                                     cudaGraphConditionalHandle{}, 0, b->passes, b->parts64,

@@ -137,18 +137,6 @@ __device__ __forceinline__ float d2f_bits(double x)
     return __uint_as_float(r);
 }
 
-// A double rounded to the nearest float (ties to even, __double2float_rn) with
-// integer operations wherever the result is a normal number.
-__device__ __forceinline__ float d2f_rn_bits(double x)
-{
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const unsigned ef = ((hi >> 20) & 0x7ffu) - 896u;   // the float's biased exponent
-    if (ef - 1u >= 254u) return __double2float_rn(x);
-    const unsigned m = (ef << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29), rest = lo & 0x1fffffffu;
-    const unsigned up = rest > 0x10000000u - (m & 1u) ? 1u : 0u;   // above half, or half of an odd one
-    return __uint_as_float((hi & 0x80000000u) | (m + up));
-}
-
 __device__ __forceinline__ float frcp(float x)
 {
     float r;

@@ -42,7 +42,7 @@ FParams fparams(const Derived& dv);
 LaunchCfg tuned_config(const ptd_params& p);
 int z_march16(const ptd_params& p);
 int z_march8(const ptd_params& p, int per_sm);
-int rb3d_rows(long long nx, long long ny, long long nz);
+int rb3d_rows(int model, long long nx, long long ny, long long nz);
 bool rb3d_pair(int model, long long nx, long long ny, long long nz);
 int z_march_pair(const ptd_params& p);
 int rb_base_march(const ptd_params& p);

@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(512, 2) rb3d_tb2_kernel(RbArgs a, int chunk)
     if (CHECK) block_reduce_residual(a.acc, a.norm_max, part, pmax, a.parts, block_slot());
 }
 
-// CTAs of 31 x 15 updated cells, 31 x 7 for small grids (rb3d_rows).  (32-row tiles, 1024-thread CTAs
+// CTAs of 31 x 7 updated cells, 31 x 15 for large LIN grids (rb3d_rows).  (32-row tiles, 1024-thread CTAs
 // of 31 x 31 cells, gave the same iterates bit for bit but took 1.31 against
 // 1.24 ms per iteration at 512^3: the per-plane barrier of twice the warps.)
 template <int MODEL, bool CHECK, int R>
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256) rb_base_kernel(RbBaseArgs b, const RbDev*
          t += (long long)gridDim.x * blockDim.x) {
         const int ix = (int)(t % b.nx);
         const long long rest = t / b.nx;
-        rb_base_cell<false>(b, ix, (int)(rest % b.ny), (int)(rest / b.ny), part, pmax);
+        rb_base_cell(b, ix, (int)(rest % b.ny), (int)(rest / b.ny), part, pmax);
     }
     block_reduce_residual(b.acc64, b.norm_max, part, pmax, b.parts, blockIdx.x);
 }
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256) rb_base_kernel(RbBaseArgs b, const RbDev*
 // first step evaluate theirs, and in 3D both y faces are evaluated per cell.
 // Every face is the same rb_u64 evaluation, so the quantities are
 // rb_base_cell's bit for bit; the residual goes into the block's slot.
-template <int NDIM, bool Q>
+template <int NDIM>
 __global__ void __launch_bounds__(256) rb_base_march_kernel(RbBaseArgs b, const RbDev* st, int chunk)
 {
     if (st && st->step_done) return;   // uniform over the grid
@@ -168,36 +168,39 @@ __global__ void __launch_bounds__(256) rb_base_march_kernel(RbBaseArgs b, const 
             const bool min_ = k >= 1 && k <= nm - 2;
             const bool inner = xin && yin && min_;
             // x faces: right by every lane, left from the lane below
-            const double ur = ixc <= b.nx - 2 ? rb_u64<Q>(b, c, c + 1) : 0.0;
+            const double ur = ixc <= b.nx - 2 ? rb_u64(b, c, c + 1) : 0.0;
             double ul = __shfl_up_sync(FULL, ur, 1);
-            if (lane == 0 && inner) ul = rb_u64<Q>(b, c - 1, c);
+            if (lane == 0 && inner) ul = rb_u64(b, c - 1, c);
             // march faces: above now, below from the previous step
-            const double uup = k <= nm - 2 ? rb_u64<Q>(b, c, c + sm) : 0.0;
-            if (k == k0 && inner) udn = rb_u64<Q>(b, c - sm, c);
+            const double uup = k <= nm - 2 ? rb_u64(b, c, c + sm) : 0.0;
+            if (k == k0 && inner) udn = rb_u64(b, c - sm, c);
             if (own) {
-                b.Hf[c] = rb_f32<Q>(b.H[c]);
+                b.Hf[c] = __double2float_rn(b.H[c]);
                 const int dm = NDIM - 1;   // the march direction's index
-                if (ixc <= b.nx - 2) rb_base_face<Q>(b, 0, c, ur);
-                if (k <= nm - 2) rb_base_face<Q>(b, dm, c, uup);
+                if (ixc <= b.nx - 2) b.tb[0][c] = (float)(b.wb[0][c] + ur);
+                if (k <= nm - 2) b.tb[dm][c] = (float)(b.wb[dm][c] + uup);
                 double uyr = 0.0;
                 if (NDIM == 3 && iy <= b.ny - 2) {
-                    uyr = rb_u64<Q>(b, c, c + b.sy);
-                    rb_base_face<Q>(b, 1, c, uyr);
+                    uyr = rb_u64(b, c, c + b.sy);
+                    b.tb[1][c] = (float)(b.wb[1][c] + uyr);
                 }
                 if (inner) {
                     // the order of rb_base_cell: x, y, z
-                    double divu = fma(ur - ul, b.sig[0], 0.0);
-                    if (NDIM == 3) divu = fma(uyr - rb_u64<Q>(b, c - b.sy, c), b.sig[1], divu);
+                    double divw = 0.0, divu = 0.0;
+                    divw = fma(b.wb[0][c] - b.wb[0][c - 1], b.sig[0], divw);
+                    divu = fma(ur - ul, b.sig[0], divu);
+                    if (NDIM == 3) {
+                        const double uyl = rb_u64(b, c - b.sy, c);
+                        divw = fma(b.wb[1][c] - b.wb[1][c - b.sy], b.sig[1], divw);
+                        divu = fma(uyr - uyl, b.sig[1], divu);
+                    }
+                    divw = fma(b.wb[dm][c] - b.wb[dm][c - sm], b.sig[dm], divw);
                     divu = fma(uup - udn, b.sig[dm], divu);
                     const double dh = (b.H[c] - b.Hold[c]) * b.rdt;
-                    if (!Q) {
-                        double divw = fma(b.wb[0][c] - b.wb[0][c - 1], b.sig[0], 0.0);
-                        divw = fma(b.wb[dm][c] - b.wb[dm][c - sm], b.sig[dm], divw);
-                        b.Rb[c] = rb_f32<Q>(dh + divw);
-                    }
+                    b.Rb[c] = (float)(dh + divw);
                     const double cb = divu - dh;
-                    b.Cb[c] = rb_f32<Q>(cb);
                     if (NDIM == 3) b.Cb64[c] = cb;
+                    else b.Cb[c] = (float)cb;
                     accumulate_residual(cb, part, pmax);
                 }
             }
@@ -292,9 +295,8 @@ struct RbState {
     float* d[2] = {nullptr, nullptr};
     float* w[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
     float* tb[3] = {nullptr, nullptr, nullptr};
-    bool q = false;                               // carries the flux defect (rb_qform)
-    float* Rb = nullptr;                          // not in the q form
-    float* Cb = nullptr;                          // base check residual, FP32
+    float* Rb = nullptr;
+    float* Cb = nullptr;                          // base check residual (1D, 2D: FP32)
     double* Cb64 = nullptr;                       // base check residual (3D: FP64)
     float* Hf = nullptr;
     float* Df = nullptr;
@@ -395,7 +397,7 @@ cudaError_t rb_launch_model(const RbArgs& a, int ndim, const LaunchCfg& cfg, cud
         return launch_pdl(rb3d_pair_kernel<MODEL, CHECK>, grid, dim3(32, 8), s, a, cfg.chunk3d);
     } else {
         const int tx = (a.nx - 2 + 30) / 31;
-        const int R = rb3d_rows(a.nx, a.ny, a.nz);
+        const int R = rb3d_rows(MODEL, a.nx, a.ny, a.nz);
         dim3 grid(tx, (a.ny - 2 + R - 2) / (R - 1), (a.nz - 2 + cfg.chunk3d - 1) / cfg.chunk3d);
         return R == 8 ? launch_pdl(rb3d_kernel<MODEL, CHECK, 8>, grid, dim3(32, 8), s, a, cfg.chunk3d)
                       : launch_pdl(rb3d_kernel<MODEL, CHECK, 16>, grid, dim3(32, 16), s, a, cfg.chunk3d);
@@ -454,7 +456,7 @@ long long rb_check_slots(const RbState* rb)
     const long long nzc = (p.nz - 2 + c.chunk3d - 1) / c.chunk3d;
     if (rb->tblk == 2) return (long long)((p.nx - 2 + 27) / 28) * ((p.ny - 2 + 11) / 12) * nzc;
     if (rb3d_pair(p.model, p.nx, p.ny, p.nz)) return (long long)((p.nx - 2 + 61) / 62) * ((p.ny - 2 + 6) / 7) * nzc;
-    const int R = rb3d_rows(p.nx, p.ny, p.nz);
+    const int R = rb3d_rows(p.model, p.nx, p.ny, p.nz);
     return (long long)((p.nx - 2 + 30) / 31) * ((p.ny - 2 + R - 2) / (R - 1)) * nzc;
 }
 
@@ -472,9 +474,8 @@ dim3 base_grid(const RbState* rb)
 cudaError_t launch_base(const RbState* rb, const RbBaseArgs& b, const RbDev* st)
 {
     if (rb->p.ndim == 1) rb_base_kernel<<<fill_blocks(), 256, 0, rb->s>>>(b, st);
-    else if (rb->p.ndim == 3) rb_base_march_kernel<3, true><<<base_grid(rb), dim3(32, 8), 0, rb->s>>>(b, st, rb->base_chunk);
-    else if (rb->q) rb_base_march_kernel<2, true><<<base_grid(rb), dim3(32, 8), 0, rb->s>>>(b, st, rb->base_chunk);
-    else rb_base_march_kernel<2, false><<<base_grid(rb), dim3(32, 8), 0, rb->s>>>(b, st, rb->base_chunk);
+    else if (rb->p.ndim == 2) rb_base_march_kernel<2><<<base_grid(rb), dim3(32, 8), 0, rb->s>>>(b, st, rb->base_chunk);
+    else rb_base_march_kernel<3><<<base_grid(rb), dim3(32, 8), 0, rb->s>>>(b, st, rb->base_chunk);
     return cudaGetLastError();
 }
 
@@ -516,7 +517,6 @@ RbFoldArgs fold_args(const RbState* rb)
         f.wb[d] = rb->wb[d];
         f.w[d][0] = rb->w[d][0];
         f.w[d][1] = rb->w[d][1];
-        f.tb[d] = rb->q ? rb->tb[d] : nullptr;
     }
     return f;
 }
@@ -539,7 +539,6 @@ RbBaseArgs base_args(const RbState* rb)
     for (int d = 0; d < rb->p.ndim; ++d) {
         b.wb[d] = rb->wb[d];
         b.tb[d] = rb->tb[d];
-        for (int q = 0; q < 2; ++q) b.q[d][q] = rb->q ? rb->w[d][q] : nullptr;
     }
     b.D = rb->D;
     b.Rb = rb->Rb;
@@ -707,9 +706,8 @@ int rb_create(const ptd_ctx_base& g, const ptd_params& p, const Derived& dv, cud
         for (int q = 0; q < 2 && !rc; ++q) rc = alloc((void**)&rb->w[d][q], fb);
         if (!rc) rc = alloc((void**)&rb->tb[d], fb);
     }
-    rb->q = rb_qform(p.model, p.ndim);
-    if (!rc && !rb->q) rc = alloc((void**)&rb->Rb, fb);
-    if (!rc) rc = alloc((void**)&rb->Cb, fb);
+    if (!rc) rc = alloc((void**)&rb->Rb, fb);
+    if (!rc && p.ndim < 3) rc = alloc((void**)&rb->Cb, (size_t)g.nfield * sizeof(float));
     if (!rc && p.ndim == 3) rc = alloc((void**)&rb->Cb64, (size_t)g.nfield * sizeof(double));
     if (!rc) rc = alloc((void**)&rb->Hf, fb);
     if (!rc && (p.model == PTD_MODEL_LINSTEP || p.model == PTD_MODEL_NONLIN_EXPM)) rc = alloc((void**)&rb->Df, fb);
@@ -730,7 +728,7 @@ int rb_create(const ptd_ctx_base& g, const ptd_params& p, const Derived& dv, cud
             // faces past the last one of each direction are read (never used) by the halo lanes
             if (e == cudaSuccess) e = cudaMemsetAsync(rb->tb[d], 0, fb, s);
         }
-        if (e == cudaSuccess) e = cudaMemsetAsync(rb->q ? rb->Cb : rb->Rb, 0, fb, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(rb->Rb, 0, fb, s);
         if (e != cudaSuccess) rc = cuda_fail(e, "rb: cudaMemsetAsync");
     }
     if (rc) {

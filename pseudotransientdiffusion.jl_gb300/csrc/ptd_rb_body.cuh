@@ -14,24 +14,19 @@
 // div w_b (the base update residual) and u_d = u(H_b + delta) - u(H_b) are
 // formed so that no FP32 quantity carries H or w themselves, only changes
 // since the base and defects of the base, all of which shrink as the step
-// converges: FP32 rounding is relative to them and sets no floor.  For D = H^3
+// converges: FP32 rounding is relative to them and sets no floor.  (Carrying
+// the flux defect q = t_b + omega instead would read neither t_b nor R_b, 32
+// bytes per cell instead of 40 in 2D and 40 instead of 52 in 3D, but q is
+// rounded relative to t_b from a phase's start and the update takes the FP32
+// difference div q - C_b for R_b: of 1554 LINSTEP instances 12 then stopped
+// after another number of iterations, and the solution of a 3D step lay
+// further from a 64-bit one, 1.82e-13 against 1.65e-13.  Integer face fluxes
+// in the rebase, at most 0.6 ulp off, moved no count but the bits of one field
+// in 25, for 2 % of a batch step.)  For D = H^3
 // (s = H_L + H_R, g = H_R - H_L, s_d, g_d the same of delta)
 //   u_d = s_d (3 s (s + s_d) + s_d^2) g + (s + s_d)^3 g_d.
-// In 3D, and in 2D for LIN and LINSTEP (rb_qform), the flux change is carried
-// as the flux defect q = t_b + omega instead, from q = t_b at a phase's start:
-//   q^{k+1} = q^k - c (q^k + u_d(delta^k))
-//   delta^{k+1} = delta^k - e (delta^k/dt + sum_d sigma_d (q^{k+1}_R - q^{k+1}_L) - C_b)
-// with the base check residual C_b = div u(H_b) - (H_b - Hold)/dt (R_b = sum_d
-// sigma_d (t_bR - t_bL) - C_b).  The iteration then reads neither t_b nor R_b:
-// 32 bytes per cell and launch in 2D instead of 40, 40 in 3D instead of 52.  q
-// is rounded relative to t_b from the start of a phase on, omega only once it
-// has grown to it (1/c iterations): for D = H^3 on fine 2D grids and in 1D the
-// steps then took up to 2 % more iterations (2D 4096^2 6600 against 6500, 1D
-// 4096 6220 against 5850), so those keep omega.  3D and the linear models take
-// the same counts either way (2D 3000x2800 3470 and 3300, 3D 400x300x350 620).
-//
 // Every `phase` (a few hundred iterations) the base is rebased in FP64:
-// H_b += delta, w_b += omega, delta = omega = 0 (q = t_b), and t_b, R_b and the FP64
+// H_b += delta, w_b += omega, delta = omega = 0, and t_b, R_b and the FP64
 // residual of the base are recomputed.  Unlike a defect-correction loop
 // (ptd_dc.cu) that restarts an inner solve from zero for each correction,
 // this keeps the PT iteration's momentum (the fluxes) across rebases, so a
@@ -51,7 +46,6 @@
 #pragma once
 
 #include "ptd_device.cuh"
-#include "ptd_intflux.cuh"
 #include "ptd_kernels.h"
 
 namespace ptd {
@@ -65,12 +59,12 @@ struct RbArgs {
     FParams f;
     const float* din;     // delta (iteration k)
     float* dout;          // delta (iteration k+1)
-    const float* win[3];  // omega, or q
+    const float* win[3];  // omega
     float* wout[3];
-    const float* tb[3];   // base flux defect w_b + u(H_b), per face (not read in the q form)
-    const float* Rb;      // base update residual (not read in the q form)
-    const float* Cb;      // base check residual, rounded to FP32 (1D, 2D and the q form)
-    const double* Cb64;   // base check residual, FP64 (3D; read on check iterations only)
+    const float* tb[3];   // base flux defect w_b + u(H_b), per face
+    const float* Rb;      // base update residual
+    const float* Cb;      // base check residual, rounded to FP32 (1D, 2D; read on check iterations only)
+    const double* Cb64;   // base check residual, FP64 (3D)
     const float* Hf;      // H_b as FP32 (iteration parameters, u_d)
     const float* Df;      // LINSTEP: D, NONLIN_EXPM: exp(m), as FP32
     const int* skip;
@@ -81,12 +75,6 @@ struct RbArgs {
     double* parts;
     int norm_max;
 };
-
-// Whether a form carries the flux defect q (see above).
-__host__ __device__ constexpr bool rb_qform(int model, int ndim)
-{
-    return ndim == 3 || (ndim == 2 && (model == LIN || model == LINSTEP));
-}
 
 struct RbDev {
     int skip;         // PT kernels return at entry: the phase is over or the step done
@@ -116,9 +104,8 @@ __device__ __forceinline__ float rb_e(const FParams& f, float h3)
     return frcp(__fmaf_rn(p, f.fk1, f.frdt));
 }
 
-// One face: new omega (Q: new q; tb is not used), and u_d (the change of the
-// undamped flux) when U.
-template <int MODEL, bool U, bool Q>
+// One face: new omega, and u_d (the change of the undamped flux) when U.
+template <int MODEL, bool U>
 __device__ __forceinline__ float rb_face(const RbArgs& a, float dL, float dR, float hL, float hR, float DL,
                                          float DR, float w, float tb, float& u)
 {
@@ -146,7 +133,7 @@ __device__ __forceinline__ float rb_face(const RbArgs& a, float dL, float dR, fl
         }
     }
     if (U) u = ud;
-    return __fmaf_rn(-c, __fadd_rn(w, Q ? ud : __fadd_rn(tb, ud)), w);
+    return __fmaf_rn(-c, w + (tb + ud), w);
 }
 
 template <int MODEL>
@@ -163,7 +150,7 @@ __device__ __forceinline__ float rb_cell_e(const RbArgs& a, float h, float dmax)
 // work with constant operands, which scalar instructions take for free)
 // scalar.  3 sb is formed as (sb + sb) + sb: sb + sb is exact, so the sum
 // rounds once, like the scalar 3.0f * sb.
-template <int MODEL, bool U, bool Q>
+template <int MODEL, bool U>
 __device__ __forceinline__ float2 rb_face2(const RbArgs& a, float2 dL, float2 dR, float2 hL, float2 hR, float2 DL,
                                            float2 DR, float2 w, float2 tb, float2& u)
 {
@@ -182,7 +169,7 @@ __device__ __forceinline__ float2 rb_face2(const RbArgs& a, float2 dL, float2 dR
         cy = face_c_rn(a.f, __fmul_rn(0.125f, st3.y));
     }
     if (U) u = ud;
-    return fma2(f2(-cx, -cy), add2(w, Q ? ud : add2(tb, ud)), w);
+    return fma2(f2(-cx, -cy), add2(w, add2(tb, ud)), w);
 }
 
 __device__ __forceinline__ bool rb_skip(const int* skip) { return __ldcg(skip) != 0; }
@@ -192,7 +179,6 @@ __device__ __forceinline__ bool rb_skip(const int* skip) { return __ldcg(skip) !
 template <int MODEL, bool CHECK>
 __device__ __forceinline__ void rb1d_body(const RbArgs& a, int bx, float& part, unsigned& pmax)
 {
-    constexpr bool Q = false;
     constexpr bool LS = MODEL == LINSTEP;
     constexpr bool HASD = LS || MODEL == NONLIN_EXPM;   // a per-cell field in Df
     const int i = bx * blockDim.x + threadIdx.x;
@@ -203,13 +189,13 @@ __device__ __forceinline__ void rb1d_body(const RbArgs& a, int bx, float& part, 
     float wr = 0.0f, ur = 0.0f, Dr = 0.0f;
     if (i <= nx - 2) {
         Dr = HASD ? a.Df[i + 1] : 0.0f;
-        wr = rb_face<MODEL, CHECK, Q>(a, dc, a.din[i + 1], hc, a.Hf[i + 1], Dc, Dr, a.win[0][i], a.tb[0][i], ur);
+        wr = rb_face<MODEL, CHECK>(a, dc, a.din[i + 1], hc, a.Hf[i + 1], Dc, Dr, a.win[0][i], a.tb[0][i], ur);
         a.wout[0][i] = wr;
     }
     if (i >= 1 && i <= nx - 2) {
         const float Dl = HASD ? a.Df[i - 1] : 0.0f;
         float ul = 0.0f;
-        const float wl = rb_face<MODEL, CHECK, Q>(a, a.din[i - 1], dc, a.Hf[i - 1], hc, Dl, Dc, a.win[0][i - 1],
+        const float wl = rb_face<MODEL, CHECK>(a, a.din[i - 1], dc, a.Hf[i - 1], hc, Dl, Dc, a.win[0][i - 1],
                                                a.tb[0][i - 1], ul);
         const float e = rb_cell_e<MODEL>(a, hc + dc, LS ? fmaxf(fmaxf(Dl, Dr), Dc) : Dc);
         const float dnew = fmaf(-e, fmaf(dc, a.rdt, a.Rb[i] + (wr - wl) * a.sig[0]), dc);
@@ -226,7 +212,6 @@ template <int MODEL, bool CHECK>
 __device__ __forceinline__ void rb2d_body(const RbArgs& a, int tile, int cy, int chunk, float& part,
                                           unsigned& pmax, long long slot = 0)
 {
-    constexpr bool Q = rb_qform(MODEL, 2);   // carries q, not omega
     constexpr bool LS = MODEL == LINSTEP;
     constexpr bool HASD = LS || MODEL == NONLIN_EXPM;   // a per-cell field in Df
     const int lane = threadIdx.x;
@@ -246,15 +231,14 @@ __device__ __forceinline__ void rb2d_body(const RbArgs& a, int tile, int cy, int
         float wyb = 0.0f, uyb = 0.0f;
         if (upd) {
             Db = HASD ? a.Df[idx - sy] : 0.0f;
-            wyb = rb_face<MODEL, CHECK, Q>(a, a.din[idx - sy], dc, a.Hf[idx - sy], hc, Db, Dc, a.win[1][idx - sy],
-                                           Q ? 0.0f : a.tb[1][idx - sy], uyb);
+            wyb = rb_face<MODEL, CHECK>(a, a.din[idx - sy], dc, a.Hf[idx - sy], hc, Db, Dc, a.win[1][idx - sy],
+                                        a.tb[1][idx - sy], uyb);
             if (j0 == 1) a.wout[1][idx - sy] = wyb;
         }
         for (int j = j0; j < j1; ++j, idx += sy) {
             const float dn = a.din[idx + sy], hn = a.Hf[idx + sy];
             const float wx = a.win[0][idx], wy = a.win[1][idx];
-            const float tbx = Q ? 0.0f : a.tb[0][idx], tby = Q ? 0.0f : a.tb[1][idx];
-            const float base = Q ? -a.Cb[idx] : a.Rb[idx];
+            const float tbx = a.tb[0][idx], tby = a.tb[1][idx], rb = a.Rb[idx];
             const float Dn = HASD ? a.Df[idx + sy] : 0.0f;
             float dr = __shfl_down_sync(FULL, dc, 1);
             float hr = __shfl_down_sync(FULL, hc, 1);
@@ -266,8 +250,8 @@ __device__ __forceinline__ void rb2d_body(const RbArgs& a, int tile, int cy, int
                 if (HASD) Dr = ok ? a.Df[idx + 1] : Dc;
             }
             float ux = 0.0f, uy = 0.0f, wxn = 0.0f, wyn = 0.0f;
-            if (xface) wxn = rb_face<MODEL, CHECK, Q>(a, dc, dr, hc, hr, Dc, Dr, wx, tbx, ux);
-            if (upd) wyn = rb_face<MODEL, CHECK, Q>(a, dc, dn, hc, hn, Dc, Dn, wy, tby, uy);
+            if (xface) wxn = rb_face<MODEL, CHECK>(a, dc, dr, hc, hr, Dc, Dr, wx, tbx, ux);
+            if (upd) wyn = rb_face<MODEL, CHECK>(a, dc, dn, hc, hn, Dc, Dn, wy, tby, uy);
             const float wxl = __shfl_up_sync(FULL, wxn, 1);
             const float uxl = CHECK ? __shfl_up_sync(FULL, ux, 1) : 0.0f;
             const float Dl = HASD ? __shfl_up_sync(FULL, Dc, 1) : 0.0f;
@@ -276,7 +260,7 @@ __device__ __forceinline__ void rb2d_body(const RbArgs& a, int tile, int cy, int
                 a.wout[1][idx] = wyn;
                 const float e = rb_cell_e<MODEL>(a, hc + dc, LS ? fmaxf(fmaxf(fmaxf(Dc, Dl), fmaxf(Dr, Db)), Dn) : Dc);
                 const float div = fmaf(wyn - wyb, a.sig[1], (wxn - wxl) * a.sig[0]);
-                const float dnew = fmaf(-e, fmaf(dc, a.rdt, base + div), dc);
+                const float dnew = fmaf(-e, fmaf(dc, a.rdt, rb + div), dc);
                 a.dout[idx] = dnew;
                 if (CHECK) {
                     const float divu = fmaf(uy - uyb, a.sig[1], (ux - uxl) * a.sig[0]);
@@ -321,7 +305,6 @@ template <int MODEL, bool CHECK>
 __device__ __forceinline__ void rb2d_tb2_body(const RbArgs& a, int tile, int cy, int chunk, float& part,
                                               unsigned& pmax, long long slot = 0)
 {
-    constexpr bool Q = rb_qform(MODEL, 2);   // carries q, not omega
     constexpr bool HASD = MODEL == LINSTEP || MODEL == NONLIN_EXPM;
     const int lane = threadIdx.x;
     const int nx = a.nx, ny = a.ny;
@@ -342,16 +325,14 @@ __device__ __forceinline__ void rb2d_tb2_body(const RbArgs& a, int tile, int cy,
     const float s0 = a.sig[0], s1 = a.sig[1], rdt = a.rdt;
     float u;
 
-    // the base term of the update
-    auto base = [&](long long o) { return Q ? -a.Cb[o] : a.Rb[o]; };
     // level-1 x face of a row at offset o (flux omega of the input state);
     // hr, Dr: the right neighbour's H_b and D, reused by level 2
     auto x1 = [&](long long o, float d, float h, float D, float& tbx, float& hr, float& Dr) {
         const float dr = __shfl_down_sync(FULL, d, 1);
         hr = __shfl_down_sync(FULL, h, 1);
         Dr = HASD ? __shfl_down_sync(FULL, D, 1) : 0.0f;
-        tbx = Q ? 0.0f : a.tb[0][o];
-        return rb_face<MODEL, false, Q>(a, d, dr, h, hr, D, Dr, a.win[0][o], tbx, u);
+        tbx = a.tb[0][o];
+        return rb_face<MODEL, false>(a, d, dr, h, hr, D, Dr, a.win[0][o], tbx, u);
     };
     auto cell = [&](float d, float e, float r, float wx, float wxl, float wy, float wyb) {
         return fmaf(-e, fmaf(d, rdt, r + fmaf(wy - wyb, s1, (wx - wxl) * s0)), d);
@@ -365,25 +346,25 @@ __device__ __forceinline__ void rb2d_tb2_body(const RbArgs& a, int tile, int cy,
     const float DB = HASD ? a.Df[oB] : 0.0f;
     float d1 = a.din[oC], h1 = a.Hf[oC];    // row j0+1 <= ny-1
     float D1 = HASD ? a.Df[oC] : 0.0f;
-    const float tbyA = Q ? 0.0f : a.tb[1][oA];
-    const float wyAB = rb_face<MODEL, false, Q>(a, dA, dB, hA, hB, DA, DB, a.win[1][oA], tbyA, u);  // omega'_y(j0-1/2)
+    const float tbyA = a.tb[1][oA];
+    const float wyAB = rb_face<MODEL, false>(a, dA, dB, hA, hB, DA, DB, a.win[1][oA], tbyA, u);  // omega'_y(j0-1/2)
     float pA = dA;                          // delta'(j0-1)
     if (j0 >= 2) {                          // row j0-1 is interior: level 1 there
         const long long oZ = oA - sy;
         const float dZ = a.din[oZ], hZ = a.Hf[oZ];
         const float DZ = HASD ? a.Df[oZ] : 0.0f;
-        const float wyZA = rb_face<MODEL, false, Q>(a, dZ, dA, hZ, hA, DZ, DA, a.win[1][oZ], Q ? 0.0f : a.tb[1][oZ], u);
+        const float wyZA = rb_face<MODEL, false>(a, dZ, dA, hZ, hA, DZ, DA, a.win[1][oZ], a.tb[1][oZ], u);
         float tbxA, hAr, DAr;
         const float wxA = x1(oA, dA, hA, DA, tbxA, hAr, DAr);
         const float wxAl = __shfl_up_sync(FULL, wxA, 1);
         const float eA = rb_cell_e<MODEL>(a, hA + dA, rb_star<MODEL>(DA, DZ, DB));
-        if (upd1) pA = cell(dA, eA, base(oA), wxA, wxAl, wyAB, wyZA);
+        if (upd1) pA = cell(dA, eA, a.Rb[oA], wxA, wxAl, wyAB, wyZA);
     }
     float tbx0, h0r, D0r;
     float wx1p = x1(oB, dB, hB, DB, tbx0, h0r, D0r);       // omega'_x(j0)
-    float tby0 = Q ? 0.0f : a.tb[1][oB];
-    float wy1p = rb_face<MODEL, false, Q>(a, dB, d1, hB, h1, DB, D1, a.win[1][oB], tby0, u);  // omega'_y(j0+1/2)
-    float r0 = base(oB);
+    float tby0 = a.tb[1][oB];
+    float wy1p = rb_face<MODEL, false>(a, dB, d1, hB, h1, DB, D1, a.win[1][oB], tby0, u);  // omega'_y(j0+1/2)
+    float r0 = a.Rb[oB];
     float p0 = dB;                                         // delta'(j0)
     {
         const float wxl = __shfl_up_sync(FULL, wx1p, 1);
@@ -391,7 +372,7 @@ __device__ __forceinline__ void rb2d_tb2_body(const RbArgs& a, int tile, int cy,
         if (upd1) p0 = cell(dB, eB, r0, wx1p, wxl, wy1p, wyAB);
     }
     float uy2b = 0.0f;
-    float wy2b = rb_face<MODEL, CHECK, Q>(a, pA, p0, hA, hB, DA, DB, wyAB, tbyA, uy2b);   // omega''_y(j0-1/2)
+    float wy2b = rb_face<MODEL, CHECK>(a, pA, p0, hA, hB, DA, DB, wyAB, tbyA, uy2b);   // omega''_y(j0-1/2)
     if (j0 == 1 && upd2) a.wout[1][oA] = wy2b;
     float h0 = hB, D0 = DB, Dm1 = DA;
 
@@ -410,21 +391,21 @@ __device__ __forceinline__ void rb2d_tb2_body(const RbArgs& a, int tile, int cy,
             const float d2 = a.din[o + sy];
             h2 = a.Hf[o + sy];
             if (HASD) D2 = a.Df[o + sy];
-            r1 = base(o);
-            tbx1 = Q ? 0.0f : a.tb[0][o];
-            tby1 = Q ? 0.0f : a.tb[1][o];
+            r1 = a.Rb[o];
+            tbx1 = a.tb[0][o];
+            tby1 = a.tb[1][o];
             const float d1r = __shfl_down_sync(FULL, d1, 1);
             h1r = __shfl_down_sync(FULL, h1, 1);
             if (HASD) D1r = __shfl_down_sync(FULL, D1, 1);
             if (PACKF) {
                 float2 uu;
-                const float2 w1 = rb_face2<MODEL, false, Q>(a, f2(d1), f2(d1r, d2), f2(h1), f2(h1r, h2), f2(D1),
+                const float2 w1 = rb_face2<MODEL, false>(a, f2(d1), f2(d1r, d2), f2(h1), f2(h1r, h2), f2(D1),
                                                          f2(D1r, D2), f2(a.win[0][o], a.win[1][o]), f2(tbx1, tby1), uu);
                 wx1 = w1.x;
                 wy1 = w1.y;
             } else {
-                wx1 = rb_face<MODEL, false, Q>(a, d1, d1r, h1, h1r, D1, D1r, a.win[0][o], tbx1, u);
-                wy1 = rb_face<MODEL, false, Q>(a, d1, d2, h1, h2, D1, D2, a.win[1][o], tby1, u);
+                wx1 = rb_face<MODEL, false>(a, d1, d1r, h1, h1r, D1, D1r, a.win[0][o], tbx1, u);
+                wy1 = rb_face<MODEL, false>(a, d1, d2, h1, h2, D1, D2, a.win[1][o], tby1, u);
             }
             const float wx1l = __shfl_up_sync(FULL, wx1, 1);
             const float e1 = rb_cell_e<MODEL>(a, h1 + d1, rb_star<MODEL>(D1, D0, D2));
@@ -436,15 +417,15 @@ __device__ __forceinline__ void rb2d_tb2_body(const RbArgs& a, int tile, int cy,
         float wx2, wy2, ux2 = 0.0f, uy2 = 0.0f;
         if (PACKF) {
             float2 u2 = f2(0.0f);
-            const float2 w2 = rb_face2<MODEL, CHECK, Q>(a, f2(p0), f2(p0r, p1), f2(h0), f2(h0r, h1), f2(D0), f2(D0r, D1),
+            const float2 w2 = rb_face2<MODEL, CHECK>(a, f2(p0), f2(p0r, p1), f2(h0), f2(h0r, h1), f2(D0), f2(D0r, D1),
                                                      f2(wx1p, wy1p), f2(tbx0, tby0), u2);
             wx2 = w2.x;
             wy2 = w2.y;
             ux2 = u2.x;
             uy2 = u2.y;
         } else {
-            wx2 = rb_face<MODEL, CHECK, Q>(a, p0, p0r, h0, h0r, D0, D0r, wx1p, tbx0, ux2);
-            wy2 = rb_face<MODEL, CHECK, Q>(a, p0, p1, h0, h1, D0, D1, wy1p, tby0, uy2);
+            wx2 = rb_face<MODEL, CHECK>(a, p0, p0r, h0, h0r, D0, D0r, wx1p, tbx0, ux2);
+            wy2 = rb_face<MODEL, CHECK>(a, p0, p1, h0, h1, D0, D1, wy1p, tby0, uy2);
         }
         const float wx2l = __shfl_up_sync(FULL, wx2, 1);
         const float ux2l = CHECK ? __shfl_up_sync(FULL, ux2, 1) : 0.0f;
@@ -457,7 +438,7 @@ __device__ __forceinline__ void rb2d_tb2_body(const RbArgs& a, int tile, int cy,
             a.wout[1][os] = wy2;
             if (CHECK) {
                 const float divu = fmaf(uy2 - uy2b, s1, (ux2 - ux2l) * s0);
-                accumulate_residual32(fmaf(-q, rdt, (Q ? -r0 : a.Cb[os]) + divu), part, pmax);
+                accumulate_residual32(fmaf(-q, rdt, a.Cb[os] + divu), part, pmax);
             }
         }
         // shift the windows
@@ -496,7 +477,6 @@ template <int MODEL, bool CHECK>
 __device__ __forceinline__ void rb2d_tb2_pair_body(const RbArgs& a, int tile, int cy, int chunk, float& part,
                                                    unsigned& pmax, long long slot = 0)
 {
-    constexpr bool Q = rb_qform(MODEL, 2);   // carries q, not omega
     static_assert(MODEL == LIN || MODEL == NONLIN, "the pair kernel serves LIN and NONLIN");
     const int lane = threadIdx.x;
     const int nx = a.nx, ny = a.ny;
@@ -525,12 +505,6 @@ __device__ __forceinline__ void rb2d_tb2_pair_body(const RbArgs& a, int tile, in
     const float2 s0 = f2(a.sig[0]), s1 = f2(a.sig[1]), rdt = f2(a.rdt);
     float2 u;
     auto ld2 = [&](const float* p, long long o) { return *reinterpret_cast<const float2*>(p + o); };
-    auto ldt = [&](int d, long long o) { return Q ? f2(0.0f) : ld2(a.tb[d], o); };
-    auto base = [&](long long o) {   // the base term of the update
-        if (!Q) return ld2(a.Rb, o);
-        const float2 c = ld2(a.Cb, o);
-        return f2(-c.x, -c.y);
-    };
     auto st2 = [&](float* p, long long o, float2 v, bool ma, bool mb) {
         if (ma && mb) {
             *reinterpret_cast<float2*>(p + o) = v;
@@ -557,25 +531,25 @@ __device__ __forceinline__ void rb2d_tb2_pair_body(const RbArgs& a, int tile, in
     const float2 dA = ld2(a.din, oA), hA = ld2(a.Hf, oA);
     const float2 dB = ld2(a.din, oB), hB = ld2(a.Hf, oB);
     float2 d1 = ld2(a.din, oC), h1 = ld2(a.Hf, oC);   // row j0+1 <= ny-1
-    const float2 tbyA = ldt(1, oA);
-    const float2 wyAB = rb_face2<MODEL, false, Q>(a, dA, dB, hA, hB, f2(0.0f), f2(0.0f), ld2(a.win[1], oA), tbyA, u);
+    const float2 tbyA = ld2(a.tb[1], oA);
+    const float2 wyAB = rb_face2<MODEL, false>(a, dA, dB, hA, hB, f2(0.0f), f2(0.0f), ld2(a.win[1], oA), tbyA, u);
     float2 pA = dA;
     if (j0 >= 2) {   // row j0-1 is interior: level 1 there
         const long long oZ = oA - sy;
         const float2 dZ = ld2(a.din, oZ), hZ = ld2(a.Hf, oZ);
-        const float2 wyZA = rb_face2<MODEL, false, Q>(a, dZ, dA, hZ, hA, f2(0.0f), f2(0.0f), ld2(a.win[1], oZ),
-                                                   ldt(1, oZ), u);
-        const float2 wxA = rb_face2<MODEL, false, Q>(a, dA, right(dA), hA, right(hA), f2(0.0f), f2(0.0f),
-                                                  ld2(a.win[0], oA), ldt(0, oA), u);
-        pA = sel(cell2(dA, cell_e2(hA, dA), base(oA), wxA, left(wxA), wyAB, wyZA), dA, u1a, u1b);
+        const float2 wyZA = rb_face2<MODEL, false>(a, dZ, dA, hZ, hA, f2(0.0f), f2(0.0f), ld2(a.win[1], oZ),
+                                                   ld2(a.tb[1], oZ), u);
+        const float2 wxA = rb_face2<MODEL, false>(a, dA, right(dA), hA, right(hA), f2(0.0f), f2(0.0f),
+                                                  ld2(a.win[0], oA), ld2(a.tb[0], oA), u);
+        pA = sel(cell2(dA, cell_e2(hA, dA), ld2(a.Rb, oA), wxA, left(wxA), wyAB, wyZA), dA, u1a, u1b);
     }
     float2 h0r = right(hB);
-    float2 tbx0 = ldt(0, oB), tby0 = ldt(1, oB), r0 = base(oB);
-    float2 wx1p = rb_face2<MODEL, false, Q>(a, dB, right(dB), hB, h0r, f2(0.0f), f2(0.0f), ld2(a.win[0], oB), tbx0, u);
-    float2 wy1p = rb_face2<MODEL, false, Q>(a, dB, d1, hB, h1, f2(0.0f), f2(0.0f), ld2(a.win[1], oB), tby0, u);
+    float2 tbx0 = ld2(a.tb[0], oB), tby0 = ld2(a.tb[1], oB), r0 = ld2(a.Rb, oB);
+    float2 wx1p = rb_face2<MODEL, false>(a, dB, right(dB), hB, h0r, f2(0.0f), f2(0.0f), ld2(a.win[0], oB), tbx0, u);
+    float2 wy1p = rb_face2<MODEL, false>(a, dB, d1, hB, h1, f2(0.0f), f2(0.0f), ld2(a.win[1], oB), tby0, u);
     float2 p0 = sel(cell2(dB, cell_e2(hB, dB), r0, wx1p, left(wx1p), wy1p, wyAB), dB, u1a, u1b);
     float2 uy2b = f2(0.0f);
-    float2 wy2b = rb_face2<MODEL, CHECK, Q>(a, pA, p0, hA, hB, f2(0.0f), f2(0.0f), wyAB, tbyA, uy2b);
+    float2 wy2b = rb_face2<MODEL, CHECK>(a, pA, p0, hA, hB, f2(0.0f), f2(0.0f), wyAB, tbyA, uy2b);
     if (j0 == 1) st2(a.wout[1], oA, wy2b, u2a, u2b);
     float2 h0 = hB;
 
@@ -594,19 +568,19 @@ __device__ __forceinline__ void rb2d_tb2_pair_body(const RbArgs& a, int tile, in
         if (s + 1 <= ny - 2) {   // row s+1 interior (uniform): level 1 there
             const float2 d2 = ld2(a.din, o + sy);
             h2 = ld2(a.Hf, o + sy);
-            r1 = base(o);
-            tbx1 = ldt(0, o);
-            tby1 = ldt(1, o);
+            r1 = ld2(a.Rb, o);
+            tbx1 = ld2(a.tb[0], o);
+            tby1 = ld2(a.tb[1], o);
             h1r = right(h1);
-            wx1 = rb_face2<MODEL, false, Q>(a, d1, right(d1), h1, h1r, f2(0.0f), f2(0.0f), ld2(a.win[0], o), tbx1, u);
-            wy1 = rb_face2<MODEL, false, Q>(a, d1, d2, h1, h2, f2(0.0f), f2(0.0f), ld2(a.win[1], o), tby1, u);
+            wx1 = rb_face2<MODEL, false>(a, d1, right(d1), h1, h1r, f2(0.0f), f2(0.0f), ld2(a.win[0], o), tbx1, u);
+            wy1 = rb_face2<MODEL, false>(a, d1, d2, h1, h2, f2(0.0f), f2(0.0f), ld2(a.win[1], o), tby1, u);
             p1 = sel(cell2(d1, cell_e2(h1, d1), r1, wx1, left(wx1), wy1, wy1p), d1, u1a, u1b);
             d1 = d2;
         }
         // level 2 of row s
         float2 ux2 = f2(0.0f), uy2 = f2(0.0f);
-        const float2 wx2 = rb_face2<MODEL, CHECK, Q>(a, p0, right(p0), h0, h0r, f2(0.0f), f2(0.0f), wx1p, tbx0, ux2);
-        const float2 wy2 = rb_face2<MODEL, CHECK, Q>(a, p0, p1, h0, h1, f2(0.0f), f2(0.0f), wy1p, tby0, uy2);
+        const float2 wx2 = rb_face2<MODEL, CHECK>(a, p0, right(p0), h0, h0r, f2(0.0f), f2(0.0f), wx1p, tbx0, ux2);
+        const float2 wy2 = rb_face2<MODEL, CHECK>(a, p0, p1, h0, h1, f2(0.0f), f2(0.0f), wy1p, tby0, uy2);
         const float2 q = cell2(p0, cell_e2(h0, p0), r0, wx2, left(wx2), wy2, wy2b);
         const long long os = o - sy;
         st2(a.wout[0], os, wx2, oxa, oxb);
@@ -615,8 +589,8 @@ __device__ __forceinline__ void rb2d_tb2_pair_body(const RbArgs& a, int tile, in
         if (CHECK) {
             const float2 ux2l = left(ux2);
             const float2 divu = fma2(sub2(uy2, uy2b), s1, mul2(sub2(ux2, ux2l), s0));
-            if (u2a) accumulate_residual32(fmaf(-q.x, rdt.x, (Q ? -r0.x : a.Cb[os]) + divu.x), part, pmax);
-            if (u2b) accumulate_residual32(fmaf(-q.y, rdt.y, (Q ? -r0.y : a.Cb[os + 1]) + divu.y), part, pmax);
+            if (u2a) accumulate_residual32(fmaf(-q.x, rdt.x, a.Cb[os] + divu.x), part, pmax);
+            if (u2b) accumulate_residual32(fmaf(-q.y, rdt.y, a.Cb[os + 1] + divu.y), part, pmax);
         }
         // shift the windows
         p0 = p1;
@@ -649,7 +623,6 @@ template <int MODEL, bool CHECK, int R>
 __device__ __forceinline__ void rb3d_body(const RbArgs& a, int bx, int by, int bz, int chunk, double& part,
                                           unsigned long long& pmax)
 {
-    constexpr bool Q = true;   // carries q, not omega
     constexpr bool LS = MODEL == LINSTEP;
     constexpr bool HASD = LS || MODEL == NONLIN_EXPM;   // a per-cell field in Df
     __shared__ float sd[2][R][32];
@@ -679,7 +652,8 @@ __device__ __forceinline__ void rb3d_body(const RbArgs& a, int bx, int by, int b
         float wzb = 0.0f, uzb = 0.0f;
         if (upd) {
             Db = HASD ? a.Df[idx - sz] : 0.0f;
-            wzb = rb_face<MODEL, CHECK, Q>(a, a.din[idx - sz], dc, a.Hf[idx - sz], hc, Db, Dc, a.win[2][idx - sz], 0.0f, uzb);
+            wzb = rb_face<MODEL, CHECK>(a, a.din[idx - sz], dc, a.Hf[idx - sz], hc, Db, Dc, a.win[2][idx - sz],
+                                        a.tb[2][idx - sz], uzb);
             if (k0 == 1) a.wout[2][idx - sz] = wzb;
         }
         int p = 0;
@@ -690,7 +664,7 @@ __device__ __forceinline__ void rb3d_body(const RbArgs& a, int bx, int by, int b
         for (int k = k0; k < k1; ++k, idx += sz) {
             const float dn = a.din[idx + sz], hn = a.Hf[idx + sz];
             const float wx = a.win[0][idx], wy = a.win[1][idx], wz = a.win[2][idx];
-            const float base = -a.Cb[idx];
+            const float tbx = a.tb[0][idx], tby = a.tb[1][idx], tbz = a.tb[2][idx], rb = a.Rb[idx];
             const float Dn = HASD ? a.Df[idx + sz] : 0.0f;
             float du, hu, Du = 0.0f;
             if (!top) {
@@ -713,9 +687,9 @@ __device__ __forceinline__ void rb3d_body(const RbArgs& a, int bx, int by, int b
                 if (HASD) Dr = ok ? a.Df[idx + 1] : Dc;
             }
             float ux = 0.0f, uy = 0.0f, uz = 0.0f, wxn = 0.0f, wyn = 0.0f, wzn = 0.0f;
-            if (xface) wxn = rb_face<MODEL, CHECK, Q>(a, dc, dr, hc, hr, Dc, Dr, wx, 0.0f, ux);
-            if (yface) wyn = rb_face<MODEL, CHECK, Q>(a, dc, du, hc, hu, Dc, Du, wy, 0.0f, uy);
-            if (upd) wzn = rb_face<MODEL, CHECK, Q>(a, dc, dn, hc, hn, Dc, Dn, wz, 0.0f, uz);
+            if (xface) wxn = rb_face<MODEL, CHECK>(a, dc, dr, hc, hr, Dc, Dr, wx, tbx, ux);
+            if (yface) wyn = rb_face<MODEL, CHECK>(a, dc, du, hc, hu, Dc, Du, wy, tby, uy);
+            if (upd) wzn = rb_face<MODEL, CHECK>(a, dc, dn, hc, hn, Dc, Dn, wz, tbz, uz);
             if (own_x) a.wout[0][idx] = wxn;
             if (own_y) a.wout[1][idx] = wyn;
             if (upd) a.wout[2][idx] = wzn;
@@ -733,7 +707,7 @@ __device__ __forceinline__ void rb3d_body(const RbArgs& a, int bx, int by, int b
                 const float e = rb_cell_e<MODEL>(
                     a, hc + dc, LS ? fmaxf(fmaxf(fmaxf(Dc, Dl), fmaxf(Dr, Du)), fmaxf(fmaxf(Dd, Db), Dn)) : Dc);
                 const float div = fmaf(wzn - wzb, a.sig[2], fmaf(wyn - wyb, a.sig[1], (wxn - wxl) * a.sig[0]));
-                const float dnew = fmaf(-e, fmaf(dc, a.rdt, base + div), dc);
+                const float dnew = fmaf(-e, fmaf(dc, a.rdt, rb + div), dc);
                 a.dout[idx] = dnew;
                 if (CHECK) {
                     const float uyb = su[p][r - 1][lane];
@@ -763,18 +737,18 @@ __device__ __forceinline__ void rb3d_body(const RbArgs& a, int bx, int by, int b
 // (one aligned 8-byte pair; 1..62 are updated), every pair of faces and cells
 // as one FP32x2 evaluation, and the loads of a plane issued a plane ahead.
 // Each cell's arithmetic is rb3d_body's, operation for operation.  Fewer
-// instructions per cell (NONLIN 320x255x191: 89 against 109 million of a warp), but half the
-// warps; bound by the latency of a plane on small grids and by HBM on large
-// ones.  us per iteration with checks every 10, rb3d_body / here: LIN 64^3 8.0,
-// 6.4; 128^3 26.4, 22.6; 320x255x191 146, 133; 512^3 1164, 1012; NONLIN 64^3
-// 8.6, 6.9; 96^3 17.9, 15.9; 128^3 30.4, 29.4; 192^3 82, 86; 320x255x191 153,
-// 158.  (Staging the loads through a shared-memory ring with cp.async was
-// slower: 128^3 40; so were 16 rows and, for LIN, 32-bit offsets.)
+// instructions per cell, but half the warps: bound by the latency of a plane,
+// and on grids past the L2 cache by HBM like rb3d_body.  us per iteration with
+// checks every 10 at the best march, rebases included, rb3d_body / here: LIN
+// 48^3 5.9, 5.6; 64^3 7.1, 6.5; 96^3 13.4, 12.6; 110^3 16.5, 15.6; 128^3 24.4,
+// 28.1; 320x255x191 153, 152; NONLIN 64^3 8.2, 7.9; 96^3 18.6, 18.5; 110^3 24.0,
+// 21.9; 128^3 35.8, 39.4; 192^3 97, 107; 320x255x191 187, 197.  (Staging the
+// loads through a shared-memory ring with cp.async was slower, and so were 16
+// rows.)
 template <int MODEL, bool CHECK, int R>
 __device__ __forceinline__ void rb3d_pair_body(const RbArgs& a, int bx, int by, int bz, int chunk, double& part,
                                                unsigned long long& pmax)
 {
-    constexpr bool Q = true;   // carries q, not omega
     static_assert(MODEL == LIN || MODEL == NONLIN, "the pair kernel serves LIN and NONLIN");
     __shared__ float2 sd[2][R][32];
     __shared__ float2 sh[2][R][32];
@@ -813,23 +787,28 @@ __device__ __forceinline__ void rb3d_pair_body(const RbArgs& a, int bx, int by, 
     long long idx = (long long)k0 * sz + (long long)jc * sy + cl;
     float2 dc = ld2(a.din, idx), hc = ld2(a.Hf, idx), wzb = z2, uzb = z2;
     if (row) {
-        wzb = rb_face2<MODEL, CHECK, Q>(a, ld2(a.din, idx - sz), dc, ld2(a.Hf, idx - sz), hc, z2, z2,
-                                        ld2(a.win[2], idx - sz), z2, uzb);
+        wzb = rb_face2<MODEL, CHECK>(a, ld2(a.din, idx - sz), dc, ld2(a.Hf, idx - sz), hc, z2, z2,
+                                     ld2(a.win[2], idx - sz), ld2(a.tb[2], idx - sz), uzb);
         if (k0 == 1) st2(a.wout[2], idx - sz, wzb, u0, u1);
     }
     int p = 0;
     sd[0][r][lane] = dc;
     sh[0][r][lane] = hc;
     // the loads of a plane are issued a plane ahead
-    float2 dn = z2, hn = z2, wx = z2, wy = z2, wz = z2, cb = z2, du = dc, hu = hc;
+    float2 dn = z2, hn = z2, wx = z2, wy = z2, wz = z2, tx = z2, ty = z2, tz = z2, rb = z2, du = dc, hu = hc;
     auto load = [&](long long o) {
         dn = ld2(a.din, o + sz);
         hn = ld2(a.Hf, o + sz);
-        if (yf) wy = ld2(a.win[1], o);
+        if (yf) {
+            wy = ld2(a.win[1], o);
+            ty = ld2(a.tb[1], o);
+        }
         if (row) {
             wx = ld2(a.win[0], o);
             wz = ld2(a.win[2], o);
-            cb = ld2(a.Cb, o);
+            tx = ld2(a.tb[0], o);
+            tz = ld2(a.tb[2], o);
+            rb = ld2(a.Rb, o);
         }
         if (top && up_ok) {
             du = ld2(a.din, o + sy);
@@ -845,7 +824,7 @@ __device__ __forceinline__ void rb3d_pair_body(const RbArgs& a, int bx, int by, 
         }
         float2 ux = z2, uy = z2, uz = z2, wxn = z2, wyn = z2, wzn = z2;
         if (yf) {
-            wyn = rb_face2<MODEL, CHECK, Q>(a, dc, du, hc, hu, z2, z2, wy, z2, uy);
+            wyn = rb_face2<MODEL, CHECK>(a, dc, du, hc, hu, z2, z2, wy, ty, uy);
             if (ystore) st2(a.wout[1], idx, wyn, u0, u1);
         }
         sw[p][r][lane] = wyn;
@@ -853,12 +832,12 @@ __device__ __forceinline__ void rb3d_pair_body(const RbArgs& a, int bx, int by, 
         sd[p ^ 1][r][lane] = dn;
         sh[p ^ 1][r][lane] = hn;
         if (row) {
-            wxn = rb_face2<MODEL, CHECK, Q>(a, dc, right(dc), hc, right(hc), z2, z2, wx, z2, ux);
-            wzn = rb_face2<MODEL, CHECK, Q>(a, dc, dn, hc, hn, z2, z2, wz, z2, uz);
+            wxn = rb_face2<MODEL, CHECK>(a, dc, right(dc), hc, right(hc), z2, z2, wx, tx, ux);
+            wzn = rb_face2<MODEL, CHECK>(a, dc, dn, hc, hn, z2, z2, wz, tz, uz);
             st2(a.wout[0], idx, wxn, x0, x1);
             st2(a.wout[2], idx, wzn, u0, u1);
         }
-        const float2 d0 = dc, h0 = hc, cb0 = cb;
+        const float2 d0 = dc, h0 = hc, rb0 = rb;
         dc = dn;
         hc = hn;
         if (k + 1 < k1) load(idx + sz);
@@ -867,7 +846,7 @@ __device__ __forceinline__ void rb3d_pair_body(const RbArgs& a, int bx, int by, 
             const float2 wyb = sw[p][r - 1][lane], wxl = left(wxn);
             const float2 e = f2(-rb_cell_e<MODEL>(a, h0.x + d0.x, 0.0f), -rb_cell_e<MODEL>(a, h0.y + d0.y, 0.0f));
             const float2 div = fma2(sub2(wzn, wzb), s2, fma2(sub2(wyn, wyb), s1, mul2(sub2(wxn, wxl), s0)));
-            const float2 dnew = fma2(e, fma2(d0, rdt, sub2(div, cb0)), d0);
+            const float2 dnew = fma2(e, fma2(d0, rdt, add2(rb0, div)), d0);
             st2(a.dout, idx, dnew, u0, u1);
             if (CHECK) {
                 const float2 uyb = su[p][r - 1][lane], uxl = left(ux);
@@ -908,7 +887,6 @@ template <int MODEL, bool CHECK, int R>
 __device__ __forceinline__ void rb3d_tb2_body(const RbArgs& a, int bx, int by, int bz, int chunk, double& part,
                                               unsigned long long& pmax)
 {
-    constexpr bool Q = true;   // carries q, not omega
     static_assert(MODEL == LIN || MODEL == NONLIN, "the 3D two-iteration kernel serves LIN and NONLIN");
     __shared__ float sdi[2][R][32];   // level-1 input delta of a plane (row above)
     __shared__ float shi[2][R][32];   // H_b (FP32) of a plane (row above)
@@ -946,8 +924,9 @@ __device__ __forceinline__ void rb3d_tb2_body(const RbArgs& a, int bx, int by, i
     float p0 = a.din[o0];                 // delta' of plane ks: exact at the boundary plane, else unused
     float h0 = a.Hf[o0];
     float d1 = a.din[o0 + sz], h1 = a.Hf[o0 + sz];
-    float wz1b = rb_face<MODEL, false, Q>(a, p0, d1, h0, h1, 0.0f, 0.0f, a.win[2][o0], 0.0f, u);   // level 1, ks+1/2
-    float wx1p = 0.0f, wy1p = 0.0f, rb0 = 0.0f, hu0 = h0;
+    float tbz0 = a.tb[2][o0];
+    float wz1b = rb_face<MODEL, false>(a, p0, d1, h0, h1, 0.0f, 0.0f, a.win[2][o0], tbz0, u);   // level 1, ks+1/2
+    float wx1p = 0.0f, wy1p = 0.0f, tbx0 = 0.0f, tby0 = 0.0f, rb0 = 0.0f, hu0 = h0;
     float wz2b = 0.0f, uz2b = 0.0f;
     sdi[(ks + 1) & 1][r][lane] = d1;
     shi[(ks + 1) & 1][r][lane] = h1;
@@ -964,14 +943,14 @@ __device__ __forceinline__ void rb3d_tb2_body(const RbArgs& a, int bx, int by, i
             h2 = a.Hf[on + sz];
         }
         const float wx = a.win[0][on], wy = a.win[1][on], wz = a.win[2][on];
-        const float rb1 = -a.Cb[on];
+        const float tbx1 = a.tb[0][on], tby1 = a.tb[1][on], tbz1 = a.tb[2][on], rb1 = a.Rb[on];
         const float du = up ? sdi[kn & 1][r + 1][lane] : d1;
         const float hu = up ? shi[kn & 1][r + 1][lane] : h1;
         const float d1r = __shfl_down_sync(FULL, d1, 1);
         const float h1r = __shfl_down_sync(FULL, h1, 1);
-        const float wx1 = rb_face<MODEL, false, Q>(a, d1, d1r, h1, h1r, 0.0f, 0.0f, wx, 0.0f, u);
-        const float wy1 = rb_face<MODEL, false, Q>(a, d1, du, h1, hu, 0.0f, 0.0f, wy, 0.0f, u);
-        const float wz1 = rb_face<MODEL, false, Q>(a, d1, d2, h1, h2, 0.0f, 0.0f, wz, 0.0f, u);   // kn+1/2
+        const float wx1 = rb_face<MODEL, false>(a, d1, d1r, h1, h1r, 0.0f, 0.0f, wx, tbx1, u);
+        const float wy1 = rb_face<MODEL, false>(a, d1, du, h1, hu, 0.0f, 0.0f, wy, tby1, u);
+        const float wz1 = rb_face<MODEL, false>(a, d1, d2, h1, h2, 0.0f, 0.0f, wz, tbz1, u);   // kn+1/2
         sy1[r][lane] = wy1;
         sdi[(kn + 1) & 1][r][lane] = d2;
         shi[(kn + 1) & 1][r][lane] = h2;
@@ -990,9 +969,9 @@ __device__ __forceinline__ void rb3d_tb2_body(const RbArgs& a, int bx, int by, i
         const float h0r = __shfl_down_sync(FULL, h0, 1);
         const float p0u = up ? sd1[k & 1][r + 1][lane] : p0;
         float ux2 = 0.0f, uy2 = 0.0f, uz2 = 0.0f;
-        const float wx2 = rb_face<MODEL, CHECK, Q>(a, p0, p0r, h0, h0r, 0.0f, 0.0f, wx1p, 0.0f, ux2);
-        const float wy2 = rb_face<MODEL, CHECK, Q>(a, p0, p0u, h0, hu0, 0.0f, 0.0f, wy1p, 0.0f, uy2);
-        const float wz2 = rb_face<MODEL, CHECK, Q>(a, p0, p1, h0, h1, 0.0f, 0.0f, wz1b, 0.0f, uz2);   // k+1/2
+        const float wx2 = rb_face<MODEL, CHECK>(a, p0, p0r, h0, h0r, 0.0f, 0.0f, wx1p, tbx0, ux2);
+        const float wy2 = rb_face<MODEL, CHECK>(a, p0, p0u, h0, hu0, 0.0f, 0.0f, wy1p, tby0, uy2);
+        const float wz2 = rb_face<MODEL, CHECK>(a, p0, p1, h0, h1, 0.0f, 0.0f, wz1b, tbz0, uz2);   // k+1/2
         sy2[r][lane] = wy2;
         if (CHECK) su2[r][lane] = uy2;
         __syncthreads();
@@ -1027,6 +1006,9 @@ __device__ __forceinline__ void rb3d_tb2_body(const RbArgs& a, int bx, int by, i
         wz1b = wz1;
         wx1p = wx1;
         wy1p = wy1;
+        tbx0 = tbx1;
+        tby0 = tby1;
+        tbz0 = tbz1;
         rb0 = rb1;
         wz2b = wz2;
         uz2b = uz2;
@@ -1036,16 +1018,13 @@ __device__ __forceinline__ void rb3d_tb2_body(const RbArgs& a, int bx, int by, i
 // ---------------------------------------------------------------------------
 // Rebase, FP64.  Fold the changes of buffer parity `parity` into the base:
 // H_b += delta, w_b += omega (positions that are never updated hold zeros),
-// and clear both buffers, so that the next iteration may start on either.  In
-// the q form omega = q - t_b (a phase starts with q = t_b in both buffers), and
-// the base kernel fills the buffers of q.
+// and clear both buffers, so that the next iteration may start on either.
 struct RbFoldArgs {
     long long n;
     double* H;
     double* wb[3];
     float* d[2];
     float* w[3][2];
-    const float* tb[3];   // the q form; NULL otherwise
     int ndim;
 };
 
@@ -1057,8 +1036,8 @@ __device__ __forceinline__ void rb_fold_pair(const RbFoldArgs& f, int parity, lo
         f.H[t] += (double)dp[t];
         f.d[0][t] = f.d[1][t] = 0.0f;
         for (int d = 0; d < f.ndim; ++d) {
-            f.wb[d][t] += (double)f.w[d][parity][t] - (f.tb[d] ? (double)f.tb[d][t] : 0.0);
-            if (!f.tb[d]) f.w[d][0][t] = f.w[d][1][t] = 0.0f;
+            f.wb[d][t] += (double)f.w[d][parity][t];
+            f.w[d][0][t] = f.w[d][1][t] = 0.0f;
         }
         return;
     }
@@ -1076,25 +1055,19 @@ __device__ __forceinline__ void rb_fold_pair(const RbFoldArgs& f, int parity, lo
         if (d < f.ndim) {
             const float2 w = *at2(parity ? f.w[d][1] : f.w[d][0]);
             double2 b = *at2d(f.wb[d]);
-            if (f.tb[d]) {
-                const float2 tb = *at2(f.tb[d]);
-                b.x += (double)w.x - (double)tb.x;
-                b.y += (double)w.y - (double)tb.y;
-            } else {
-                b.x += (double)w.x;
-                b.y += (double)w.y;
-                *at2(f.w[d][0]) = zero;
-                *at2(f.w[d][1]) = zero;
-            }
+            b.x += (double)w.x;
+            b.y += (double)w.y;
             *at2d(f.wb[d]) = b;
+            *at2(f.w[d][0]) = zero;
+            *at2(f.w[d][1]) = zero;
         }
     }
 }
 
 // Base quantities, FP64 (one thread per cell): t_b = w_b + u(H_b) for the
 // face to +d of every cell, and for inner cells R_b = (H_b - Hold)/dt +
-// div w_b (not in the q form), C_b = div u(H_b) - (H_b - Hold)/dt (its norm
-// into acc64), plus H_b as FP32; in the q form t_b also into both buffers of q.
+// div w_b, C_b = div u(H_b) - (H_b - Hold)/dt (its norm into acc64), plus
+// H_b as FP32.
 struct RbBaseArgs {
     int nx, ny, nz, ndim, model;
     long long sy, sz;
@@ -1105,9 +1078,8 @@ struct RbBaseArgs {
     const double* wb[3];
     const double* D;
     float* tb[3];
-    float* q[3][2];      // the q form; NULL otherwise
-    float* Rb;           // NULL in the q form
-    float* Cb;           // 1D, 2D and the q form: C_b rounded to FP32
+    float* Rb;
+    float* Cb;           // 1D, 2D: C_b rounded to FP32
     double* Cb64;        // 3D: C_b
     float* Hf;
     double* acc64;
@@ -1115,26 +1087,8 @@ struct RbBaseArgs {
     int norm_max;
 };
 
-// The undamped flux of a face.  In the q form with integer arithmetic
-// (ptd_intflux.cuh): a rebase is bound by the FP64 pipe (84 % busy).  (Not in
-// the omega form of D = H^3 in 1D and 2D, where a last-bit change of t_b can
-// move a step's iteration count.)
-template <bool Q>
 __device__ __forceinline__ double rb_u64(const RbBaseArgs& b, long long cL, long long cR)
 {
-    if (Q) {
-        auto bits = [](double x) { return (uint64_t)__double_as_longlong(x); };
-        const uint64_t hl = bits(b.H[cL]), hr = bits(b.H[cR]);
-        uint64_t r;
-        bool ok;
-        if (b.model == LIN) ok = if_flux_lin(hl, hr, r);
-        else if (b.model == LINSTEP) ok = if_flux_step(hl, hr, bits(b.D[cL]), bits(b.D[cR]), r);
-        else ok = if_flux_cube(hl, hr, r);
-        if (ok) {
-            const double u = __longlong_as_double((long long)r);
-            return b.model == NONLIN_EXPM ? (b.D[cL] + b.D[cR]) * u : u;
-        }
-    }
     const double g = b.H[cR] - b.H[cL];
     if (b.model == LIN) return g;
     if (b.model == LINSTEP) return (b.D[cL] + b.D[cR]) * g;
@@ -1143,29 +1097,8 @@ __device__ __forceinline__ double rb_u64(const RbBaseArgs& b, long long cL, long
     return s * s * s * g;
 }
 
-// A double rounded to the nearest float, in the q form with integer operations
-// (the hardware conversion issues on the FP64 pipe).
-template <bool Q>
-__device__ __forceinline__ float rb_f32(double x)
-{
-    return Q ? d2f_rn_bits(x) : __double2float_rn(x);
-}
-
-// t_b of the face to +d of cell c, whose undamped flux is u
-template <bool Q>
-__device__ __forceinline__ void rb_base_face(const RbBaseArgs& b, int d, long long c, double u)
-{
-    const float t = rb_f32<Q>(b.wb[d][c] + u);
-    b.tb[d][c] = t;
-    if (Q) {
-        b.q[d][0][c] = t;
-        b.q[d][1][c] = t;
-    }
-}
-
 // The base quantities of the cell (ix, iy, iz); its check residual goes into
 // (part, pmax).
-template <bool Q>
 __device__ __forceinline__ void rb_base_cell(const RbBaseArgs& b, int ix, int iy, int iz, double& part,
                                              unsigned long long& pmax)
 {
@@ -1173,7 +1106,7 @@ __device__ __forceinline__ void rb_base_cell(const RbBaseArgs& b, int ix, int iy
     const int co[3] = {ix, iy, iz};
     const int nn[3] = {b.nx, b.ny, b.nz};
     const long long c = iz * b.sz + iy * b.sy + ix;
-    b.Hf[c] = rb_f32<Q>(b.H[c]);
+    b.Hf[c] = __double2float_rn(b.H[c]);
     bool inner = true;
 #pragma unroll
     for (int d = 0; d < 3; ++d) inner = inner && (d >= b.ndim || (co[d] >= 1 && co[d] <= nn[d] - 2));
@@ -1183,20 +1116,20 @@ __device__ __forceinline__ void rb_base_cell(const RbBaseArgs& b, int ix, int iy
         if (d >= b.ndim) continue;
         double ur = 0.0;
         if (co[d] <= nn[d] - 2) {
-            ur = rb_u64<Q>(b, c, c + stp[d]);
-            rb_base_face<Q>(b, d, c, ur);
+            ur = rb_u64(b, c, c + stp[d]);
+            b.tb[d][c] = (float)(b.wb[d][c] + ur);
         }
         if (inner) {
-            const double ul = rb_u64<Q>(b, c - stp[d], c);
-            if (!Q) divw = fma(b.wb[d][c] - b.wb[d][c - stp[d]], b.sig[d], divw);
+            const double ul = rb_u64(b, c - stp[d], c);
+            divw = fma(b.wb[d][c] - b.wb[d][c - stp[d]], b.sig[d], divw);
             divu = fma(ur - ul, b.sig[d], divu);
         }
     }
     if (inner) {
         const double dh = (b.H[c] - b.Hold[c]) * b.rdt;
-        if (!Q) b.Rb[c] = rb_f32<Q>(dh + divw);
+        b.Rb[c] = (float)(dh + divw);
         const double cb = divu - dh;
-        b.Cb[c] = rb_f32<Q>(cb);
+        b.Cb[c] = (float)cb;
         accumulate_residual(cb, part, pmax);
     }
 }

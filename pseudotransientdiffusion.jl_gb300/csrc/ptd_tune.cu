@@ -69,10 +69,9 @@ long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 
 }  // namespace
 
-// z march of the 16-row FP32 kernels (defect correction, rebased form on large
-// grids): us per iteration at march 16 and at the march taken: rebased NONLIN
-// 64^3 19.4, 8.6 (4); 128^3 33.5, 30.4 (4); 192^3 83.7, 82.2 (8); 320x255x191
-// 153 (16).
+// z march of the 16-row FP32 kernels (defect correction, rebased LIN on large
+// grids): us per iteration at march 16 and at the march taken: rebased LINSTEP
+// 64^3 17.6, 8.1 (4); 96^3 21.3, 17.2 (4); 128^3 35.7, 33.8 (4); 192^3 95.7 (16).
 int z_march16(const ptd_params& p)
 {
     const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, 15);
@@ -80,17 +79,18 @@ int z_march16(const ptd_params& p)
     return march_length(16, 4, 17 * sm / 2, sm, [&](int m) { return bxy * ceil_div(p.nz - 2, m); });
 }
 
-// Whether the 3D rebased form runs two cells per lane (rb3d_pair_body): always
-// for LIN; for NONLIN, whose one-cell kernel hides its longer chains behind
-// twice the warps, while the fields (40 bytes a cell) fit the L2 cache.
+// Whether the 3D rebased form runs two cells per lane (rb3d_pair_body): LIN and
+// NONLIN grids that are bound by the latency of a plane (the figures are at
+// rb3d_pair_body: 110^3 is the largest cube where it is faster, at 128^3 the
+// one-cell kernel is).
 bool rb3d_pair(int model, long long nx, long long ny, long long nz)
 {
-    return model == LIN || (model == NONLIN && nx * ny * nz <= 2400000);
+    return (model == LIN || model == NONLIN) && nx * ny * nz <= 1500000;
 }
 
-// Its march: us per iteration at marches 2, 4, 8, 16: NONLIN 64^3 6.9, 8.3,
-// 12.0, 19.5; 96^3 15.4, 15.9, 16.5, 22.0; LIN 192^3 85, 74.5, 72.0, 72.3;
-// 512^3 1239, 1107, 1046, 1012.
+// Its march: us per iteration at marches 1, 2, 4, 8, 16: NONLIN 96^3 20.8, 18.5,
+// 19.0, 19.2, 25.7; 110^3 30.1, 24.8, 23.6, 21.9, 29.9; LIN 96^3 15.3, 12.8, 12.6,
+// 13.0, 18.0.
 int z_march_pair(const ptd_params& p)
 {
     const long long bxy = ceil_div(p.nx - 2, 62) * ceil_div(p.ny - 2, 7);
@@ -98,9 +98,16 @@ int z_march_pair(const ptd_params& p)
     return march_length(16, 4, 4 * sm, 7 * sm / 4, [&](int m) { return bxy * ceil_div(p.nz - 2, m); });
 }
 
-// Rows of a CTA of the 3D rebased form's one-cell kernel: 8 while the fields
-// fit the L2 cache (half the warps per barrier), 16 above (less halo).
-int rb3d_rows(long long nx, long long ny, long long nz) { return nx * ny * nz <= 2400000 ? 8 : 16; }
+// Rows of a CTA of the 3D rebased form's one-cell kernel: 8 (half the warps per
+// barrier), for LIN grids past the L2 cache 16 (less halo).  us per iteration,
+// 8 / 16 rows at the best march: NONLIN 128^3 36.2, 37.9; 256x200x180 122, 126;
+// 320x255x191 187, 188; LINSTEP 48^3 6.0, 6.6; 128^3 30.3, 33.8; 320x255x191 176,
+// 182; 400^3 681, 702; LIN 128^3 24.5, 26.7; 192^3 80.5, 80.3; 320x255x191 155.6,
+// 152.2.
+int rb3d_rows(int model, long long nx, long long ny, long long nz)
+{
+    return model == LIN && nx * ny * nz > 2400000 ? 16 : 8;
+}
 
 // z march of the 8-row FP32 kernels and of the adjoint, at least per_sm CTAs
 // per SM down to a march of one plane.  A gradient of 72^3 at marches 1, 2, 3,
@@ -114,9 +121,10 @@ int z_march8(const ptd_params& p, int per_sm)
 }
 
 // March of the rebased form's base kernel (rows in 2D, planes in 3D, per warp
-// of 32 cells): us of a rebase at march 32 and at the march taken: 2D NONLIN
-// 256^2 124, 28 (1); 600x500 134, 53 (4); 2048^2 506, 457 (8); 3D NONLIN
-// 50x40x45 131, 33 (2); 100x90x80 175, 106 (8); 320x255x191 1290, 1239 (16).
+// of 32 cells): us of two rebases, one launch and the step's overhead (about
+// 100) at march 32 and at the march taken: 2D NONLIN 256^2 308, 128 (1); 600x500
+// 314, 165 (4); 2048^2 925, 830 (8); 4096^2 2907, 2832 (16); 3D NONLIN 50x40x45
+// 357, 137 (1); 100x90x80 433, 395 (8); 320x255x191 3865, 3841 (16).
 int rb_base_march(const ptd_params& p)
 {
     const long long sm = sm_count(), line = ceil_div(p.nx, 32) * (p.ndim == 3 ? p.ny : 1), n = p.ndim == 3 ? p.nz : p.ny;
@@ -172,7 +180,7 @@ LaunchCfg tuned_config(const ptd_params& p)
     } else if (p.ndim == 3 && (p.precision == PTD_PREC_FP32_RB || p.precision == PTD_PREC_FP32_DC)) {
         c.rows3d = 16;
         const bool pair = p.precision == PTD_PREC_FP32_RB && rb3d_pair(p.model, p.nx, p.ny, p.nz);
-        const bool rb8 = p.precision == PTD_PREC_FP32_RB && rb3d_rows(p.nx, p.ny, p.nz) == 8;
+        const bool rb8 = p.precision == PTD_PREC_FP32_RB && rb3d_rows(p.model, p.nx, p.ny, p.nz) == 8;
         c.chunk3d = pair ? z_march_pair(p) : rb8 ? z_march8(p, 2) : z_march16(p);
     } else if (p.ndim == 3) {
         // The FP64-accuracy forms: 256-thread CTAs of 31 x 7 updated cells.

@@ -36,6 +36,15 @@ namespace {
 constexpr int kMaxWarps = 8;     // warps per CTA (13824 cells in all; at 16384 one launch per iteration is as fast)
 constexpr int kMaxCluster = 16;  // CTAs (above 8 the size is not portable: granted by kernel attribute)
 
+// Dynamic shared memory of a CTA.  The largest, 8 warps x 126 cells, is under
+// the 48 KB that a kernel has without an attribute, and no plan sets that
+// attribute: it belongs to the kernel, which all contexts share.
+constexpr size_t line_smem(int warps, int core)
+{
+    return (size_t)(4 * warps * core + 2 * kMaxWarps + kHostErr) * sizeof(double);
+}
+static_assert(line_smem(kMaxWarps, 32 * 4 - 2) <= 48 * 1024, "a line CTA needs no shared-memory attribute");
+
 // One cell window of a warp: C consecutive cells per lane.
 template <int MODEL, int C>
 __global__ void __launch_bounds__(32 * kMaxWarps) pt_line_kernel(PTArgs a, LineArgs l)
@@ -244,7 +253,7 @@ cudaLaunchConfig_t launch_of(const LinePlan& p, cudaStream_t s, cudaLaunchAttrib
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.ctas);
     cfg.blockDim = dim3(32, p.warps);
-    cfg.dynamicSmemBytes = (size_t)(4 * p.warps * p.core + 2 * kMaxWarps + kHostErr) * sizeof(double);
+    cfg.dynamicSmemBytes = line_smem(p.warps, p.core);
     cfg.stream = s;
     at->id = cudaLaunchAttributeClusterDimension;
     at->val.clusterDim.x = p.ctas;
@@ -287,8 +296,8 @@ bool line_plan(int model, int nx, int nchk, LinePlan& p)
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = launch_of(p, nullptr, &at);
     int n = 0;
-    bool ok = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) == cudaSuccess;
-    if (ok && p.ctas > 8) ok = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    bool ok = true;
+    if (p.ctas > 8) ok = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     ok = ok && cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess && n >= 1;
     if (!ok) cudaGetLastError();
     return ok;

@@ -584,7 +584,7 @@ extern "C" int ptd_create(ptd_ctx** out, const ptd_params* p)
     c->line = p->ndim == 1 && p->precision == PTD_PREC_FP64 && p->resid_mode == PTD_RESID_MIXED &&
               line_plan(p->model, p->nx, p->nchk, c->lplan);
     if (p->ndim > 1 && p->precision == PTD_PREC_FP64 && p->resid_mode == PTD_RESID_MIXED &&
-        !(p->flags & PTD_FLAG_AUTOTUNE))
+        p->nchk <= kFlowCheck && !(p->flags & PTD_FLAG_AUTOTUNE))
         flow_plan(p->model, p->ndim, p->nx, p->ny, p->nz, c->flow);
     if (!rc && c->flow.rows) rc = alloc(&c->flow_mem, flow_bytes(c->flow));
     if ((c->line || c->flow.rows) && c->errcap < 1 << 30) c->errcap += kHostErr;   // room for several steps

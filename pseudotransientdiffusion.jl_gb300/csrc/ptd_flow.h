@@ -42,6 +42,11 @@ struct FlowArgs {
     double tol, norm_den;
 };
 
+// Iterations of a check block at most: the judge's wait spans one (4 s of the
+// largest grids, of the 20 that it may take).  A context with a longer cadence
+// runs one iteration per launch.
+constexpr int kFlowCheck = 1 << 18;
+
 // Done states besides DONE_*: a wait that gave up; a step that converged, and
 // the next one begins in the same launch.
 enum { FLOW_TIMEOUT = 4, FLOW_NEXT = 5 };

@@ -51,7 +51,8 @@ typedef enum ptd_status {
     PTD_ECUDA = 4,     /* a CUDA runtime call failed */
     PTD_ENOMEM = 5,    /* device or host allocation failed */
     PTD_ESTATE = 6,    /* call out of order (e.g. stepping before a state was set) */
-    PTD_ETIMEOUT = 7   /* a device-side wait gave up (never expected) */
+    PTD_ETIMEOUT = 7   /* a device-side wait gave up (never expected): the state is lost, and calls that need
+                          one return this status until a new one is set */
 } ptd_status;
 
 /* Diffusion models of the reference's solver scripts:
@@ -193,6 +194,10 @@ PTD_API int ptd_set_launch_config(ptd_ctx* ctx, const int32_t cfg[4]);
 /* The context's CUDA stream (cudaStream_t) and a device synchronize of it. */
 PTD_API void* ptd_stream(ptd_ctx* ctx);
 PTD_API int ptd_sync(ptd_ctx* ctx);
+
+/* Polls after which a device-side wait of the one-launch steps gives up
+ * (PTD_ETIMEOUT); 0: the default, about 20 s, which is also the most. */
+PTD_API int ptd_set_wait_limit(ptd_ctx* ctx, int32_t polls);
 
 /* Counters since ptd_create: kernels launched by the library (each kernel of
  * a replayed CUDA graph counts; several steps in one launch count as one) and

@@ -284,6 +284,7 @@ struct ptd_ctx : ptd_ctx_base {
     FlowPlan flow;                // 2D, 3D FP64: steps are one launch of the flow kernel (rows > 0)
     void* flow_mem = nullptr;     // its exchange buffers
     unsigned flow_tag = 1;        // tags used so far
+    int flow_wait = kFlowWait;    // polls of a wait
     cudaGraphExec_t gstep[2] = {nullptr, nullptr};   // one physical step's check loop, per start parity
     cudaGraphExec_t gplain[2] = {nullptr, nullptr};
     int blocks_per_pass = 1;      // check blocks in the body of the step graph's loop
@@ -648,6 +649,15 @@ extern "C" int ptd_launch_config(ptd_ctx* c, int32_t cfg[4])
     return PTD_OK;
 }
 
+// Whether a wait of a flow launch gave up (for certain after a wait for the
+// stream).  The state is lost then, until a new one is set.
+static int flow_state(const ptd_ctx* c)
+{
+    if (c->flow.rows && c->h_st->pad)
+        return fail(PTD_ETIMEOUT, "a wait of the one-launch step gave up: the state is lost, set a new one");
+    return PTD_OK;
+}
+
 extern "C" int ptd_set_launch_config(ptd_ctx* c, const int32_t cfg[4])
 {
     if (!c || !cfg) return fail(PTD_EINVAL, "ptd_set_launch_config: NULL argument");
@@ -662,9 +672,10 @@ extern "C" int ptd_set_launch_config(ptd_ctx* c, const int32_t cfg[4])
     k.rows3d = cfg[2];
     k.chunk3d = cfg[3];
     CK(cudaStreamSynchronize(c->stream));
+    int rc = flow_state(c);
+    if (rc) return rc;
     c->cfg = k;
     c->flow = FlowPlan();   // the shape is one of the kernel of one iteration per launch
-    int rc = PTD_OK;
     if (c->dc) {
         rc = dc_set_config(c->dc, k);
     } else if (c->rb) {
@@ -683,10 +694,11 @@ extern "C" int ptd_set_launch_config(ptd_ctx* c, const int32_t cfg[4])
     return rc;
 }
 
-// After a wait for the stream: whether a wait of a flow launch gave up.
-static int flow_state(const ptd_ctx* c)
+extern "C" int ptd_set_wait_limit(ptd_ctx* c, int32_t polls)
 {
-    if (c->flow.rows && c->h_st->pad) return fail(PTD_ETIMEOUT, "a wait of the one-launch step gave up");
+    if (!c) return fail(PTD_EINVAL, "ctx is NULL");
+    if (polls < 0) return fail(PTD_EINVAL, "polls must be >= 0");
+    c->flow_wait = polls ? std::min((int)polls, kFlowWait) : kFlowWait;
     return PTD_OK;
 }
 
@@ -743,6 +755,14 @@ extern "C" int ptd_set_state2(ptd_ctx* c, const double* H, const double* Hold, c
     if (c->p.model == PTD_MODEL_LINSTEP && !D) return fail(PTD_EINVAL, "the step model needs D");
     if (c->p.model == PTD_MODEL_NONLIN_EXPM && !D) return fail(PTD_EINVAL, "the exp(m) H^3 model needs m (in D)");
     const size_t bytes = (size_t)c->nfield * sizeof(double);
+    if (c->flow.rows) {
+        CK(cudaStreamSynchronize(c->stream));
+        if (c->h_st->pad) {   // a launch that gave up: its tags are part used, its status is told
+            CK(cudaMemsetAsync(c->flow_mem, 0, flow_bytes(c->flow), c->stream));
+            c->flow_tag = 1;
+            c->h_st->pad = 0;
+        }
+    }
     // padding stays zero: clear whole buffers first
     double* Hdst = c->df64 ? c->stage : c->H[0];
     if (c->sy != c->nx) CK(cudaMemsetAsync(Hdst, 0, bytes, c->stream));
@@ -854,6 +874,8 @@ static int run_line(ptd_ctx* c, int nsteps, int niter)
 // iterations without.
 static int run_flow(ptd_ctx* c, int nsteps, int niter)
 {
+    const int lost = flow_state(c);
+    if (lost) return lost;
     if (c->flow_tag > 1u << 30) {   // long before tags come round
         CK(cudaMemsetAsync(c->flow_mem, 0, flow_bytes(c->flow), c->stream));
         c->flow_tag = 1;
@@ -873,6 +895,7 @@ static int run_flow(ptd_ctx* c, int nsteps, int niter)
     f.niter = niter;
     f.nsteps = c->p.nchk <= 4096 ? nsteps : std::min(nsteps, 1);   // (tags of a launch: see flow_tags)
     f.itlimit = 1 << 17;
+    f.wait = c->flow_wait;
     f.tol = c->p.tol;
     f.norm_den = c->dv.norm_den;
     CK(launch_flow(a, f, c->p.model, c->flow, c->stream));

@@ -50,7 +50,6 @@
 namespace ptd {
 
 constexpr int kWarps = kFlowWarps;
-constexpr int kFlowWait = 1 << 25;   // polls of one wait before it gives up (about 20 s: another kernel may hold an SM)
 
 __device__ __forceinline__ uint4 flow_load(const uint4* p)
 {
@@ -87,7 +86,7 @@ __device__ __forceinline__ void flow_judge(const PTArgs& a, const FlowArgs& f)
         unsigned long long mx = 0ull;
         for (int i = t; t < nt && i < f.nwarps; i += nt) {
             uint4 v = flow_load(parts + i);
-            for (int left = kFlowWait; !flow_ready(v, tag) && left > 0; --left) v = flow_load(parts + i);
+            for (int left = f.wait; !flow_ready(v, tag) && left > 0; --left) v = flow_load(parts + i);
             if (!flow_ready(v, tag)) {
                 s_lost = 1;
                 break;
@@ -355,7 +354,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) pt2d_flow_kernel(PTArgs a, Flo
             if (k >= 0 && --left_in_block == 0) {
                 left_in_block = f.nchk;
                 // the snapshot of two checks ago is given up: its decision must be known
-                for (int wait = kFlowWait; nd < nchecks - 1 && done == DONE_RUNNING; --wait) {
+                for (int wait = f.wait; nd < nchecks - 1 && done == DONE_RUNNING; --wait) {
                     decided(lane == 0 ? *ctl : 0ull, nd, done);
                     if (wait == 0) done = FLOW_TIMEOUT;
                 }
@@ -372,7 +371,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) pt2d_flow_kernel(PTArgs a, Flo
             if (!f.checks && k == f.niter - 1) break;
             // the neighbours' edges of the same iteration
             bool ok = stop;
-            for (int wait = kFlowWait; !ok; --wait) {
+            for (int wait = f.wait; !ok; --wait) {
                 uint4 vb = make_uint4(0, tag, 0, tag), vt = vb, vx[R];
                 if (gety_b) vb = flow_load(hy(par, w - f.ntx, 1));
                 if (gety_t) vt = flow_load(hy(par, w + f.ntx, 0));

@@ -39,12 +39,13 @@ struct FlowArgs {
     int ntx, nty, nwarps;      // warp tiles in x, in y and in all
     int nchk, itmax, checks, niter;   // checks 0: niter iterations without checks
     int nsteps, itlimit;       // steps at most, and none begun after that many iterations
+    int wait;                  // polls of one wait before it gives up
     double tol, norm_den;
 };
 
+constexpr int kFlowWait = 1 << 25;   // about 20 s: another kernel may hold an SM
 // Iterations of a check block at most: the judge's wait spans one (4 s of the
-// largest grids, of the 20 that it may take).  A context with a longer cadence
-// runs one iteration per launch.
+// largest grids).  A context with a longer cadence runs one iteration per launch.
 constexpr int kFlowCheck = 1 << 18;
 
 // Done states besides DONE_*: a wait that gave up; a step that converged, and

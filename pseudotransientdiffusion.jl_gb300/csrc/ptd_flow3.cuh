@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(32 * W, 1) pt3d_flow_kernel(PTArgs a, FlowArgs
             if (k >= 0 && --left_in_block == 0) {
                 left_in_block = f.nchk;
                 // the snapshot of two checks ago is given up: its decision must be known
-                for (int wait = kFlowWait; nd < nchecks - 1 && done == DONE_RUNNING; --wait) {
+                for (int wait = f.wait; nd < nchecks - 1 && done == DONE_RUNNING; --wait) {
                     decided(lane == 0 ? *ctl : 0ull, nd, done);
                     if (wait == 0) done = FLOW_TIMEOUT;
                 }
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(32 * W, 1) pt3d_flow_kernel(PTArgs a, FlowArgs
             if (!f.checks && k == f.niter - 1) break;
             // the neighbours' edges of the same iteration
             bool ok = stop;
-            for (int wait = kFlowWait; !ok; --wait) {
+            for (int wait = f.wait; !ok; --wait) {
                 // (all loads first: what follows one waits for it)
                 uint4 vf[RZ], vk[RZ], vb[RY], vt[RY], vx[RZ][RY];
 #pragma unroll

@@ -103,6 +103,7 @@ def lib():
         "ptd_get_state": (C.c_int, [vp, vp]),
         "ptd_stream": (C.c_void_p, [vp]),
         "ptd_sync": (C.c_int, [vp]),
+        "ptd_set_wait_limit": (C.c_int, [vp, C.c_int32]),
         "ptd_counters": (C.c_int, [vp, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
         "ptd_launch_config": (C.c_int, [vp, C.POINTER(C.c_int32)]),
         "ptd_set_launch_config": (C.c_int, [vp, C.POINTER(C.c_int32)]),

@@ -158,6 +158,10 @@ class Solver:
         _abi.check(_abi.lib().ptd_get_state(self._h, _ptr(out)), "ptd_get_state")
         return out
 
+    def set_wait_limit(self, polls: int):
+        """Polls after which a device-side wait of the one-launch steps gives up (0: the default)."""
+        _abi.check(_abi.lib().ptd_set_wait_limit(self._h, polls), "ptd_set_wait_limit")
+
     def sync(self):
         _abi.check(_abi.lib().ptd_sync(self._h), "ptd_sync")
 

@@ -8,7 +8,7 @@
 // edges of H with its four neighbours: each iteration it publishes its edge
 // cells and waits for theirs.  An edge value travels with its tag (the
 // iteration it belongs to) in the same 8 bytes, {32 bits of the double, tag}
-// twice in one 16-byte store, so a reader that sees the tag has the value: no
+// twice in one 16-byte store, so a reader that sees both tags has the value: no
 // fence, no flag, no barrier, and a warp waits for its neighbours only.  The
 // faces on a tile's left and lower edge are evolved by both tiles that touch
 // them, from the same values.  Slots alternate by iteration parity; a warp
@@ -51,17 +51,21 @@ namespace ptd {
 
 constexpr int kWarps = kFlowWarps;
 
+// A slot is two 64-bit words, each {32 bits of the value, tag} (the layout of
+// NCCL's low-latency protocol), moved by one vector instruction.  A vector
+// access is one scalar access per element in the memory model, so a word
+// arrives whole; as four 32-bit elements a value could part from its tag.
 __device__ __forceinline__ uint4 flow_load(const uint4* p)
 {
     uint4 v;
-    asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("{ .reg .b64 a, b; ld.volatile.global.v2.b64 {a,b}, [%4]; mov.b64 {%0,%1}, a; mov.b64 {%2,%3}, b; }"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ void flow_store(uint4* p, double x, unsigned tag)
 {
-    asm volatile("st.volatile.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"((unsigned)__double2loint(x)), "r"(tag),
-                 "r"((unsigned)__double2hiint(x)), "r"(tag) : "memory");
+    asm volatile("{ .reg .b64 a, b; mov.b64 a, {%1,%3}; mov.b64 b, {%2,%3}; st.volatile.global.v2.b64 [%0], {a,b}; }" ::"l"(p),
+                 "r"((unsigned)__double2loint(x)), "r"((unsigned)__double2hiint(x)), "r"(tag) : "memory");
 }
 __device__ __forceinline__ double flow_value(const uint4& v) { return __hiloint2double((int)v.z, (int)v.x); }
 __device__ __forceinline__ bool flow_ready(const uint4& v, unsigned tag) { return v.y == tag && v.w == tag; }

@@ -302,8 +302,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) pt2d_flow_kernel(PTArgs a, Flo
                 const double dx = N::sub(wx[q], wxl), dy = N::sub(wup, wlow), Ho = sHo[q][lane];
                 float e = a.fe_lin;
                 if (MODEL == LINSTEP) e = sE[MODEL == LINSTEP ? q : 0][lane];
-                if (MODEL == NONLIN || MODEL == NONLIN_EXPM)
-                    e = cell_e<MODEL>(a, hc, MODEL == NONLIN_EXPM ? N::lo_f(Dc) : 0.0f);
+                if (MODEL == NONLIN) e = cell_e<MODEL>(a, hc, 0.0f);
                 const double Hn =
                     a.sq ? h_update_sq<N>(a, Hcur, Ho, N::add(dy, dx), e)
                          : h_update<N>(a, Hcur, Ho, N::mad(dy, cst<N>(a, 1), N::mul(dx, cst<N>(a, 0))), e);

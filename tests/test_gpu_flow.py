@@ -48,6 +48,7 @@ def test_flow_step_is_the_march_step(name, shape):
 
 
 # rows per tile 1, 2, 3, 4, 6 and the first grid that does not fit (152 SMs)
+# (of these grids: 1, 2, 3, 4, 5 rows and one that does not fit; 6 rows: test_gpu_plans.py)
 @pytest.mark.parametrize("name,shape", [("diff_2D_nonlin", (300, 280)), ("diff_2D_linstep", (500, 333)),
                                         ("diff_2D_lin", (512, 512)), ("diff_2D_nonlin", (600, 521)),
                                         ("diff_2D_linstep", (701, 643)), ("diff_2D_nonlin", (900, 800))])

@@ -906,7 +906,12 @@ static int run_flow(ptd_ctx* c, int nsteps, int niter)
 // Run n PT iterations without checks starting from buffer c->cur.
 static int run_plain(ptd_ctx* c, long long n)
 {
-    while (c->line && n > 0) {
+    // (1D: a few iterations as a launch each, below, where that is faster; us a
+    // call of 1, 2, 5 and 10, launch each / line kernel: 512 cells 4.1, 8.2, 20.5,
+    // 41 / 6.2, 6.2, 6.2, 8.2; 4096 4.1, 8.2, 20.5, 41 / 6.2, 8.2, 11.3, 16.4;
+    // 13000 4.1, 8.2, 20.5, 41 / 10.3, 12.9, 21.5, 35.2)
+    const long long few = c->p.nx > 8192 ? 5 : 1;
+    while (c->line && n > few) {
         const int k = (int)std::min<long long>(n, 1 << 20);   // a launch of seconds at most
         int rc = run_line(c, 0, k);
         if (rc) return rc;

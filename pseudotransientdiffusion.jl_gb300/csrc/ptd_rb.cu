@@ -439,6 +439,13 @@ cudaError_t rb_run_plain(const RbState* rb, int32_t niter, const int* skip, int&
     return cudaSuccess;
 }
 
+// CTAs of the fold: two elements a thread (small fields in the full grid of
+// fill_blocks() take 2 us more for its empty CTAs).
+int fold_blocks(const RbState* rb)
+{
+    return (int)std::min<long long>((rb->g.nfield + 511) / 512, fill_blocks());
+}
+
 // The check-residual slots of the check launch (the grids of
 // rb_launch_model): warps in 2D, blocks in 1D and 3D.
 long long rb_check_slots(const RbState* rb)
@@ -622,7 +629,7 @@ int rb_capture(RbState* rb)
             err = cudaStreamBeginCaptureToGraph(rb->s, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                                 cudaStreamCaptureModeThreadLocal);
         if (err != cudaSuccess) break;
-        rb_fold_kernel<<<fill_blocks(), 256, 0, rb->s>>>(fold_args(rb), par);
+        rb_fold_kernel<<<fold_blocks(rb), 256, 0, rb->s>>>(fold_args(rb), par);
         err = cudaGetLastError();
         if (err == cudaSuccess) err = launch_base(rb, base_args(rb), rb->dev);
         if (err == cudaSuccess) {
@@ -821,7 +828,7 @@ int rb_step(RbState* rb, int32_t* iters, double* err_hist, int32_t err_cap, int3
         int par = 0;
         long long nl = 0;
         RCK(rb_run_plain(rb, tail, rb->zero_flag, par, nl));
-        rb_fold_kernel<<<fill_blocks(), 256, 0, rb->s>>>(fold_args(rb), par);
+        rb_fold_kernel<<<fold_blocks(rb), 256, 0, rb->s>>>(fold_args(rb), par);
         RCK(cudaGetLastError());
         rb->k.launches += nl + 1;
         iter = rb->p.itmax;
@@ -849,7 +856,7 @@ int rb_iterate(RbState* rb, int32_t niter)
     int par = 0;
     long long nl = 0;
     RCK(rb_run_plain(rb, niter, rb->zero_flag, par, nl));
-    rb_fold_kernel<<<fill_blocks(), 256, 0, rb->s>>>(fold_args(rb), par);
+    rb_fold_kernel<<<fold_blocks(rb), 256, 0, rb->s>>>(fold_args(rb), par);
     RCK(cudaGetLastError());
     rb->k.launches += nl + 2;
     rb->k.iterations += niter;

@@ -135,6 +135,7 @@ LaunchCfg tuned_config(const ptd_params& p)
 {
     LaunchCfg c;
     const long long sm = sm_count();
+    const bool often = p.nchk < 4;
     if (p.ndim == 2) {
         // short y marches in small CTAs: many independent warps per SM hide
         // the memory latency of the march.  Measured over warps {1,2,4,8} x
@@ -165,7 +166,10 @@ LaunchCfg tuned_config(const ptd_params& p)
         case PTD_PREC_DFH:
         case PTD_PREC_DF64:
             c.warps2d = p.precision == PTD_PREC_DFH ? 1 : 2;
-            c.chunk2d = march_length(8, 4, 52 * sm, 29 * sm / 2, warps(62, 1));
+            // (with a field and checks every iteration 8 rows sooner: DF64 LINSTEP
+            // 1000x1001 27.7 (4), 26.7 (8) us, DFH 34.1, 30.8)
+            if (often && coef) c.chunk2d = march_length(8, 8, 52 * sm, 12 * sm, warps(62, 1));
+            else c.chunk2d = march_length(8, 4, 52 * sm, 29 * sm / 2, warps(62, 1));
             break;
         case PTD_PREC_FP32_RB:
             if (coef) c.chunk2d = march_length(8, 1, 30 * sm, 30 * sm, warps(tb ? 28 : 31, tb ? 2 : 1));
@@ -182,6 +186,14 @@ LaunchCfg tuned_config(const ptd_params& p)
         const bool pair = p.precision == PTD_PREC_FP32_RB && rb3d_pair(p.model, p.nx, p.ny, p.nz);
         const bool rb8 = p.precision == PTD_PREC_FP32_RB && rb3d_rows(p.model, p.nx, p.ny, p.nz) == 8;
         c.chunk3d = pair ? z_march_pair(p) : rb8 ? z_march8(p, 2) : z_march16(p);
+        // FP32_DC with checks (nearly) every iteration: a check launch costs by
+        // its CTAs.  ms of a step at the march above, at the one taken: LIN
+        // 96^3 4.08 (4), 3.76 (8); 130x100x127 6.83 (4), 5.91 (16); 160x150x140
+        // 15.4 (4), 14.8 (16); LINSTEP 130x100x127 9.5 (4), 8.4 (16)
+        if (p.precision == PTD_PREC_FP32_DC && often) {
+            const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, 15);
+            c.chunk3d = march_length(16, 16, 0, 3 * sm / 2, [&](int m) { return bxy * ceil_div(p.nz - 2, m); });
+        }
     } else if (p.ndim == 3) {
         // The FP64-accuracy forms: 256-thread CTAs of 31 x 7 updated cells.
         // Their per-plane barrier joins half the warps of 512-thread CTAs (31

@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(32 * R) adj3d_kernel(const AdjArgs* __restrict
             __syncthreads();
             if (upd) {
                 const T wyb = sW[p][r - 1][lane], nyb = sN[p][r - 1][lane];
-                const float e = nonlin_cell_e(a.f, hc, EXPM ? N::lo_f(Ec) : 1.0f);
+                const float e = nonlin_cell_e<true>(a.f, hc, EXPM ? N::lo_f(Ec) : 1.0f);
                 // sum_d sigma_d [(w_+ - w_-) + (n_+ + n_-)]
                 T div = N::mul(N::add(N::sub(wxn, wxl), N::add(nx_, nxl)), acst<N>(a, 0));
                 div = N::mad(N::add(N::sub(wyn, wyb), N::add(ny_, nyb)), acst<N>(a, 1), div);

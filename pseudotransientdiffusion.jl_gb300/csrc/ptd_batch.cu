@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256) pt2d_batch_kernel(const PTArgs* __restric
     unsigned long long pmax = 0ull;
     // the body flushes its check partials into its warp's slot (work item k,
     // warp w -> k * W + w; last step of its march)
-    pt2d_body<N, MODEL, CHECK>(a, w.y * blockDim.y + threadIdx.y, w.z, chunk, part, pmax,
+    pt2d_body<N, MODEL, CHECK, true>(a, w.y * blockDim.y + threadIdx.y, w.z, chunk, part, pmax,
                                (long long)blockIdx.x * blockDim.y + threadIdx.y);
 }
 
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(256) dc2d_batch_kernel(const DcArgs* __restric
     float part = 0.0f;
     unsigned pmax = 0u;
     // the body flushes its check partials into its warp's slot (last step of its march)
-    dc2d_body<MODEL, CHECK>(a, w.y * blockDim.y + threadIdx.y, w.z, chunk, part, pmax,
+    dc2d_body<MODEL, CHECK, true>(a, w.y * blockDim.y + threadIdx.y, w.z, chunk, part, pmax,
                             (long long)blockIdx.x * blockDim.y + threadIdx.y);
 }
 
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256) dc2d_tb2_batch_kernel(const DcArgs* __res
     float part = 0.0f;
     unsigned pmax = 0u;
     // the body flushes its check partials into its warp's slot (last step of its march)
-    dc2d_tb2_body<MODEL, CHECK>(a, w.y * blockDim.y + threadIdx.y, w.z, chunk, part, pmax,
+    dc2d_tb2_body<MODEL, CHECK, true>(a, w.y * blockDim.y + threadIdx.y, w.z, chunk, part, pmax,
                                 (long long)blockIdx.x * blockDim.y + threadIdx.y);
 }
 

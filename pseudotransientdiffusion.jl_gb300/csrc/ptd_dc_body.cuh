@@ -98,12 +98,12 @@ __device__ __forceinline__ float2 face32x2(const DcArgs& a, float2 dL, float2 dR
     return fma2(f2(-cx, -cy), add2(w, uu), w);
 }
 
-template <int MODEL>
+template <int MODEL, bool TAB = false>
 __device__ __forceinline__ float cell_e32(const DcArgs& a, float h, float dmax)
 {
     if (MODEL == LIN) return a.e_lin;
     if (MODEL == LINSTEP) return linstep_cell_e(a.f, dmax);
-    return nonlin_cell_e(a.f, h);
+    return nonlin_cell_e<TAB>(a.f, h);
 }
 
 __device__ __forceinline__ bool dc_done(const int* done) { return __ldcg(done) != 0; }
@@ -137,7 +137,7 @@ __device__ __forceinline__ void dc1d_body(const DcArgs& a, int bx, float& part, 
     }
 }
 
-template <int MODEL, bool CHECK>
+template <int MODEL, bool CHECK, bool TAB = false>
 __device__ __forceinline__ void dc2d_body(const DcArgs& a, int tile, int cy, int chunk, float& part,
                                           unsigned& pmax, long long slot = 0)
 {
@@ -183,7 +183,7 @@ __device__ __forceinline__ void dc2d_body(const DcArgs& a, int tile, int cy, int
             if (own_x) a.wout[0][idx] = wxn;
             if (upd) {
                 a.wout[1][idx] = wyn;
-                const float e = cell_e32<MODEL>(a, hc, fmaxf(fmaxf(fmaxf(Dc, Dl), fmaxf(Dr, Db)), Dn));
+                const float e = cell_e32<MODEL, TAB>(a, hc, fmaxf(fmaxf(fmaxf(Dc, Dl), fmaxf(Dr, Db)), Dn));
                 const float div = fmaf(wyn - wyb, a.sig[1], (wxn - wxl) * a.sig[0]);
                 const float dnew = fmaf(-e, fmaf(dc, a.rdt, div - rr), dc);
                 a.dout[idx] = dnew;
@@ -245,7 +245,7 @@ __device__ __forceinline__ float dc_star(float Dc, float Db, float Dn)
     return fmaxf(fmaxf(fmaxf(Dc, Dl), fmaxf(Dr, Db)), Dn);
 }
 
-template <int MODEL, bool CHECK>
+template <int MODEL, bool CHECK, bool TAB = false>
 __device__ __forceinline__ void dc2d_tb2_body(const DcArgs& a, int tile, int cy, int chunk, float& part,
                                               unsigned& pmax, long long slot = 0)
 {
@@ -293,7 +293,7 @@ __device__ __forceinline__ void dc2d_tb2_body(const DcArgs& a, int tile, int cy,
         const float wyZA = face32<MODEL, false>(a, dZ, dA, hZ, hA, DZ, DA, a.win[1][oZ], u);
         const float wxA = x1(oA, dA, hA, DA);
         const float wxAl = __shfl_up_sync(FULL, wxA, 1);
-        const float eA = cell_e32<MODEL>(a, hA, dc_star<MODEL>(DA, DZ, DB));
+        const float eA = cell_e32<MODEL, TAB>(a, hA, dc_star<MODEL>(DA, DZ, DB));
         if (upd1) pA = dc_update(a, dA, wxA, wxAl, wyAB, wyZA, a.r[oA], eA);
     }
     float wx1p = x1(oB, dB, hB, DB);                                                  // w'_x(j0)
@@ -302,7 +302,7 @@ __device__ __forceinline__ void dc2d_tb2_body(const DcArgs& a, int tile, int cy,
     float p0 = dB;                                                                    // delta'(j0)
     {
         const float wxl = __shfl_up_sync(FULL, wx1p, 1);
-        const float eB = cell_e32<MODEL>(a, hB, dc_star<MODEL>(DB, DA, D1));
+        const float eB = cell_e32<MODEL, TAB>(a, hB, dc_star<MODEL>(DB, DA, D1));
         if (upd1) p0 = dc_update(a, dB, wx1p, wxl, wy1p, wyAB, r0, eB);
     }
     float uy2b = 0.0f;
@@ -334,7 +334,7 @@ __device__ __forceinline__ void dc2d_tb2_body(const DcArgs& a, int tile, int cy,
                 wy1 = face32<MODEL, false>(a, d1, d2, h1, h2, D1, D2, a.win[1][o], u);
             }
             const float wx1l = __shfl_up_sync(FULL, wx1, 1);
-            const float e1 = cell_e32<MODEL>(a, h1, dc_star<MODEL>(D1, D0, D2));
+            const float e1 = cell_e32<MODEL, TAB>(a, h1, dc_star<MODEL>(D1, D0, D2));
             if (upd1) p1 = dc_update(a, d1, wx1, wx1l, wy1, wy1p, r1, e1);
             d1 = d2;
         }
@@ -356,7 +356,7 @@ __device__ __forceinline__ void dc2d_tb2_body(const DcArgs& a, int tile, int cy,
         }
         const float wx2l = __shfl_up_sync(FULL, wx2, 1);
         const float ux2l = CHECK ? __shfl_up_sync(FULL, ux2, 1) : 0.0f;
-        const float e0 = cell_e32<MODEL>(a, h0, dc_star<MODEL>(D0, Dm1, D1));
+        const float e0 = cell_e32<MODEL, TAB>(a, h0, dc_star<MODEL>(D0, Dm1, D1));
         const long long os = o - sy;
         if (own_x) a.wout[0][os] = wx2;
         if (upd2) {

@@ -170,11 +170,15 @@ __device__ __forceinline__ float nonlin_face_c(const FParams& a, float hsum, flo
 
 // NONLIN cell: e = 1/(1/dtau + 1/dt) with
 // 1/dtau = H^3 Re / (Vpdtau L Resc) = (pi H^3 + sqrt(pi^2 H^6 + L^2 H^3/dt)) * k1
-// (scripts/diff_2D_nonlin.jl:23,26); finite for H^3 -> 0 (e -> dt).
+// (scripts/diff_2D_nonlin.jl:23,26); finite for H^3 -> 0 (e -> dt).  TAB, the
+// kernels that read their parameters from a table in memory (batch, adjoint):
+// the root's argument fused over the other of its two products.  Either is as
+// near; a last-bit change of e moves iteration counts of the defect correction.
+template <bool TAB = false>
 __device__ __forceinline__ float nonlin_cell_e(const FParams& a, float h, float efac = 1.0f)
 {
-    const float h3 = __fmul_rn(__fmul_rn(__fmul_rn(efac, h), h), h);
-    const float q = __fmaf_rn(__fmul_rn(a.fpi2, h3), h3, __fmul_rn(a.fA, h3));
+    const float h3 = __fmul_rn(__fmul_rn(__fmul_rn(efac, h), h), h), p = __fmul_rn(a.fpi2, h3);
+    const float q = TAB ? __fmaf_rn(a.fA, h3, __fmul_rn(p, h3)) : __fmaf_rn(p, h3, __fmul_rn(a.fA, h3));
     return frcp(__fmaf_rn(__fmaf_rn(a.fpi, h3, fsqrt(q)), a.fk1, a.frdt));
 }
 

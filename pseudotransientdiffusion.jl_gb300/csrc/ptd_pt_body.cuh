@@ -188,13 +188,13 @@ struct ModelTraits {
     static constexpr bool hasd = MODEL == LINSTEP || MODEL == NONLIN_EXPM;   // a per-cell field in a.D
 };
 
-template <int MODEL>
+template <int MODEL, bool TAB = false>
 __device__ __forceinline__ float cell_e(const PTArgs& a, float h, float dmax)
 {
     if (MODEL == LIN) return a.fe_lin;
     if (MODEL == LINSTEP) return linstep_cell_e(a.f, dmax);
-    if (MODEL == NONLIN_EXPM) return nonlin_cell_e(a.f, h, dmax);   // dmax carries exp(m) of the cell
-    return nonlin_cell_e(a.f, h);
+    if (MODEL == NONLIN_EXPM) return nonlin_cell_e<TAB>(a.f, h, dmax);   // dmax carries exp(m) of the cell
+    return nonlin_cell_e<TAB>(a.f, h);
 }
 
 // H - Hold: integer arithmetic for native FP64 (not in 1D).
@@ -272,8 +272,8 @@ __device__ __forceinline__ void pt1d_body(const PTArgs& a, int bx, double& part,
 // 2D: blockDim = (32, W); warp w of block b owns the x strip of tile
 // t = b*W + w: cells i = 31t + lane (lane 0 = left neighbour), and marches
 // rows j0 .. j1-1 of y chunk cy.
-// slot: the warp's slot in a.parts (when a.parts is set).
-template <class N, int MODEL, bool CHECK>
+// slot: the warp's slot in a.parts (when a.parts is set).  TAB: see nonlin_cell_e.
+template <class N, int MODEL, bool CHECK, bool TAB = false>
 __device__ __forceinline__ void pt2d_body(const PTArgs& a, int tile, int cy, int chunk, double& part,
                                           unsigned long long& pmax, long long slot = 0)
 {
@@ -352,7 +352,7 @@ __device__ __forceinline__ void pt2d_body(const PTArgs& a, int tile, int cy, int
                 st<N>(a.wout[1], idx, wyn);
                 const float dmax = MODEL == LINSTEP ? fmaxf(fmaxf(fmaxf(dcf, dlf), fmaxf(N::lo_f(Dr), dbf)), dnf)
                                                     : (MODEL == NONLIN_EXPM ? N::lo_f(Dc) : 0.0f);
-                const float e = cell_e<MODEL>(a, hc, dmax);
+                const float e = cell_e<MODEL, TAB>(a, hc, dmax);
                 // the flux differences (x, y), packed for the double-float forms
                 if constexpr (N::native) {
                     dx = N::sub(wxn, wxl);

@@ -69,7 +69,7 @@ DTYPES = {"fp64": "f64", "df64": "df64 (f32x2)", "dfh": "f64 state, df64 (f32x2)
 TRAFFIC = {("3d_nonlin_512", "fp64"): "pt_kernel_3d_nonlin_512.md",
            ("2d_nonlin_4096", "fp64"): "pt_kernel_2d_nonlin_4096.md",
            ("2d_nonlin_4096", "fp32_rb"): "rb2d_tb2_pair_nonlin_4096.md",
-           ("3d_nonlin_512", "fp32_rb"): "rb3d_nonlin_256.md"}
+           ("3d_nonlin_512", "fp32_rb"): "rb3d_nonlin_320x255x191.md"}
 
 
 def log(*a):

@@ -105,8 +105,11 @@ enum { PTD_NORM_RMS = 0, PTD_NORM_MAX = 1 };
 
 /* Flags */
 #define PTD_FLAG_STRICT 0x1   /* return PTD_ENOTCONV when a step stops at itmax */
-#define PTD_FLAG_AUTOTUNE 0x2 /* ptd_create times every launch shape of the fused kernel (2D: warps per CTA
-                                 x rows per y march; 3D: z-march length x warps per CTA) and keeps the fastest */
+#define PTD_FLAG_AUTOTUNE 0x2 /* ptd_create times every launch shape of the kernel of one iteration per launch
+                                 (2D: warps per CTA x rows per y march; 3D: z-march length x warps per CTA) and
+                                 keeps the fastest; the context runs that kernel, also on FP64 grids that would
+                                 otherwise take whole steps in one launch, which is faster there (see
+                                 ptd_launch_config) */
 #define PTD_FLAG_DC_NO_TBLOCK 0x4 /* FP32_DC and FP32_RB in 2D: one FP32 iteration per launch (default: two
                                      per launch, temporally blocked, when the check cadence is even) */
 #define PTD_FLAG_RB_TBLOCK_3D 0x8 /* FP32_RB in 3D (LIN, NONLIN): two FP32 iterations per launch (z temporal
@@ -181,8 +184,10 @@ PTD_API int ptd_get_state(ptd_ctx* ctx, double* H);    /* H out */
  * march, warps per 3D CTA, planes per 3D z march}.  (FP64 grids that take
  * whole steps in one launch use none of it until a shape is set: 1D up to
  * 13824 cells; LIN, LINSTEP and NONLIN in 2D up to about 470000 cells (LIN
- * 560000) and in 3D from 32768 to about 260000 cells (LIN 300000); mixed
- * residual.) */
+ * 560000) and in 3D from 32768 to about 260000 cells (LIN 300000; smaller 3D
+ * grids keep one launch per iteration, as readers of ptd_counters' launches
+ * expect of them); mixed residual; check blocks of up to 2^18 iterations; not
+ * with PTD_FLAG_AUTOTUNE.) */
 PTD_API int ptd_launch_config(ptd_ctx* ctx, int32_t cfg[4]);
 /* Set it (e.g. a shape found by PTD_FLAG_AUTOTUNE on another context of the
  * same size): warps per 2D CTA in {1,2,4,8}, rows per 2D march in [1,4096],

@@ -409,8 +409,8 @@ __global__ void tofloat_batch_kernel(const double* src, float* dst, long long n)
 // their remaining work rather than a table walk per work item of the whole
 // batch.  (A persistent grid walking the list held 74-98 registers against
 // the march's 40-64.)  The check variants are held to 40 registers (46-76
-// without a bound): a step of 48 LINSTEP instances of 64^2 to 512^2 7.62 ms
-// without, 7.54 at 48, 7.45 at 40, 7.80 at 32.
+// without a bound): a step of 48 LINSTEP instances of 64^2 to 512^2 9.84 ms
+// without, 9.82 at 64, 9.69 at 48, 9.46 at 40.
 template <int MODEL, bool CHECK, int TB>
 __global__ void __launch_bounds__(256, CHECK ? 6 : 0) rb2d_batch_kernel(const RbArgs* __restrict__ tab,
                                                          const int4* __restrict__ work,
@@ -1399,9 +1399,11 @@ extern "C" int ptd_batch_create(ptd_batch** out, const ptd_batch_params* p, cons
     if (b->dc && p->itmax % b->nchk) b->nchk = p->nchk;
     b->tb = ((b->dc || b->rb) && b->nchk % 2 == 0 && !(p->flags & PTD_FLAG_DC_NO_TBLOCK)) ? 2 : 1;
     {   // rows per y chunk: 32, shorter (>= 8, alloc_slots) where the batch
-        // would not fill the SMs, in 2-warp CTAs then.  FP32_RB steps, 8 warps
-        // x 32 rows / as taken: 48 grids of 64..512 11.6, 10.0 ms (16 rows);
-        // 32 of 128..200 3.7, 2.3 ms (8); 8 of 32..100 1.7, 1.1 ms (8).
+        // would not fill the SMs, in 2-warp CTAs then.  ms of a LINSTEP step at
+        // 32 rows / as taken, 48 grids of 64..512 (16 rows), 32 of 128..200
+        // (8), 8 of 32..100 (8): FP32_RB 11.3, 9.2; 3.7, 2.3; 1.5, 0.93; FP64
+        // 40.7, 34.5; 10.4, 5.9; 3.6, 1.3; DF64 22.9, 20.8; 6.0, 3.5; 2.2, 0.94;
+        // FP32_DC 14.5, 11.5; 4.8, 2.7; 1.4, 0.86.
         auto warps = [&](int ch) {
             long long n = 0;
             const int cols = b->tb == 2 ? 28 : 31;

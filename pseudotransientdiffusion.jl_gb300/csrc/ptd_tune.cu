@@ -110,9 +110,9 @@ int rb3d_rows(int model, long long nx, long long ny, long long nz)
 }
 
 // z march of the 8-row FP32 kernels and of the adjoint, at least per_sm CTAs
-// per SM down to a march of one plane.  A gradient of 72^3 at marches 1, 2, 3,
-// 4, 6: rebased 11.2, 10.4, 10.2, 10.1, 10.5 ms; FP64 37.3, 34.9, 35.6, 36.8,
-// 39.6 (16-row CTAs at their best: 10.4, 38.3).
+// per SM down to a march of one plane.  A gradient of 72^3 over three steps at
+// marches 1, 2, 3, 4, 6: rebased 12.1, 11.1, 10.4, 10.4, 10.9 ms (4 is taken);
+// FP64 36.7, 34.3, 35.0, 36.2, 38.9 (2; in 16-row CTAs 38.3 at best).
 int z_march8(const ptd_params& p, int per_sm)
 {
     const long long bxy = ceil_div(p.nx - 2, 31) * ceil_div(p.ny - 2, 7);

@@ -755,14 +755,6 @@ extern "C" int ptd_set_state2(ptd_ctx* c, const double* H, const double* Hold, c
     if (c->p.model == PTD_MODEL_LINSTEP && !D) return fail(PTD_EINVAL, "the step model needs D");
     if (c->p.model == PTD_MODEL_NONLIN_EXPM && !D) return fail(PTD_EINVAL, "the exp(m) H^3 model needs m (in D)");
     const size_t bytes = (size_t)c->nfield * sizeof(double);
-    if (c->flow.rows) {
-        CK(cudaStreamSynchronize(c->stream));
-        if (c->h_st->pad) {   // a launch that gave up: its tags are part used, its status is told
-            CK(cudaMemsetAsync(c->flow_mem, 0, flow_bytes(c->flow), c->stream));
-            c->flow_tag = 1;
-            c->h_st->pad = 0;
-        }
-    }
     // padding stays zero: clear whole buffers first
     double* Hdst = c->df64 ? c->stage : c->H[0];
     if (c->sy != c->nx) CK(cudaMemsetAsync(Hdst, 0, bytes, c->stream));
@@ -820,6 +812,11 @@ extern "C" int ptd_set_state2(ptd_ctx* c, const double* H, const double* Hold, c
         if (rc) return rc;
     }
     CK(cudaStreamSynchronize(c->stream));
+    if (c->flow.rows && c->h_st->pad) {   // a launch before this state gave up: its tags are part used, its status is told
+        CK(cudaMemsetAsync(c->flow_mem, 0, flow_bytes(c->flow), c->stream));
+        c->flow_tag = 1;
+        c->h_st->pad = 0;
+    }
     c->have_state = true;
     return PTD_OK;
 }
